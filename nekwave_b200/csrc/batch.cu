@@ -124,7 +124,7 @@ batch_stage_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
         P.k = S.k;
         P.stride = S.stride;
         P.nelt = S.nelt;
-        P._pad0 = 0;
+        P.kio = stage_kio(stage);
         P.D = S.D;
         P.geo = S.geo;
         P.conn = S.conn;
@@ -165,7 +165,7 @@ __device__ __forceinline__ StageParams slot_params(const SlotDev& S, int stage, 
     P.k = S.k;
     P.stride = S.stride;
     P.nelt = S.nelt;
-    P._pad0 = 0;
+    P.kio = stage_kio(stage);
     P.D = S.D;
     P.geo = S.geo;
     P.conn = S.conn;
@@ -280,7 +280,7 @@ struct PoolPull {
         if (!S.active) return;
         constexpr long long N3 = N * N * N;
         stage::prefetch_nodes_l2(S.u[S.par ^ (stage & 1)], S.k, S.stride, w.e0 * N3,
-                                 min(NBulk<N>::EPB, S.nelt - w.e0) * N3);
+                                 min(NBulk<N>::EPB, S.nelt - w.e0) * N3, stage_kio(stage));
     }
 };
 

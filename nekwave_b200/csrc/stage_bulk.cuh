@@ -126,11 +126,14 @@ __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, u
     const long long ca0 = c0 & ~3ll, ca1 = (c1 + 3) & ~3ll;
     const unsigned cb = static_cast<unsigned>((ca1 - ca0) * 4);
     const unsigned gb = static_cast<unsigned>(nvalid * sizeof(ElemGeo));
-    mbar_arrive_expect_tx(bar, (KSM ? 12 : 6) * ub + gb + cb);
+    const bool kread = (P.kio & kKRead) != 0;
+    mbar_arrive_expect_tx(bar, (KSM && kread ? 12 : 6) * ub + gb + cb);
     double* su = reinterpret_cast<double*>(smem + L::u0);
 #pragma unroll
     for (int c = 0; c < 6; ++c) bulk_g2s(su + c * L::CSR, P.u_in + c * S + a0, ub, bar);
-    if constexpr (KSM) {
+    if (!kread) {
+        // the first stage of a step: no k
+    } else if constexpr (KSM) {
         double* sk = reinterpret_cast<double*>(smem + L::k0);
 #pragma unroll
         for (int c = 0; c < 6; ++c) bulk_g2s(sk + c * L::CSR, P.k + c * S + a0, ub, bar);

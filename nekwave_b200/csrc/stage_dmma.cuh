@@ -52,6 +52,7 @@ __device__ __forceinline__ void dmma8_planes(const StageParams& P, const double*
                                              long long ebase, const double* __restrict__ Dc) {
     constexpr int N = 8, N3 = 512;
     const double A = P.a, B = P.b, DT = P.dt;
+    const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
     const long long S = P.stride;
 #pragma unroll
     for (int k = K0; k < K0 + NK; ++k) {
@@ -59,7 +60,8 @@ __device__ __forceinline__ void dmma8_planes(const StageParams& P, const double*
         double2 kold[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-            kold[c] = __ldcg(reinterpret_cast<const double2*>(P.k + (dst + c) * S + ebase + ms));
+            kold[c] = kread ? __ldcg(reinterpret_cast<const double2*>(P.k + (dst + c) * S + ebase + ms))
+                            : make_double2(0.0, 0.0);
         // r (original form): A[g][t] = V(l = t, j = g, k)
         double zr0 = 0.0, zr1 = 0.0, yr0 = 0.0, yr1 = 0.0;
         dmma_f64(zr0, zr1, V[2 * N3 + 64 * k + 8 * g + t], d0);
@@ -96,7 +98,8 @@ __device__ __forceinline__ void dmma8_planes(const StageParams& P, const double*
             const double kn0 = A * kold[c].x + DT * rhs0[c];
             const double kn1 = A * kold[c].y + DT * rhs1[c];
             const double2 uo = *reinterpret_cast<const double2*>(su + (dst + c) * N3 + ms);
-            __stcs(reinterpret_cast<double2*>(P.k + (dst + c) * S + ebase + ms), make_double2(kn0, kn1));
+            if (kwrite)
+                __stcs(reinterpret_cast<double2*>(P.k + (dst + c) * S + ebase + ms), make_double2(kn0, kn1));
             __stcs(reinterpret_cast<double2*>(P.u_out + (dst + c) * S + ebase + ms),
                    make_double2(uo.x + B * kn0, uo.y + B * kn1));
         }

@@ -171,7 +171,9 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const int e0,
             for (int x = tid; x < nvalid * 6; x += NT) s_conn[x] = P.conn[e0 * 6 + x];
         }
         cp_async_commit();
-        if constexpr (KSMEM) {
+        if ((P.kio & kKRead) == 0) {
+            // the first stage of a step: no k
+        } else if constexpr (KSMEM) {
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 const double* src = P.k + c * S + gbase;
@@ -291,6 +293,7 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const int e0,
         for (int c = 0; c < 9; ++c) m_[c] = static_cast<TC>(s_geo[team].met[c]);
     }
     const double A = P.a, B = P.b, DT = P.dt;
+    const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
     const long long ebase = static_cast<long long>(e) * N3;
 
     // the k-planes of a thread: unrolled (more independent work in flight) unless
@@ -408,11 +411,12 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const int e0,
         const long long g = ebase + mloc;
         double kold[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) kold[c] = KSMEM ? s_k[c * CS + sl] : __ldcg(P.k + c * S + g);
+        for (int c = 0; c < 6; ++c)
+            kold[c] = !kread ? 0.0 : (KSMEM ? s_k[c * CS + sl] : __ldcg(P.k + c * S + g));
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
             const double kn = A * kold[c] + DT * rhs[c];
-            __stcs(P.k + c * S + g, kn);
+            if (kwrite) __stcs(P.k + c * S + g, kn);
             __stcs(P.u_out + c * S + g, s_u[c * CS + sl] + B * kn);
         }
     }

@@ -128,11 +128,12 @@ __device__ __forceinline__ void stage_tile_mma8(const StageParams& P, const int 
     }
     // the LSRK register of this thread's four epilogue nodes, loaded now (shared
     // memory, not registers, limits the resident blocks, so they are free)
+    const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
     double kold[4][6];
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) kold[n][c] = __ldcg(P.k + c * S + gbase + tid + 128 * n);
+        for (int c = 0; c < 6; ++c) kold[n][c] = kread ? __ldcg(P.k + c * S + gbase + tid + 128 * n) : 0.0;
     cp_async_wait<0>();
     __syncthreads();
 
@@ -233,7 +234,7 @@ __device__ __forceinline__ void stage_tile_mma8(const StageParams& P, const int 
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
             const double kn = A * kold[n][c] + DT * s_r[c * RE + ar];
-            __stcs(P.k + c * S + gi, kn);
+            if (kwrite) __stcs(P.k + c * S + gi, kn);
             __stcs(P.u_out + c * S + gi, s_u[c * UE + au] + B * kn);
         }
     }

@@ -77,18 +77,19 @@ __device__ __forceinline__ int tile_ahead(int b) {
 }
 
 // Nodes [g0, g0 + cnt) of the six components of u and of k (component stride S)
-// pulled into L2 by twelve bulk prefetches (one thread; nothing waits on them), for
+// pulled into L2 by bulk prefetches (one thread; nothing waits on them; k when kio reads it), for
 // the block that will load them later: its own copies then read L2 instead of DRAM.
 // The ranges are rounded out to 16-byte boundaries, which stay inside the state
 // arrays (components are 512-byte aligned and padded to 64 doubles).
 __device__ __forceinline__ void prefetch_nodes_l2(const double* u, const double* k, long long S,
-                                                  long long g0, long long cnt) {
+                                                  long long g0, long long cnt, int kio) {
     const long long a0 = g0 & ~1ll, a1 = (g0 + cnt + 1) & ~1ll;
     const unsigned bytes = static_cast<unsigned>((a1 - a0) * 8);
 #pragma unroll
     for (int c = 0; c < 6; ++c)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(u + c * S + a0), "r"(bytes)
                      : "memory");
+    if ((kio & kKRead) == 0) return;
 #pragma unroll
     for (int c = 0; c < 6; ++c)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(k + c * S + a0), "r"(bytes)
@@ -98,7 +99,8 @@ __device__ __forceinline__ void prefetch_nodes_l2(const double* u, const double*
 // The u_in and k of the tile of elements [e0, e0 + n) pulled into L2.
 template <int N3>
 __device__ __forceinline__ void prefetch_tile_l2(const StageParams& P, int e0, int n) {
-    prefetch_nodes_l2(P.u_in, P.k, P.stride, static_cast<long long>(e0) * N3, static_cast<long long>(n) * N3);
+    prefetch_nodes_l2(P.u_in, P.k, P.stride, static_cast<long long>(e0) * N3, static_cast<long long>(n) * N3,
+                      P.kio);
 }
 
 // The no-op L2 pull of a tile function (see bulk_tile).
@@ -179,6 +181,7 @@ __device__ __forceinline__ void issue2(const StageParams& P, const int e0, doubl
         for (int x = tid; x < nvalid * 6; x += NT) cp_async4(sc + x, P.conn + e0 * 6 + x);
     }
     // the tile's k lines into L2; the owner threads read them in the column phase
+    if ((P.kio & kKRead) == 0) return;
     const int lines = (cnt * 8 + 127) / 128;
     for (int x = tid; x < 6 * lines; x += NT) {
         const int c = x / lines, ln = x - c * lines;
@@ -717,6 +720,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         for (int c = 0; c < 9; ++c) m_[c] = static_cast<TC>(sg[team].met[c]);
     }
     const double A = P.a, B = P.b, DT = P.dt;
+    const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
     const long long ebase = static_cast<long long>(e) * N3;
 
     if constexpr (SPLIT) {
@@ -763,7 +767,9 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         if constexpr (CONSTD) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                knext[c] = KSM ? Kf[(dst + c) * CS + i + RP * j] : __ldcg(P.k + (dst + c) * S + ebase + i + N * j);
+                knext[c] = !kread ? 0.0
+                         : (KSM ? Kf[(dst + c) * CS + i + RP * j]
+                                : __ldcg(P.k + (dst + c) * S + ebase + i + N * j));
         }
 #pragma unroll (CONSTD ? N : 1)
         for (int k = 0; k < N; ++k) {
@@ -777,12 +783,13 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
                 if (k + 1 < N) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c)
-                        knext[c] = KSM ? Kf[(dst + c) * CS + ms + PP] : __ldcg(P.k + (dst + c) * S + g + N2);
+                        knext[c] = !kread ? 0.0
+                                 : (KSM ? Kf[(dst + c) * CS + ms + PP] : __ldcg(P.k + (dst + c) * S + g + N2));
                 }
             } else {
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    kold[c] = KSM ? Kf[(dst + c) * CS + ms] : __ldcg(P.k + (dst + c) * S + g);
+                    kold[c] = !kread ? 0.0 : (KSM ? Kf[(dst + c) * CS + ms] : __ldcg(P.k + (dst + c) * S + g));
             }
             double rhs[3];
             if constexpr (GEO == GEO_BOX) {
@@ -864,7 +871,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const double kn = A * kold[c] + DT * rhs[c];
-                __stcs(P.k + (dst + c) * S + g, kn);
+                if (kwrite) __stcs(P.k + (dst + c) * S + g, kn);
                 __stcs(P.u_out + (dst + c) * S + g, Uf[(dst + c) * CS + ms] + B * kn);
             }
         }
@@ -888,7 +895,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
             double kold[6];
 #pragma unroll
             for (int c = 0; c < 6; ++c)
-                kold[c] = KSM ? sk[c * CS + team * EN3 + ms] : __ldcg(P.k + c * S + g);
+                kold[c] = !kread ? 0.0 : (KSM ? sk[c * CS + team * EN3 + ms] : __ldcg(P.k + c * S + g));
             double rhs[6];
             if constexpr (GEO == GEO_BOX) {
                 TC Hz_r = 0, Hy_r = 0, Ez_r = 0, Ey_r = 0;
@@ -967,7 +974,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 const double kn = A * kold[c] + DT * rhs[c];
-                __stcs(P.k + c * S + g, kn);
+                if (kwrite) __stcs(P.k + c * S + g, kn);
                 __stcs(P.u_out + c * S + g, Uf[c * CS + ms] + B * kn);
             }
         }
