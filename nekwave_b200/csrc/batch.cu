@@ -45,7 +45,8 @@ constexpr int bsmem() {
     using B = BShape<N>;
     if constexpr (dmma_tile<N, F32>()) return stage::DmmaLayout8::total;
     else if constexpr (B::ALG == 0) return SmemLayout<N, F32, B::EPB, false>::total;
-    else return stage::Layout2<N, F32, B::EPB, false, (((B::ALG - 2) & 4) != 0)>::total;
+    else return stage::Layout2<N, F32, B::EPB, false, (((B::ALG - 2) & 4) != 0),
+                               stage::flux_planes<GEO_BOX, (((B::ALG - 2) & 2) != 0)>()>::total;
 }
 
 // One tile of the second family without the persistent loop: stage u_in (and D,
@@ -57,7 +58,7 @@ __device__ __forceinline__ void tile2(const StageParams& P, int e0, unsigned cha
     constexpr bool SPLIT = ((ALG - 2) & 2) != 0, PAD = ((ALG - 2) & 4) != 0;
     constexpr bool CONSTD = ((ALG - 2) & 8) != 0;
     static_assert(((ALG - 2) & 1) == 0 && ((ALG - 2) & 16) == 0, "one tile per call, tile resident");
-    using L2 = stage::Layout2<N, F32, EPB, false, PAD>;
+    using L2 = stage::Layout2<N, F32, EPB, false, PAD, stage::flux_planes<GEO_BOX, SPLIT>()>;
     constexpr int NT = EPB * KS * N * N;
     double* sD = reinterpret_cast<double*>(smem + L2::D);
     double* su = reinterpret_cast<double*>(smem + L2::u0);
@@ -70,7 +71,7 @@ __device__ __forceinline__ void tile2(const StageParams& P, int e0, unsigned cha
     stage::cp_async_commit();
     stage::cp_async_wait<0>();
     __syncthreads();
-    stage::FaceGather<stage::face_points_per_thread<N, KS>()> G;
+    stage::FaceRegs<N, GEO_BOX, KS, SPLIT> G;
     stage::compute2<N, GEO_BOX, F32, KS, EPB, SPLIT, PAD, CONSTD>(P, e0, su, sg, sc, sD,
                                                                   reinterpret_cast<double*>(smem + L2::flux),
                                                                   smem + L2::uc, tid, G, Dc);
@@ -89,16 +90,16 @@ __device__ __forceinline__ void run_tile(const StageParams& P, int e0, unsigned 
         tile2<N, F32, B::KS, B::EPB, B::ALG>(P, e0, smem, tid);
 }
 
-// Carpenter-Kennedy LSRK45 (src/dg_solver.cpp:58-69).
-__constant__ double c_rk4a[5] = {0.0, -567301805773.0 / 1357537059087.0,
-                                 -2404267990393.0 / 2016746695238.0,
-                                 -3550918686646.0 / 2091501179385.0,
-                                 -1275806237668.0 / 842570457699.0};
-__constant__ double c_rk4b[5] = {1432997174477.0 / 9575080441755.0,
-                                 5161836677717.0 / 13612068292357.0,
-                                 1720146321549.0 / 2090206949498.0,
-                                 3134564353537.0 / 4481467310338.0,
-                                 2277821191437.0 / 14882151754819.0};
+// Carpenter-Kennedy LSRK45 (src/dg_solver.cpp:58-69), for the host and the device.
+#define NWB_RK4A {0.0, -567301805773.0 / 1357537059087.0, -2404267990393.0 / 2016746695238.0, \
+                  -3550918686646.0 / 2091501179385.0, -1275806237668.0 / 842570457699.0}
+#define NWB_RK4B {1432997174477.0 / 9575080441755.0, 5161836677717.0 / 13612068292357.0, \
+                  1720146321549.0 / 2090206949498.0, 3134564353537.0 / 4481467310338.0, \
+                  2277821191437.0 / 14882151754819.0}
+__constant__ double c_rk4a[5] = NWB_RK4A;
+__constant__ double c_rk4b[5] = NWB_RK4B;
+const double kRk4a[5] = NWB_RK4A;
+const double kRk4b[5] = NWB_RK4B;
 
 template <bool F32>
 __global__ void __launch_bounds__(kBatchThreads, 3)
@@ -156,16 +157,23 @@ batch_stage_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
     }
 }
 
+// What a per-N launch knows of its stage: the LSRK coefficients are kernel parameters
+// (constant-bank operands, no registers); dry: a = b = dt = 0 (timing only).
+struct BatchStage {
+    double a, b;
+    int stage, dry;
+};
+
 // Stage parameters of one tile's slot.
-__device__ __forceinline__ StageParams slot_params(const SlotDev& S, int stage, int dry) {
-    const int par = S.par ^ (stage & 1);
+__device__ __forceinline__ StageParams slot_params(const SlotDev& S, const BatchStage& bs) {
+    const int par = S.par ^ (bs.stage & 1);
     StageParams P;
     P.u_in = S.u[par];
     P.u_out = S.u[par ^ 1];
     P.k = S.k;
     P.stride = S.stride;
     P.nelt = S.nelt;
-    P.kio = stage_kio(stage);
+    P.kio = stage_kio(bs.stage);
     P.D = S.D;
     P.geo = S.geo;
     P.conn = S.conn;
@@ -179,9 +187,9 @@ __device__ __forceinline__ StageParams slot_params(const SlotDev& S, int stage, 
     P.spmask = 0;
     for (int x = 0; x < 10; ++x) P.zl[x] = S.zl[x];
     P.c0 = S.c0;
-    P.a = dry ? 0.0 : c_rk4a[stage];
-    P.b = dry ? 0.0 : c_rk4b[stage];
-    P.dt = dry ? 0.0 : S.dt;
+    P.a = bs.a;
+    P.b = bs.b;
+    P.dt = bs.dry ? 0.0 : S.dt;
     return P;
 }
 
@@ -198,12 +206,13 @@ struct DParam {
 template <int N, bool F32, int KS, int EPB, bool KSMEM, int MINB, int ALG>
 __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
 batch_stage_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
-                     int stage, int dry, const __grid_constant__ DParam dp) {
+                     const __grid_constant__ BatchStage bs,
+                     const __grid_constant__ DParam dp) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WorkItem w = work[blockIdx.x];
     const SlotDev& S = slots[w.slot];
     if (!S.active) return;
-    const StageParams P = slot_params(S, stage, dry);
+    const StageParams P = slot_params(S, bs);
     if constexpr (ALG == 0)
         stage_tile<N, GEO_BOX, F32, KS, EPB, KSMEM, true>(P, w.e0, smem, threadIdx.x);
     else
@@ -214,26 +223,26 @@ batch_stage_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restri
 // (128 threads, one element per block), D from dp (CD) or from shared memory.
 template <int MINB, bool CD>
 __global__ void __launch_bounds__(128, MINB)
-batch_dmma8_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work, int stage,
-                   int dry, const __grid_constant__ DParam dp) {
+batch_dmma8_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
+                   const __grid_constant__ BatchStage bs, const __grid_constant__ DParam dp) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WorkItem w = work[blockIdx.x];
     const SlotDev& S = slots[w.slot];
     if (!S.active) return;
-    const StageParams P = slot_params(S, stage, dry);
+    const StageParams P = slot_params(S, bs);
     stage::dmma8_tile<2>(P, w.e0, smem, threadIdx.x,
                          CD ? dp.d : reinterpret_cast<const double*>(smem + stage::DmmaLayout8::D));
 }
 
 template <bool CD>
-cudaError_t launch_dmma8_n(int stage, const SlotDev* slots, const WorkItem* work, int ntiles, int dry,
+cudaError_t launch_dmma8_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                            const DParam& dp, cudaStream_t st) {
     constexpr int smem = stage::DmmaLayout8::total;
     auto kern = batch_dmma8_kernel<4, CD>;
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    kern<<<ntiles, 128, smem, st>>>(slots, work, stage, dry, dp);
+    kern<<<ntiles, 128, smem, st>>>(slots, work, bs, dp);
     return cudaGetLastError();
 }
 
@@ -286,23 +295,23 @@ struct PoolPull {
 
 template <int N, bool CD>
 __global__ void __launch_bounds__(NBulk<N>::EPB * 2 * N * N, NBulk<N>::MINB)
-batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work, int stage,
-                    int dry, const __grid_constant__ DParam dp) {
+batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
+                    const __grid_constant__ BatchStage bs, const __grid_constant__ DParam dp) {
     extern __shared__ __align__(16) unsigned char smem[];
     const WorkItem w = work[blockIdx.x];
     const SlotDev& S = slots[w.slot];
     if (!S.active) return;
-    const StageParams P = slot_params(S, stage, dry);
+    const StageParams P = slot_params(S, bs);
     if constexpr (NBulk<N>::AHEAD > 0)
         stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, true, NBulk<N>::EARLY, NBulk<N>::VROW>(
-            P, w.e0, smem, threadIdx.x, dp.d, PoolPull<N>{slots, work, stage});
+            P, w.e0, smem, threadIdx.x, dp.d, PoolPull<N>{slots, work, bs.stage});
     else
         stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, true, NBulk<N>::EARLY, NBulk<N>::VROW>(
             P, w.e0, smem, threadIdx.x, dp.d);
 }
 
 template <int N, bool CD>
-cudaError_t launch_bulk_n(int stage, const SlotDev* slots, const WorkItem* work, int ntiles, int dry,
+cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                           const DParam& dp, cudaStream_t st) {
     constexpr int smem = stage::BulkLayout<N, NBulk<N>::EPB, true>::total;
     constexpr int threads = NBulk<N>::EPB * 2 * N * N;
@@ -310,30 +319,31 @@ cudaError_t launch_bulk_n(int stage, const SlotDev* slots, const WorkItem* work,
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    kern<<<ntiles, threads, smem, st>>>(slots, work, stage, dry, dp);
+    kern<<<ntiles, threads, smem, st>>>(slots, work, bs, dp);
     return cudaGetLastError();
 }
 
 template <int N, bool F32, int ALG>
-cudaError_t launch_n_alg(int stage, const SlotDev* slots, const WorkItem* work, int ntiles, int dry,
+cudaError_t launch_n_alg(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                          const DParam& dp, cudaStream_t st) {
     using Sh = NShape<N>;
     constexpr int threads = Sh::EPB * Sh::KS * N * N;
     constexpr int smem = ALG == 0
         ? SmemLayout<N, F32, Sh::EPB, (Sh::KSM != 0)>::total
-        : stage::Layout2<N, F32, Sh::EPB, false, (((ALG - 2) & 4) != 0)>::total;
+        : stage::Layout2<N, F32, Sh::EPB, false, (((ALG - 2) & 4) != 0),
+                         stage::flux_planes<GEO_BOX, (((ALG - 2) & 2) != 0)>()>::total;
     auto kern = batch_stage_n_kernel<N, F32, Sh::KS, Sh::EPB, (Sh::KSM != 0), Sh::MINB, ALG>;
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    kern<<<ntiles, threads, smem, st>>>(slots, work, stage, dry, dp);
+    kern<<<ntiles, threads, smem, st>>>(slots, work, bs, dp);
     return cudaGetLastError();
 }
 
 // Dh: this N's D on the host when every resident cavity of this N uses it (the
 // constant-bank form then applies), else null.
 template <int N, bool F32>
-cudaError_t launch_n(int stage, const SlotDev* slots, const WorkItem* work, int ntiles, int dry,
+cudaError_t launch_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                      const double* Dh, cudaStream_t st, int* epb_out) {
     using Sh = NShape<N>;
     if (epb_out) *epb_out = (NBulk<N>::on && !F32) ? NBulk<N>::EPB : Sh::EPB;
@@ -342,26 +352,26 @@ cudaError_t launch_n(int stage, const SlotDev* slots, const WorkItem* work, int 
         if constexpr (NBulk<N>::CD) {
             if (Dh) {
                 for (int x = 0; x < N * N; ++x) dp.d[x] = Dh[x];
-                return launch_bulk_n<N, true>(stage, slots, work, ntiles, dry, dp, st);
+                return launch_bulk_n<N, true>(bs, slots, work, ntiles, dp, st);
             }
             if (ntiles <= 0) {  // set-up call: prepare both forms
-                cudaError_t e = launch_bulk_n<N, true>(stage, slots, work, 0, dry, dp, st);
+                cudaError_t e = launch_bulk_n<N, true>(bs, slots, work, 0, dp, st);
                 if (e != cudaSuccess) return e;
             }
         }
-        return launch_bulk_n<N, false>(stage, slots, work, ntiles, dry, dp, st);
+        return launch_bulk_n<N, false>(bs, slots, work, ntiles, dp, st);
     }
     if constexpr (dmma_tile<N, F32>()) {
         DParam dp{};
         if (Dh) {
             for (int x = 0; x < N * N; ++x) dp.d[x] = Dh[x];
-            return launch_dmma8_n<true>(stage, slots, work, ntiles, dry, dp, st);
+            return launch_dmma8_n<true>(bs, slots, work, ntiles, dp, st);
         }
         if (ntiles <= 0) {  // set-up call: prepare both forms
-            cudaError_t e = launch_dmma8_n<true>(stage, slots, work, 0, dry, dp, st);
+            cudaError_t e = launch_dmma8_n<true>(bs, slots, work, 0, dp, st);
             if (e != cudaSuccess) return e;
         }
-        return launch_dmma8_n<false>(stage, slots, work, ntiles, dry, dp, st);
+        return launch_dmma8_n<false>(bs, slots, work, ntiles, dp, st);
     }
     constexpr bool cd_bit = Sh::ALG >= 2 && ((Sh::ALG - 2) & 8) != 0;
     constexpr bool has_cd = cd_bit && !F32;  // the constant-bank D is an FP64 form
@@ -370,14 +380,14 @@ cudaError_t launch_n(int stage, const SlotDev* slots, const WorkItem* work, int 
     if constexpr (has_cd) {
         if (Dh) {
             for (int x = 0; x < N * N; ++x) dp.d[x] = Dh[x];
-            return launch_n_alg<N, F32, Sh::ALG>(stage, slots, work, ntiles, dry, dp, st);
+            return launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, ntiles, dp, st);
         }
         if (ntiles <= 0) {  // set-up call: prepare both forms
-            cudaError_t e = launch_n_alg<N, F32, Sh::ALG>(stage, slots, work, 0, dry, dp, st);
+            cudaError_t e = launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, 0, dp, st);
             if (e != cudaSuccess) return e;
         }
     }
-    return launch_n_alg<N, F32, ALG_PLAIN>(stage, slots, work, ntiles, dry, dp, st);
+    return launch_n_alg<N, F32, ALG_PLAIN>(bs, slots, work, ntiles, dp, st);
 }
 
 // Does this slot record energy after the step it is taking now (post = 1), or
@@ -520,10 +530,11 @@ int max_batch_smem() {
 cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots,
                                  const WorkItem* work, int ntiles, int dry, const double* Dh,
                                  cudaStream_t st) {
+    const BatchStage bs{dry ? 0.0 : kRk4a[stage], dry ? 0.0 : kRk4b[stage], stage, dry};
     switch (N) {
 #define NWB_CASE(n) \
-        case n: return f32 ? launch_n<n, true>(stage, slots, work, ntiles, dry, Dh, st, nullptr) \
-                           : launch_n<n, false>(stage, slots, work, ntiles, dry, Dh, st, nullptr);
+        case n: return f32 ? launch_n<n, true>(bs, slots, work, ntiles, Dh, st, nullptr) \
+                           : launch_n<n, false>(bs, slots, work, ntiles, Dh, st, nullptr);
         NWB_CASE(2) NWB_CASE(3) NWB_CASE(4) NWB_CASE(5) NWB_CASE(6) NWB_CASE(7) NWB_CASE(8)
         NWB_CASE(9) NWB_CASE(10)
 #undef NWB_CASE

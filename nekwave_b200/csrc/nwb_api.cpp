@@ -98,6 +98,19 @@ int wall_code(const nwb_mesh_desc* m, long long fp, bool true_pmc) {
     return 0;
 }
 
+bool snap_axis_normals(std::vector<ElemGeo>& geo) {
+    constexpr int axis[6] = {1, 0, 1, 0, 2, 2};
+    for (const ElemGeo& G : geo)
+        for (int f = 0; f < 6; ++f)
+            for (int c = 0; c < 3; ++c)
+                if (c != axis[f] && !(std::abs(G.nrm[f][c]) <= 1e-12)) return false;
+    for (ElemGeo& G : geo)
+        for (int f = 0; f < 6; ++f)
+            for (int c = 0; c < 3; ++c)
+                if (c != axis[f]) G.nrm[f][c] = 0.0;
+    return true;
+}
+
 nwb_status analyse_mesh(const nwb_mesh_desc* m, Analysis* A, bool true_pmc) {
     const int N = m->N, nelt = m->nelt, N2 = N * N, N3 = N2 * N;
     const long long npts = static_cast<long long>(nelt) * N3;
@@ -179,6 +192,7 @@ nwb_status analyse_mesh(const nwb_mesh_desc* m, Analysis* A, bool true_pmc) {
             A->conn[6 * static_cast<size_t>(e) + f] = (eB << 6) | found;
         }
     }
+    if (affine && box) box = snap_axis_normals(A->egeo);
     A->geo = !affine ? nwb::GEO_NODAL : (box ? nwb::GEO_BOX : nwb::GEO_AFFINE);
     if (!affine) {
         A->egeo.clear();
@@ -673,6 +687,7 @@ nwb_status nwb_solver_create_box(int N, int nelx, int nely, int nelz, double xmi
         for (int c : {1, 2, 3, 5, 6, 7})
             if (std::abs(A.egeo[e].met[c]) > 1e-13 * scale) box = false;
     }
+    if (box) box = nwb::snap_axis_normals(A.egeo);
     A.geo = box ? nwb::GEO_BOX : nwb::GEO_AFFINE;
     nwb_status r = create_solver(nullptr, N, static_cast<int>(nelt), D.data(), w3.data(), A, c0, prec, out,
                                  false);

@@ -597,6 +597,7 @@ nwb_status nwb_pool_add_box(nwb_pool* p, int N, int nelx, int nely, int nelz, do
     try {
         nwb::gll(N, z, w, D);
         nwb::box_geometry(N, nelx, nely, nelz, lo, hi, periodic_mask, z, w, geo, conn);
+        nwb::snap_axis_normals(geo);
         nwb::box_probes(N, nelx, nely, nelz, lo, hi, z, nprobes, probe_xyz, pe, pw);
     } catch (const std::bad_alloc&) {
         return set_error(NWB_ENOMEM, "nwb_pool_add_box: out of host memory");

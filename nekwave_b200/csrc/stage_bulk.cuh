@@ -105,7 +105,7 @@ struct BulkLayout {
     static constexpr int conn_b = align16((EPB * 6 + 6) * 4);
     static constexpr int D = conn0 + conn_b;
     static constexpr int flux0 = D + align16(N2 * 8);
-    static constexpr int bar = flux0 + EPB * 36 * N2 * 8;
+    static constexpr int bar = flux0 + EPB * flux_planes<GEO_BOX, true>() * N2 * 8;
     static constexpr int flag = bar + 8;
     static constexpr int total = flag + 16;
 };
@@ -178,7 +178,7 @@ template <int N, int GEO, int KS, int EPB, bool CONSTD, bool DSMEM, bool KSM, bo
           bool VROW = false, bool ILP2 = false, class Pull = NoPull>
 __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, unsigned char* smem,
                                           const int tid, const double* Dc, const Pull& pull = Pull()) {
-    static_assert(GEO != GEO_NODAL, "per-element geometry and connections");
+    static_assert(GEO == GEO_BOX, "axis-aligned elements");
     using L = BulkLayout<N, EPB, KSM>;
     constexpr int NT = EPB * KS * N * N;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
@@ -190,12 +190,12 @@ __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, un
     for (int x = tid; x < L::N2; x += NT) sD[x] = P.D[x];
     __syncthreads();
     const long long g0 = static_cast<long long>(e0) * L::N3;
-    FaceGather<face_points_per_thread<N, KS>()> G;
+    BoxFaces<box_points<KS>()> G;
     if (tid == 0) {
         bulk_issue<N, EPB, KSM>(P, e0, smem);
         pull();
     }
-    if constexpr (EARLY) gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
+    if constexpr (EARLY) gather_box<N, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
     if (!bulk_wait_tile<N, EPB, KSM>(P, smem, tid)) return;
     const int off = static_cast<int>(g0 & 1);
     const double* su = reinterpret_cast<const double*>(smem + L::u0) + off;

@@ -14,7 +14,8 @@
 // taking four planes each):
 //   1. cp.async of u_in (16-byte copies), D, geometry, connections; k lines of the
 //      element into L2;
-//   2. face phase (face_phase2, one thread per face point, six per thread);
+//   2. neighbour traces requested while the copies fly; face phase (face_phase_box:
+//      faces 0..3 through shared memory, the faces across t in registers);
 //   3. warp 0 forms the E residual from V = H (+curl H), warp 1 the H residual from
 //      V = E (-curl E).  Lane 4g + t owns nodes (i = 2t, 2t+1; j = g) of every
 //      plane k.  Per plane: the r derivatives of Vz, Vy in the original form
@@ -39,19 +40,55 @@ struct DmmaLayout8 {
     static constexpr int geo = u + 6 * 512 * 8;
     static constexpr int conn = geo + static_cast<int>(sizeof(ElemGeo));
     static constexpr int D = conn + 32;
-    static constexpr int flux = D + 64 * 8;                       // [6 faces][6 comps][64]
-    static constexpr int total = flux + 36 * 64 * 8;
+    static constexpr int flux = D + 64 * 8;                       // [4 faces][4][64]
+    // the faces across t: two pairs of lifted fluxes per thread and face
+    static constexpr int zflux = flux + flux_planes<GEO_BOX, true>() * 64 * 8;
+    static constexpr int total = zflux + 4 * 128 * 8;
 };
+
+// Neighbour values (Ex, Ey, Hx, Hy) across face f (4, 5) at the nodes (i, j) and (i+1, j)
+// of element e, i even: 16-byte loads where the two are adjacent in memory.
+__device__ __forceinline__ void dmma8_z_gather(const StageParams& P, int e, int f, int i, int j, int& zv,
+                                               double (&z)[4][2]) {
+    const long long S = P.stride;
+    int v0, v1;
+    if (P.snel[0] > 0) {
+        const int nx = P.snel[0], r = e / nx;
+        const int eB = struct_neighbour(P, e - r * nx, r % P.snel[1], r / P.snel[1], e, f);
+        v0 = eB < 0 ? kConnPEC : eB * 512 + face_local<8>(f == 4 ? 5 : 4, i, j);
+        v1 = v0 + 1;
+    } else {
+        const int cd = __ldg(P.conn + e * 6 + f);
+        v0 = conn_node<8>(cd, i, j);
+        v1 = conn_node<8>(cd, i + 1, j);
+    }
+    zv = v0;
+    if (v0 < 0) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const double* u = P.u_in + (c < 2 ? c : c + 1) * S;
+        if (v1 == v0 + 1 && (v0 & 1) == 0) {
+            const double2 w = __ldg(reinterpret_cast<const double2*>(u + v0));
+            z[c][0] = w.x;
+            z[c][1] = w.y;
+        } else {
+            z[c][0] = __ldg(u + v0);
+            z[c][1] = __ldg(u + v1);
+        }
+    }
+}
 
 // Planes K0 .. K0+NK-1 of the column phase of one warp (field src -> dst).
 template <int K0, int NK>
 __device__ __forceinline__ void dmma8_planes(const StageParams& P, const double* su, const double* V,
-                                             const double* Fl, int g, int t, int dst, double sgn,
+                                             const double* Fl, int g, int t, int dst,
                                              double d0, double d1, const double (&cx)[8][2],
                                              const double (&cy)[8][2], double rx, double sy, double tz,
-                                             long long ebase, const double* __restrict__ Dc) {
+                                             long long ebase, const double* __restrict__ Dc,
+                                             const double2* zf) {
     constexpr int N = 8, N3 = 512;
     const double A = P.a, B = P.b, DT = P.dt;
+    const int hf = dst == 0 ? 0 : 1;
     const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
     const long long S = P.stride;
 #pragma unroll
@@ -84,14 +121,45 @@ __device__ __forceinline__ void dmma8_planes(const StageParams& P, const double*
             xt0 += dk * cx[l][0]; xt1 += dk * cx[l][1];
         }
         double rhs0[3], rhs1[3];
-        rhs0[0] = sgn * (sy * zs0 - tz * yt0);
-        rhs0[1] = sgn * (tz * xt0 - rx * zr0);
-        rhs0[2] = sgn * (rx * yr0 - sy * xs0);
-        rhs1[0] = sgn * (sy * zs1 - tz * yt1);
-        rhs1[1] = sgn * (tz * xt1 - rx * zr1);
-        rhs1[2] = sgn * (rx * yr1 - sy * xs1);
-        add_lifts<N, 3>(Fl, dst, 2 * t, g, k, rhs0);
-        add_lifts<N, 3>(Fl, dst, 2 * t + 1, g, k, rhs1);
+        rhs0[0] = sy * zs0 - tz * yt0;
+        rhs0[1] = tz * xt0 - rx * zr0;
+        rhs0[2] = rx * yr0 - sy * xs0;
+        rhs1[0] = sy * zs1 - tz * yt1;
+        rhs1[1] = tz * xt1 - rx * zr1;
+        rhs1[2] = rx * yr1 - sy * xs1;
+        // faces 0..3 in face order (add_lifts_xy): the lane's first node can lie on x-,
+        // its second on x+, both on y-+
+        {
+            double x0 = 0.0, x1 = 0.0;
+            double2 y0 = make_double2(0.0, 0.0), y1 = y0;
+            if (t == 0 || t == 3) {
+                const double* F = Fl + ((t == 0 ? 3 : 1) * 4 + 2 * hf) * 64 + g + 8 * k;
+                x0 = F[0];
+                x1 = F[64];
+            }
+            if (g == 0 || g == 7) {
+                const double* F = Fl + ((g == 0 ? 0 : 2) * 4 + 2 * hf) * 64 + 2 * t + 8 * k;
+                y0 = *reinterpret_cast<const double2*>(F);
+                y1 = *reinterpret_cast<const double2*>(F + 64);
+            }
+            rhs0[0] += y1.x;
+            rhs1[0] += y1.y;
+            if (t == 0) rhs0[1] += x0;
+            if (t == 3) rhs1[1] += x0;
+            const bool xfirst = t == 3 && g == 7;
+            rhs0[2] = (rhs0[2] + y0.x) + (t == 0 ? x1 : 0.0);
+            const double xb = t == 3 ? x1 : 0.0;
+            rhs1[2] = (rhs1[2] + (xfirst ? xb : y0.y)) + (xfirst ? y0.y : xb);
+        }
+        if (k == 0 || k == 7) {
+            constexpr int last = NK == 8 ? 1 : 0;
+            const double2* z = zf + (k == 0 ? 0 : last) * 128;
+            const double2 z0 = z[0], z1 = z[512 / NK];  // 512 / NK threads
+            rhs0[0] += z0.x;
+            rhs0[1] += z0.y;
+            rhs1[0] += z1.x;
+            rhs1[1] += z1.y;
+        }
         // LSRK45 (src/device/dg_kernels.cu:404-406), FP64
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -132,13 +200,6 @@ __device__ __forceinline__ void dmma8_tile(const StageParams& P, const int e, un
         if (tid == 0 && e_ahead >= 0) prefetch_tile_l2<N3>(P, e_ahead, 1);
     }
     cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-
-    FaceGather<face_points_per_thread<N, WPF>()> G;
-    face_phase2<N, GEO_BOX, false, WPF, 1, false, false>(P, e, su, sg, sc, sflux, tid, G);
-    __syncthreads();
-    if (tid >= NT) return;
 
     const int warp = tid >> 5, lane = tid & 31;
     const int field = warp / WPF, part = warp % WPF;
@@ -147,6 +208,42 @@ __device__ __forceinline__ void dmma8_tile(const StageParams& P, const int e, un
     const int dst = 3 - src;             // residual components formed
     const double sgn = field == 0 ? 1.0 : -1.0;
     const double* V = su + src * N3;
+    // neighbour traces while the tile's copies fly: the thread's points of faces 0..3,
+    // and of its two node columns across t (a part of four planes holds one end)
+    BoxFaces<box_points<WPF>()> G;
+    gather_box<N, WPF, 1, false, false, 0, false>(P, e, nullptr, nullptr, tid, G);
+    constexpr int NZ = WPF == 1 ? 2 : 1;
+    double zn[NZ][4][2];
+    int zv[NZ];
+    if (tid < NT) {
+#pragma unroll
+        for (int s = 0; s < NZ; ++s) dmma8_z_gather(P, e, 4 + (NZ == 2 ? s : part), 2 * t, g, zv[s], zn[s]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    face_phase_box<N, false, WPF, 1, false, true>(P, e, su, sg, sc, sflux, tid, G);
+    // lifted fluxes of the lane's nodes on its faces across t (components x, y), kept in
+    // shared memory: the registers of the plane loop are all taken
+    double2* zf = reinterpret_cast<double2*>(smem + L::zflux) + tid;
+    if (tid < NT) {
+#pragma unroll
+        for (int s = 0; s < NZ; ++s) {
+            const int f = 4 + (NZ == 2 ? s : part);
+            const double* own = su + (f == 4 ? 0 : 448) + 8 * g + 2 * t;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                double v[4], j[4], F[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = zn[s][c][m];
+                box_jumps(zv[s], v, own[m], own[N3 + m], own[3 * N3 + m], own[4 * N3 + m], j);
+                box_flux<double>(sg->nrm[f][2], P.c0, sg->lift[f], j, F);
+                zf[s * 128 + m * NT] = field == 0 ? make_double2(F[0], F[1]) : make_double2(F[2], F[3]);
+            }
+        }
+    }
+    __syncthreads();
+    if (tid >= NT) return;
+
     const double d0 = sD[g + 8 * t];        // D(q = g, l = t)
     const double d1 = sD[g + 8 * (4 + t)];  // D(q = g, l = 4 + t)
     // the lane's two node columns of Vx and Vy (t derivatives)
@@ -158,13 +255,13 @@ __device__ __forceinline__ void dmma8_tile(const StageParams& P, const int e, un
         cx[l][0] = a.x; cx[l][1] = a.y;
         cy[l][0] = b.x; cy[l][1] = b.y;
     }
-    const double rx = sg->met[0], sy = sg->met[4], tz = sg->met[8];
+    const double rx = sgn * sg->met[0], sy = sgn * sg->met[4], tz = sgn * sg->met[8];
     const long long ebase = static_cast<long long>(e) * N3;
     if constexpr (WPF == 1) {
-        dmma8_planes<0, 8>(P, su, V, sflux, g, t, dst, sgn, d0, d1, cx, cy, rx, sy, tz, ebase, Dc);
+        dmma8_planes<0, 8>(P, su, V, sflux, g, t, dst, d0, d1, cx, cy, rx, sy, tz, ebase, Dc, zf);
     } else {
-        if (part == 0) dmma8_planes<0, 4>(P, su, V, sflux, g, t, dst, sgn, d0, d1, cx, cy, rx, sy, tz, ebase, Dc);
-        else dmma8_planes<4, 4>(P, su, V, sflux, g, t, dst, sgn, d0, d1, cx, cy, rx, sy, tz, ebase, Dc);
+        if (part == 0) dmma8_planes<0, 4>(P, su, V, sflux, g, t, dst, d0, d1, cx, cy, rx, sy, tz, ebase, Dc, zf);
+        else dmma8_planes<4, 4>(P, su, V, sflux, g, t, dst, d0, d1, cx, cy, rx, sy, tz, ebase, Dc, zf);
     }
 }
 

@@ -120,7 +120,17 @@ __device__ __forceinline__ int pidx(int n) {
     else return n;
 }
 
-template <int N, bool F32, int EPB, bool PIPE, bool PAD>
+// Axis-aligned elements with the field split take the reduced faces (BoxFaces below):
+// the normal components of a flux are zero there, and the faces across t stay in
+// registers, so the lifted fluxes in shared memory are [4 faces][4][N^2] instead of
+// [6 faces][6][N^2].
+template <int GEO, bool SPLIT>
+__host__ __device__ constexpr bool box_faces() { return GEO == GEO_BOX && SPLIT; }
+template <int GEO, bool SPLIT>
+__host__ __device__ constexpr int flux_planes() { return box_faces<GEO, SPLIT>() ? 16 : 36; }
+
+// FP: N^2-planes of lifted fluxes per element (flux_planes)
+template <int N, bool F32, int EPB, bool PIPE, bool PAD, int FP>
 struct Layout2 {
     static constexpr int N2 = N * N, N3 = N2 * N;
     static constexpr int EN3 = PAD ? N2 * (N + 1) : N3;                  // element stride
@@ -134,7 +144,7 @@ struct Layout2 {
     static constexpr int conn0 = geo0 + NB * geo_b;
     static constexpr int D = conn0 + NB * conn_b;
     static constexpr int flux = D + align16(N2 * 8);
-    static constexpr int uc = flux + EPB * 36 * N2 * 8;
+    static constexpr int uc = flux + EPB * FP * N2 * 8;
     // FP32-bulk: the tile's deviations [6][CS] floats, then per element the linear
     // fit ([6][4]: centre value, slopes along r, s, t) and its curl ([6]), then zl,
     // then per element the largest deviation and variation (FP64 fallback test)
@@ -289,6 +299,9 @@ __device__ __forceinline__ int struct_neighbour(const StageParams& P, int ex, in
     }
 }
 
+// The face of the neighbour that meets face f on a structured box.
+__device__ __forceinline__ int opposite_face(int f) { return f < 4 ? f ^ 2 : f ^ 1; }
+
 // Neighbour values of the face points of one thread (FPT of them): the global
 // node vB across each point (< 0: the wall code kConnPEC or kConnPMC) and its six
 // field values.
@@ -338,8 +351,7 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
             } else if (structured) {
                 eB = struct_neighbour(P, ex, ey, ez, e, f);
                 if (eB >= 0) {
-                    constexpr int opp[6] = {2, 3, 0, 1, 5, 4};
-                    vB = static_cast<long long>(eB) * N3 + face_local<N>(opp[f], p, qq);
+                    vB = static_cast<long long>(eB) * N3 + face_local<N>(opposite_face(f), p, qq);
                 }
             } else {
                 int cd;
@@ -512,6 +524,253 @@ __device__ __forceinline__ void face_phase_global(const StageParams& P, const in
     }
 }
 
+// ---- faces of axis-aligned elements (field-split forms) --------------------------------
+//
+// What bounds the stage at 5 to 9 points is the bandwidth between shared memory and
+// the register file, and a quarter of what went over it were faces.  On an
+// axis-aligned element the normal of a face is s e_d (the mesh analysis makes its other
+// components exactly zero), n x v has no component along d, and only the four
+// components across d of both traces enter the flux
+//     f_E,a = -s/2 [[H]]_b + c0/2 [[E]]_a      f_E,b = +s/2 [[H]]_a + c0/2 [[E]]_b
+//     f_H,a = +s/2 [[E]]_b + c0/2 [[H]]_a      f_H,b = -s/2 [[E]]_a + c0/2 [[H]]_b
+// with (d, a, b) cyclic.  So four values are read per trace and four fluxes kept
+// instead of six, without the branch per direction.  Faces 0..3 (across s and r) have one thread
+// a face point and go through shared memory; the faces across t (4, 5) belong to
+// the node columns: the thread that owns column (i, j) of a residual requests the
+// neighbour's four values with the other traces and keeps two lifted fluxes per face in
+// registers.  The sums of the lifted terms keep the face order 0..5.
+// B200, per step, before -> after: 64x64x32 elements of 6 points 6460 -> 5544 us, 32^3 of
+// 8 points 3272 -> 2910 us, 40^3 of 5 points 2002 -> 1644 us, 22^3 of 9 points 1860 -> 1627 us.
+
+// What one thread holds of the faces: FPT points of faces 0..3 and its column's two
+// points across t: neighbour node (< 0: wall code) and the four neighbour values.
+template <int FPT>
+struct BoxFaces {
+    double nb[FPT][4];
+    double zn[2][4];
+    int vB[FPT];
+    int zv[2];
+};
+
+// Points of faces 0..3 per thread.
+template <int KS>
+__host__ __device__ constexpr int box_points() { return (4 + KS - 1) / KS; }
+
+template <int N, int GEO, int KS, bool SPLIT>
+using FaceRegs = typename std::conditional<box_faces<GEO, SPLIT>(), BoxFaces<box_points<KS>()>,
+                                           FaceGather<face_points_per_thread<N, KS>()>>::type;
+
+// Neighbour node of face point (f, p, q) of element e, or the wall code (< 0); sc: the
+// element's six connection codes (shared or global memory).  Node indices fit an int
+// (at most 2^31 - 1 nodes).
+template <int N>
+__device__ __forceinline__ int conn_node(int cd, int p, int q) {
+    if (cd < 0) return cd;
+    const int o = cd & 7;
+    int a = (o & 4) ? q : p;
+    int b = (o & 4) ? p : q;
+    if (o & 1) a = N - 1 - a;
+    if (o & 2) b = N - 1 - b;
+    return (cd >> 6) * (N * N * N) + face_local<N>((cd >> 3) & 7, a, b);
+}
+
+// Fill a BoxFaces.  FROM_SMEM: the tile is resident (connections from sc, neighbours
+// inside the tile from su); otherwise only global memory is read (and neighbours follow
+// from the box structure where there is one), so it may run while the tile's copies
+// are in flight.
+// ZF: the points across t as well.
+template <int N, int KS, int EPB, bool PAD, bool FROM_SMEM, int CSX = 0, bool ZF = true>
+__device__ __forceinline__ void gather_box(const StageParams& P, const int e0, const double* su,
+                                           const int* sc, const int tid, BoxFaces<box_points<KS>()>& G) {
+    constexpr int N2 = N * N, N3 = N2 * N;
+    constexpr int TPE = KS * N2;
+    constexpr int CS = CSX ? CSX : EPB * (PAD ? N2 * (N + 1) : N3);
+    constexpr int FPT = box_points<KS>();
+    const int team = tid / TPE;
+    const int lt = tid - team * TPE;
+    const int h = lt / N2, pq = lt - h * N2;
+    const int p = pq % N, q = pq / N;
+    const int nvalid = min(EPB, P.nelt - e0);
+    const int e = e0 + team;
+    const long long S = P.stride;
+    if (team >= nvalid) {
+#pragma unroll
+        for (int x = 0; x < FPT; ++x) G.vB[x] = kConnPEC;
+        G.zv[0] = G.zv[1] = kConnPEC;
+        return;
+    }
+    const bool structured = !FROM_SMEM && P.snel[0] > 0;
+    int ex = 0, ey = 0, ez = 0;
+    if (structured) {
+        ex = e % P.snel[0];
+        const int r = e / P.snel[0];
+        ey = r % P.snel[1];
+        ez = r / P.snel[1];
+    }
+    auto node = [&](int f) -> int {
+        if (structured) {
+            const int eB = struct_neighbour(P, ex, ey, ez, e, f);
+            return eB < 0 ? kConnPEC : eB * N3 + face_local<N>(opposite_face(f), p, q);
+        }
+        int cd;
+        if constexpr (FROM_SMEM) cd = sc[team * 6 + f];
+        else cd = __ldg(P.conn + e * 6 + f);
+        return conn_node<N>(cd, p, q);
+    };
+    auto fetch = [&](int vB, int ca, int cb, double (&v)[4]) {
+        if constexpr (FROM_SMEM) {
+            const int l = vB - e0 * N3;
+            if (l >= 0 && l < nvalid * N3) {
+                const int el = l / N3;
+                const int x = el * (PAD ? N2 * (N + 1) : N3) + pidx<N, PAD>(l - el * N3);
+                v[0] = su[ca * CS + x];
+                v[1] = su[cb * CS + x];
+                v[2] = su[(3 + ca) * CS + x];
+                v[3] = su[(3 + cb) * CS + x];
+                return;
+            }
+        }
+        const double* u = P.u_in + vB;
+        v[0] = __ldg(u + ca * S);
+        v[1] = __ldg(u + cb * S);
+        v[2] = __ldg(u + (3 + ca) * S);
+        v[3] = __ldg(u + (3 + cb) * S);
+    };
+#pragma unroll
+    for (int x = 0; x < FPT; ++x) {
+        const int f = x * KS + h;  // odd: across r (a, b = y, z), even: across s (z, x)
+        G.vB[x] = kConnPEC;
+        if (KS * FPT == 4 || f < 4) {
+            G.vB[x] = node(f);
+            if (G.vB[x] >= 0) fetch(G.vB[x], (f & 1) ? 1 : 2, (f & 1) ? 2 : 0, G.nb[x]);
+        }
+    }
+    if constexpr (ZF) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            G.zv[s] = node(4 + s);
+            if (G.zv[s] >= 0) fetch(G.zv[s], 0, 1, G.zn[s]);
+        }
+    }
+}
+
+// Jumps of the four components of one face point: nb - own, or the wall's mirror (PEC:
+// [[E]] = -2E, [[H]] = 0; PMC: [[E]] = 0, [[H]] = -2H).
+__device__ __forceinline__ void box_jumps(int vB, const double (&nb)[4], double ea, double eb, double ha,
+                                          double hb, double (&j)[4]) {
+    if (vB >= 0) {
+        j[0] = nb[0] - ea; j[1] = nb[1] - eb; j[2] = nb[2] - ha; j[3] = nb[3] - hb;
+    } else if (vB == kConnPMC) {
+        j[0] = 0.0; j[1] = 0.0; j[2] = -2.0 * ha; j[3] = -2.0 * hb;
+    } else {
+        j[0] = -2.0 * ea; j[1] = -2.0 * eb; j[2] = 0.0; j[3] = 0.0;
+    }
+}
+
+// The four lifted fluxes of one face point (see above); nd = s, the normal's one
+// component (0 on a degenerate face: no flux).
+template <typename TC>
+__device__ __forceinline__ void box_flux(double nd, double c0, double lift, const double (&j)[4],
+                                         double (&F)[4]) {
+    const TC hs = static_cast<TC>(0.5 * nd), hc = static_cast<TC>(0.5 * c0 * (nd * nd));
+    const TC ea = static_cast<TC>(j[0]), eb = static_cast<TC>(j[1]);
+    const TC ha = static_cast<TC>(j[2]), hb = static_cast<TC>(j[3]);
+    F[0] = lift * static_cast<double>(hc * ea - hs * hb);
+    F[1] = lift * static_cast<double>(hs * ha + hc * eb);
+    F[2] = lift * static_cast<double>(hs * eb + hc * ha);
+    F[3] = lift * static_cast<double>(hc * hb - hs * ea);
+}
+
+// Face phase over faces 0..3: lifted fluxes into sflux [team][face][4][N^2].
+template <int N, bool F32, int KS, int EPB, bool PAD, bool EARLY, int CSX = 0>
+__device__ __forceinline__ void face_phase_box(const StageParams& P, const int e0, const double* su,
+                                               const ElemGeo* sg, const int* sc, double* sflux, const int tid,
+                                               BoxFaces<box_points<KS>()>& G) {
+    using TC = typename std::conditional<F32, float, double>::type;
+    constexpr int N2 = N * N;
+    constexpr int EN3 = (PAD ? N + 1 : N) * N2;
+    constexpr int TPE = KS * N2;
+    constexpr int CS = CSX ? CSX : EPB * EN3;
+    constexpr int FPT = box_points<KS>();
+    if constexpr (!EARLY) gather_box<N, KS, EPB, PAD, true, CSX>(P, e0, su, sc, tid, G);
+    const int team = tid / TPE;
+    if (team >= min(EPB, P.nelt - e0)) return;
+    const int lt = tid - team * TPE;
+    const int h = lt / N2, pq = lt - h * N2;
+    const int p = pq % N, q = pq / N;
+    const double* U = su + team * EN3;
+#pragma unroll
+    for (int x = 0; x < FPT; ++x) {
+        const int f = x * KS + h;
+        if (KS * FPT != 4 && f >= 4) break;
+        const int ca = (f & 1) ? 1 : 2, cb = (f & 1) ? 2 : 0;
+        const double* own = U + pidx<N, PAD>(face_local<N>(f, p, q));
+        double j[4], F[4];
+        box_jumps(G.vB[x], G.nb[x], own[ca * CS], own[cb * CS], own[(3 + ca) * CS], own[(3 + cb) * CS], j);
+        box_flux<TC>(sg[team].nrm[f][(f & 1) ? 0 : 1], P.c0, sg[team].lift[f], j, F);
+        double* out = sflux + (team * 4 + f) * 4 * N2 + pq;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) out[c * N2] = F[c];
+    }
+}
+
+// face_phase_box from global memory only (own traces, normals and lifts too), while the
+// tile's copies are in flight.
+template <int N, bool F32, int KS, int EPB>
+__device__ __forceinline__ void face_phase_box_global(const StageParams& P, const int e0, double* sflux,
+                                                      const int tid, BoxFaces<box_points<KS>()>& G) {
+    using TC = typename std::conditional<F32, float, double>::type;
+    constexpr int N2 = N * N, N3 = N2 * N;
+    constexpr int TPE = KS * N2;
+    constexpr int FPT = box_points<KS>();
+    gather_box<N, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
+    const int team = tid / TPE;
+    if (team >= min(EPB, P.nelt - e0)) return;
+    const int lt = tid - team * TPE;
+    const int h = lt / N2, pq = lt - h * N2;
+    const int p = pq % N, q = pq / N;
+    const long long S = P.stride;
+    const ElemGeo* Gp = P.geo + e0 + team;
+#pragma unroll
+    for (int x = 0; x < FPT; ++x) {
+        const int f = x * KS + h;
+        if (KS * FPT != 4 && f >= 4) break;
+        const int ca = (f & 1) ? 1 : 2, cb = (f & 1) ? 2 : 0;
+        const double* own = P.u_in + static_cast<long long>(e0 + team) * N3 + face_local<N>(f, p, q);
+        double j[4], F[4];
+        box_jumps(G.vB[x], G.nb[x], __ldg(own + ca * S), __ldg(own + cb * S), __ldg(own + (3 + ca) * S),
+                  __ldg(own + (3 + cb) * S), j);
+        box_flux<TC>(__ldg(&Gp->nrm[f][(f & 1) ? 0 : 1]), P.c0, __ldg(&Gp->lift[f]), j, F);
+        double* out = sflux + (team * 4 + f) * 4 * N2 + pq;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) out[c * N2] = F[c];
+    }
+}
+
+// Lifted terms of faces 0..3 at node (i, j, k) for the residual of field hf (0: E,
+// 1: H), in face order: y- (0), x+ (1), y+ (2), x- (3).  A node lies on at most one x and
+// one y face; only the z component gets both, and only at x+ with y+ does x come first.
+template <int N>
+__device__ __forceinline__ void add_lifts_xy(const double* Fl, int hf, int i, int j, int k, double* rhs) {
+    constexpr int N2 = N * N;
+    const bool onx = i == 0 || i == N - 1, ony = j == 0 || j == N - 1;
+    double x0 = 0.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
+    if (onx) {
+        const double* F = Fl + ((i == 0 ? 3 : 1) * 4 + 2 * hf) * N2 + j + N * k;
+        x0 = F[0];   // y component
+        x1 = F[N2];  // z component
+    }
+    if (ony) {
+        const double* F = Fl + ((j == 0 ? 0 : 2) * 4 + 2 * hf) * N2 + i + N * k;
+        y0 = F[0];   // z component
+        y1 = F[N2];  // x component
+    }
+    const bool xfirst = i == N - 1 && j == N - 1;
+    rhs[0] += y1;
+    rhs[1] += x0;
+    rhs[2] = (rhs[2] + (xfirst ? x1 : y0)) + (xfirst ? y0 : x1);
+}
+
 // Barrier of the threads that share one tile (the whole block in every form here).
 struct CtaBar {
     __device__ __forceinline__ void sync() const { __syncthreads(); }
@@ -558,7 +817,7 @@ template <int N, int GEO, bool F32, int KS, int EPB, bool SPLIT, bool PAD, bool 
 __device__ __forceinline__ void compute2(const StageParams& P, const int e0, const double* su,
                                          const ElemGeo* sg, const int* sc, const double* sD,
                                          double* sflux, unsigned char* smem_uc, const int tid,
-                                         FaceGather<face_points_per_thread<N, KS>()>& G,
+                                         FaceRegs<N, GEO, KS, SPLIT>& G,
                                          const double* __restrict__ Dc = nullptr, Bar bar = Bar(),
                                          const double* sk = nullptr) {
     using TC = typename std::conditional<F32, float, double>::type;
@@ -570,6 +829,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     constexpr int NT = EPB * TPE;
     constexpr int KPT = (N + KS - 1) / KS;
     constexpr int CS = CSX ? CSX : EPB * EN3;
+    constexpr bool BOXF = box_faces<GEO, SPLIT>();
     static_assert(CSX == 0 || !F32, "tiles with slack: FP64 only");
     static_assert(!KSM || (!PAD && !F32), "k in shared memory: unpadded FP64 tiles");
     static_assert(!SPLIT || KS == 1 || KS == 2, "the field split: one or two threads per column");
@@ -668,8 +928,10 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     }
 
     // ---- face phase (unless the caller ran it from global memory) -------------------
-    if constexpr (!FACEDONE)
-        face_phase2<N, GEO, F32, KS, EPB, PAD, EARLY, CSX>(P, e0, su, sg, sc, sflux, tid, G);
+    if constexpr (!FACEDONE) {
+        if constexpr (BOXF) face_phase_box<N, F32, KS, EPB, PAD, EARLY, CSX>(P, e0, su, sg, sc, sflux, tid, G);
+        else face_phase2<N, GEO, F32, KS, EPB, PAD, EARLY, CSX>(P, e0, su, sg, sc, sflux, tid, G);
+    }
     bar.sync();
 
     if constexpr (F32 && GEO != GEO_NODAL) {
@@ -707,7 +969,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     if (!active) return;
     const TC* U = s_uc + team * EN3;
     const double* Uf = su + team * EN3;
-    const double* Fl = sflux + team * 36 * N2;
+    const double* Fl = sflux + team * flux_planes<GEO, SPLIT>() * N2;
     TC Dr[N], Ds[N];
 #pragma unroll
     for (int l = 0; l < N; ++l) {
@@ -757,6 +1019,31 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         for (int c = 0; c < NC; ++c)
 #pragma unroll
             for (int l = 0; l < N; ++l) col[c][l] = V[c * CS + i + RP * j + PP * l];
+        // the lifted fluxes of the faces across t at this column, components x and y of
+        // this residual (box_flux with d = z, a = x, b = y)
+        double zf[2][2];
+        if constexpr (BOXF) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int m = i + RP * j + (s ? PP * (N - 1) : 0);
+                const double* own = Uf + m;
+                double sx, sy;  // the differentiated field's trace: in registers when FP64
+                if constexpr (F32) {
+                    sx = own[src * CS];
+                    sy = own[(src + 1) * CS];
+                } else {
+                    sx = static_cast<double>(col[0][s ? N - 1 : 0]);
+                    sy = static_cast<double>(col[1][s ? N - 1 : 0]);
+                }
+                const double dx = own[dst * CS], dy = own[(dst + 1) * CS];
+                double jmp[4], F[4];
+                box_jumps(G.zv[s], G.zn[s], hf == 0 ? dx : sx, hf == 0 ? dy : sy, hf == 0 ? sx : dx,
+                          hf == 0 ? sy : dy, jmp);
+                box_flux<TC>(sg[team].nrm[4 + s][2], P.c0, sg[team].lift[4 + s], jmp, F);
+                zf[s][0] = hf == 0 ? F[0] : F[2];
+                zf[s][1] = hf == 0 ? F[1] : F[3];
+            }
+        }
         // CONSTD (plane loop unrolled): k of the next plane is requested before this
         // plane's stores, which the compiler may not move a later load above, so its
         // latency overlaps the sums (B200: 3-5% faster at N = 7, 9; the rolled loop
@@ -866,7 +1153,13 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
 #pragma unroll
                 for (int c = 0; c < 3; ++c) rhs[c] += s_lin[team * LIN + 24 + dst + c];
             }
-            add_lifts<N, 3>(Fl, dst, i, j, k, rhs);
+            if constexpr (BOXF) {
+                add_lifts_xy<N>(Fl, hf, i, j, k, rhs);
+                if (k == 0) { rhs[0] += zf[0][0]; rhs[1] += zf[0][1]; }
+                if (k == N - 1) { rhs[0] += zf[1][0]; rhs[1] += zf[1][1]; }
+            } else {
+                add_lifts<N, 3>(Fl, dst, i, j, k, rhs);
+            }
             // LSRK45 (src/device/dg_kernels.cu:404-406), FP64
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -986,7 +1279,7 @@ template <int N, int GEO, bool F32, int KS, int EPB, int MINB, bool PIPE, bool S
 __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     stage2_kernel(const __grid_constant__ StageParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
-    using L = Layout2<N, F32, EPB, PIPE, PAD>;
+    using L = Layout2<N, F32, EPB, PIPE, PAD, flux_planes<GEO, SPLIT>()>;
     constexpr int NT = EPB * KS * N * N;
     const int tid = threadIdx.x;
     const int ntiles = (P.nelt + EPB - 1) / EPB;
@@ -999,11 +1292,15 @@ __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     auto sg = [&](int b) { return reinterpret_cast<ElemGeo*>(smem + L::geo0 + b * L::geo_b); };
     auto sc = [&](int b) { return reinterpret_cast<int*>(smem + L::conn0 + b * L::conn_b); };
     static_assert(!((EARLY || FACEFIRST) && PIPE), "early forms belong to the one-tile form");
-    FaceGather<face_points_per_thread<N, KS>()> G;
+    FaceRegs<N, GEO, KS, SPLIT> G;
     issue2<N, GEO, EPB, NT, PAD>(P, t * EPB, su(0), sg(0), sc(0), tid);
     cp_async_commit();
     if constexpr (!PIPE) {
-        if constexpr (FACEFIRST) face_phase_global<N, GEO, F32, KS, EPB>(P, t * EPB, sflux, tid);
+        if constexpr (FACEFIRST && box_faces<GEO, SPLIT>())
+            face_phase_box_global<N, F32, KS, EPB>(P, t * EPB, sflux, tid, G);
+        else if constexpr (FACEFIRST) face_phase_global<N, GEO, F32, KS, EPB>(P, t * EPB, sflux, tid);
+        else if constexpr (EARLY && box_faces<GEO, SPLIT>())
+            gather_box<N, KS, EPB, PAD, false>(P, t * EPB, nullptr, nullptr, tid, G);
         else if constexpr (EARLY) gather2<N, GEO, KS, EPB, PAD, false>(P, t * EPB, nullptr, nullptr, tid, G);
         cp_async_wait<0>();
         __syncthreads();
@@ -1031,7 +1328,7 @@ template <int N, int GEO, bool F32, int KS, int EPB, int MINB, bool PIPE, bool S
           bool CONSTD, bool EARLY, bool FACEFIRST, bool DSMEM>
 cudaError_t launch2(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
     constexpr int threads = EPB * KS * N * N;
-    constexpr int smem = Layout2<N, F32, EPB, PIPE, PAD>::total;
+    constexpr int smem = Layout2<N, F32, EPB, PIPE, PAD, flux_planes<GEO, SPLIT>()>::total;
     auto kern = stage2_kernel<N, GEO, F32, KS, EPB, MINB, PIPE, SPLIT, PAD, CONSTD, EARLY, FACEFIRST, DSMEM>;
     if (cfg) *cfg = StageConfig{KS, EPB, threads, smem, 0, MINB};
     // resident blocks on the device, per kernel and device (0: not yet set up)
