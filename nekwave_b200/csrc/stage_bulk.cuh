@@ -92,7 +92,7 @@ __device__ __forceinline__ void report(const StageParams& P, int code) {
 
 // Shared-memory layout of one tile: u_in (and with KSM k) [6][CSR] doubles with
 // slack, geometry, connections, D, the lifted fluxes, the mbarrier and a flag.
-template <int N, int EPB, bool KSM>
+template <int N, int EPB, bool KSM, int GEO = GEO_BOX>
 struct BulkLayout {
     static constexpr int N2 = N * N, N3 = N2 * N;
     static constexpr int CSR = (EPB * N3 + 2 + 1) / 2 * 2;
@@ -100,12 +100,12 @@ struct BulkLayout {
     static constexpr int u0 = 0;
     static constexpr int k0 = u0 + tile_u;
     static constexpr int geo0 = k0 + (KSM ? tile_u : 0);
-    static constexpr int geo_b = EPB * static_cast<int>(sizeof(ElemGeo));
+    static constexpr int geo_b = GEO == GEO_NODAL ? 0 : EPB * static_cast<int>(sizeof(ElemGeo));
     static constexpr int conn0 = geo0 + geo_b;
     static constexpr int conn_b = align16((EPB * 6 + 6) * 4);
     static constexpr int D = conn0 + conn_b;
     static constexpr int flux0 = D + align16(N2 * 8);
-    static constexpr int bar = flux0 + EPB * flux_planes<GEO_BOX, true>() * N2 * 8;
+    static constexpr int bar = flux0 + EPB * flux_planes<GEO, true>() * N2 * 8;
     static constexpr int flag = bar + 8;
     static constexpr int total = flag + 16;
 };
@@ -113,9 +113,9 @@ struct BulkLayout {
 // Thread 0's part of a tile load: the tile's u_in (and with KSM its k; otherwise k's
 // lines are prefetched into L2), geometry and connections as bulk copies that
 // complete on the mbarrier at smem + L::bar, which must be initialised.
-template <int N, int EPB, bool KSM>
+template <int N, int EPB, bool KSM, int GEO>
 __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, unsigned char* smem) {
-    using L = BulkLayout<N, EPB, KSM>;
+    using L = BulkLayout<N, EPB, KSM, GEO>;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     const long long S = P.stride;
     const long long g0 = static_cast<long long>(e0) * L::N3;
@@ -127,7 +127,7 @@ __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, u
     const unsigned cb = static_cast<unsigned>((ca1 - ca0) * 4);
     const unsigned gb = static_cast<unsigned>(nvalid * sizeof(ElemGeo));
     const bool kread = (P.kio & kKRead) != 0;
-    mbar_arrive_expect_tx(bar, (KSM && kread ? 12 : 6) * ub + gb + cb);
+    mbar_arrive_expect_tx(bar, (KSM && kread ? 12 : 6) * ub + (GEO == GEO_NODAL ? 0 : gb + cb));
     double* su = reinterpret_cast<double*>(smem + L::u0);
 #pragma unroll
     for (int c = 0; c < 6; ++c) bulk_g2s(su + c * L::CSR, P.u_in + c * S + a0, ub, bar);
@@ -141,16 +141,22 @@ __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, u
 #pragma unroll
         for (int c = 0; c < 6; ++c) bulk_prefetch_l2(P.k + c * S + a0, ub);
     }
-    bulk_g2s(smem + L::geo0, P.geo + e0, gb, bar);
-    bulk_g2s(smem + L::conn0, P.conn + ca0, cb, bar);
+    if constexpr (GEO == GEO_NODAL) {
+        // the column phase reads the metrics plane by plane: into L2 meanwhile
+#pragma unroll
+        for (int c = 0; c < 9; ++c) bulk_prefetch_l2(P.met_n + c * S + a0, ub);
+    } else {
+        bulk_g2s(smem + L::geo0, P.geo + e0, gb, bar);
+        bulk_g2s(smem + L::conn0, P.conn + ca0, cb, bar);
+    }
 }
 
 // Every thread's wait for the tile issued by bulk_issue: true when it is resident.
 // On expiry thread 0 records the code, waits once more (bounded) for the copies so
 // that none lands in a finished block, and every thread gets false.
-template <int N, int EPB, bool KSM>
+template <int N, int EPB, bool KSM, int GEO>
 __device__ __forceinline__ bool bulk_wait_tile(const StageParams& P, unsigned char* smem, const int tid) {
-    using L = BulkLayout<N, EPB, KSM>;
+    using L = BulkLayout<N, EPB, KSM, GEO>;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     int* flag = reinterpret_cast<int*>(smem + L::flag);
     if (tid == 0) *flag = mbar_wait(bar, 0) ? 1 : 0;
@@ -178,8 +184,7 @@ template <int N, int GEO, int KS, int EPB, bool CONSTD, bool DSMEM, bool KSM, bo
           bool VROW = false, bool ILP2 = false, class Pull = NoPull>
 __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, unsigned char* smem,
                                           const int tid, const double* Dc, const Pull& pull = Pull()) {
-    static_assert(GEO == GEO_BOX, "axis-aligned elements");
-    using L = BulkLayout<N, EPB, KSM>;
+    using L = BulkLayout<N, EPB, KSM, GEO>;
     constexpr int NT = EPB * KS * N * N;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     double* sD = reinterpret_cast<double*>(smem + L::D);
@@ -190,13 +195,14 @@ __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, un
     for (int x = tid; x < L::N2; x += NT) sD[x] = P.D[x];
     __syncthreads();
     const long long g0 = static_cast<long long>(e0) * L::N3;
-    BoxFaces<box_points<KS>()> G;
+    FaceRegs<N, GEO, KS, true> G;
     if (tid == 0) {
-        bulk_issue<N, EPB, KSM>(P, e0, smem);
+        bulk_issue<N, EPB, KSM, GEO>(P, e0, smem);
         pull();
     }
-    if constexpr (EARLY) gather_box<N, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
-    if (!bulk_wait_tile<N, EPB, KSM>(P, smem, tid)) return;
+    if constexpr (EARLY && GEO == GEO_BOX) gather_box<N, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
+    else if constexpr (EARLY) gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
+    if (!bulk_wait_tile<N, EPB, KSM, GEO>(P, smem, tid)) return;
     const int off = static_cast<int>(g0 & 1);
     const double* su = reinterpret_cast<const double*>(smem + L::u0) + off;
     const double* sk = KSM ? reinterpret_cast<const double*>(smem + L::k0) + off : nullptr;
@@ -261,7 +267,7 @@ __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
 template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
           bool ZCOL, bool VROW, bool ILP2, int AHEAD = 0>
 cudaError_t launch_bulk(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
-    using L = BulkLayout<N, EPB, KSM>;
+    using L = BulkLayout<N, EPB, KSM, GEO>;
     constexpr int threads = EPB * KS * N * N;
     auto kern = stage_bulk_kernel<N, GEO, KS, EPB, MINB, CONSTD, DSMEM, KSM, EARLY, ZCOL, VROW, ILP2, AHEAD>;
     if (cfg) *cfg = StageConfig{KS, EPB, threads, L::total, KSM ? 1 : 0, MINB};
@@ -270,6 +276,36 @@ cudaError_t launch_bulk(const StageParams* p, cudaStream_t st, StageConfig* cfg)
     if (!p) return cudaSuccess;
     kern<<<(p->nelt + EPB - 1) / EPB, threads, L::total, st>>>(*p);
     return cudaGetLastError();
+}
+
+// Shapes of the general classes (affine and per-node geometry) in FP64: the bulk-copy
+// tile with the field split, k in shared memory and the face data requested while the
+// copies fly.  Bound by latency and the shared pipe: three derivatives of three
+// components per field (18 sums a node instead of 12) and, per node, nine metrics
+// (72 B on top of the 192), which thread 0 pulls into L2 and the column phase requests
+// one plane ahead.  MINB leaves the registers that takes; CD: t-derivative coefficients from
+// the parameter bank with the plane loop unrolled (at 7 and 8 points only where the
+// metrics do not need the registers, CDN / CDA).  From a sweep of four shapes per N
+// on 1.5 to 1.7 M nodes.  B200, per step, before (per-thread copies, k and metrics
+// read from L2 in the plane loop) -> now, per-node class: 17x15x19 elements of 6 points
+// 572 -> 375 us, 26x26x24 of 4 points 504 -> 323 us, 12x13x12 of 8 points 452 -> 366 us;
+// affine class, 16x16x12 of 8 points 449 -> 378 us.
+template <int N> struct GeneralShape;
+template <> struct GeneralShape<2> { static constexpr int EPB = 8, MINB = 6, CDN = 1, CDA = 1; };
+template <> struct GeneralShape<3> { static constexpr int EPB = 8, MINB = 3, CDN = 1, CDA = 1; };
+template <> struct GeneralShape<4> { static constexpr int EPB = 4, MINB = 3, CDN = 1, CDA = 1; };
+template <> struct GeneralShape<5> { static constexpr int EPB = 1, MINB = 8, CDN = 1, CDA = 1; };
+template <> struct GeneralShape<6> { static constexpr int EPB = 1, MINB = 4, CDN = 1, CDA = 1; };
+template <> struct GeneralShape<7> { static constexpr int EPB = 1, MINB = 3, CDN = 0, CDA = 1; };
+template <> struct GeneralShape<8> { static constexpr int EPB = 1, MINB = 3, CDN = 0, CDA = 1; };
+template <> struct GeneralShape<9> { static constexpr int EPB = 1, MINB = 2, CDN = 1, CDA = 1; };
+template <> struct GeneralShape<10> { static constexpr int EPB = 1, MINB = 1, CDN = 1, CDA = 1; };
+
+template <int N, int GEO>
+cudaError_t launch_general(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
+    using Sh = GeneralShape<N>;
+    constexpr bool cd = (GEO == GEO_NODAL ? Sh::CDN : Sh::CDA) != 0;
+    return launch_bulk<N, GEO, 2, Sh::EPB, Sh::MINB, cd, false, true, true, false, false, false>(p, st, cfg);
 }
 
 }  // namespace stage

@@ -59,7 +59,9 @@ inline int shape_index(int geo, int f32, int variant) {
 // vid: shape index (shape_index)
 template <int GEO, bool F32, int I>
 cudaError_t launch_variant(int vid, const StageParams* p, cudaStream_t st, StageConfig* cfg) {
-    if constexpr (I < kNumShapes) {
+    if constexpr (GEO != GEO_BOX && !F32) {
+        return launch_general<NWB_N, GEO>(p, st, cfg);
+    } else if constexpr (I < kNumShapes) {
         if (vid == I) {
             constexpr Shape v = kShapes[I];
             if constexpr (v.alg == 1) {

@@ -305,10 +305,11 @@ __device__ __forceinline__ int opposite_face(int f) { return f < 4 ? f ^ 2 : f ^
 // Neighbour values of the face points of one thread (FPT of them): the global
 // node vB across each point (< 0: the wall code kConnPEC or kConnPMC) and its six
 // field values.
-template <int FPT>
+template <int FPT, bool NODAL = false>
 struct FaceGather {
     double nb[FPT][6];
     long long vB[FPT];
+    double nl[NODAL ? FPT : 1][4];  // per-node class: normal and lift of each point
 };
 
 // Fill a FaceGather.  FROM_SMEM: the tile is resident (connections from sc,
@@ -316,7 +317,8 @@ struct FaceGather {
 // it may run while the tile's copies are still in flight.
 template <int N, int GEO, int KS, int EPB, bool PAD, bool FROM_SMEM, int FPT, int CSX = 0>
 __device__ __forceinline__ void gather2(const StageParams& P, const int e0, const double* su,
-                                        const int* sc, const int tid, FaceGather<FPT>& G) {
+                                        const int* sc, const int tid,
+                                        FaceGather<FPT, GEO == GEO_NODAL>& G) {
     constexpr int N2 = N * N, N3 = N2 * N;
     constexpr int TPE = KS * N2;
     // component stride of the shared tile (CSX: a tile with slack between components)
@@ -346,7 +348,12 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
             const int p = pq % N, qq = pq / N;
             int eB = -1;
             if constexpr (GEO == GEO_NODAL) {
-                vB = P.fplus[(static_cast<long long>(e) * 6 + f) * N2 + pq];
+                const long long g = (static_cast<long long>(e) * 6 + f) * N2 + pq;
+                vB = __ldg(P.fplus + g);
+                G.nl[q][0] = __ldg(P.fnrm + g);
+                G.nl[q][1] = __ldg(P.fnrm + P.nfp + g);
+                G.nl[q][2] = __ldg(P.fnrm + 2 * P.nfp + g);
+                G.nl[q][3] = __ldg(P.flift + g);
                 if (vB >= 0) eB = static_cast<int>(vB / N3);
             } else if (structured) {
                 eB = struct_neighbour(P, ex, ey, ez, e, f);
@@ -403,7 +410,7 @@ template <int N, int GEO, bool F32, int KS, int EPB, bool PAD, bool EARLY, int C
 __device__ __forceinline__ void face_phase2(const StageParams& P, const int e0, const double* su,
                                             const ElemGeo* sg, const int* sc, double* sflux,
                                             const int tid,
-                                            FaceGather<face_points_per_thread<N, KS>()>& G) {
+                                            FaceGather<face_points_per_thread<N, KS>(), GEO == GEO_NODAL>& G) {
     using TC = typename std::conditional<F32, float, double>::type;
     constexpr int N2 = N * N;
     constexpr int RP = PAD ? N + 1 : N;
@@ -431,11 +438,10 @@ __device__ __forceinline__ void face_phase2(const StageParams& P, const int e0, 
             const double Hxm = U[3 * CS + m], Hym = U[4 * CS + m], Hzm = U[5 * CS + m];
             double nxd, nyd, nzd, lift;
             if constexpr (GEO == GEO_NODAL) {
-                const long long g = (static_cast<long long>(e) * 6 + f) * N2 + pq;
-                nxd = P.fnrm[g];
-                nyd = P.fnrm[P.nfp + g];
-                nzd = P.fnrm[2 * P.nfp + g];
-                lift = P.flift[g];
+                nxd = G.nl[q][0];
+                nyd = G.nl[q][1];
+                nzd = G.nl[q][2];
+                lift = G.nl[q][3];
             } else {
                 const ElemGeo& G = sg[team];
                 nxd = G.nrm[f][0];
@@ -475,7 +481,7 @@ __device__ __forceinline__ void face_phase_global(const StageParams& P, const in
     const int e = e0 + team;
     if (team >= min(EPB, P.nelt - e0)) return;
     const long long S = P.stride;
-    FaceGather<FPT> G;
+    FaceGather<FPT, GEO == GEO_NODAL> G;
     gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
     double own[FPT][6];
 #pragma unroll
@@ -497,11 +503,10 @@ __device__ __forceinline__ void face_phase_global(const StageParams& P, const in
         const int pq = fp - f * N2;
         double nxd, nyd, nzd, lift;
         if constexpr (GEO == GEO_NODAL) {
-            const long long gf = (static_cast<long long>(e) * 6 + f) * N2 + pq;
-            nxd = __ldg(P.fnrm + gf);
-            nyd = __ldg(P.fnrm + P.nfp + gf);
-            nzd = __ldg(P.fnrm + 2 * P.nfp + gf);
-            lift = __ldg(P.flift + gf);
+            nxd = G.nl[q][0];
+            nyd = G.nl[q][1];
+            nzd = G.nl[q][2];
+            lift = G.nl[q][3];
         } else {
             const ElemGeo* Gp = P.geo + e;
             nxd = __ldg(&Gp->nrm[f][0]);
@@ -558,7 +563,7 @@ __host__ __device__ constexpr int box_points() { return (4 + KS - 1) / KS; }
 
 template <int N, int GEO, int KS, bool SPLIT>
 using FaceRegs = typename std::conditional<box_faces<GEO, SPLIT>(), BoxFaces<box_points<KS>()>,
-                                           FaceGather<face_points_per_thread<N, KS>()>>::type;
+                                           FaceGather<face_points_per_thread<N, KS>(), GEO == GEO_NODAL>>::type;
 
 // Neighbour node of face point (f, p, q) of element e, or the wall code (< 0); sc: the
 // element's six connection codes (shared or global memory).  Node indices fit an int
@@ -1049,6 +1054,13 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         // latency overlaps the sums (B200: 3-5% faster at N = 7, 9; the rolled loop
         // is faster without it)
         double knext[3];
+        // per-node class: the metrics of the next plane are requested while this plane's
+        // sums run, for the same reason
+        double mnext[GEO == GEO_NODAL ? 9 : 1];
+        if constexpr (GEO == GEO_NODAL) {
+#pragma unroll
+            for (int c = 0; c < 9; ++c) mnext[c] = __ldg(P.met_n + c * S + ebase + i + N * j);
+        }
         // KSM: k staged in shared memory with the tile's layout (unpadded)
         const double* Kf = KSM ? sk + team * EN3 : nullptr;
         if constexpr (CONSTD) {
@@ -1077,6 +1089,15 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
                     kold[c] = !kread ? 0.0 : (KSM ? Kf[(dst + c) * CS + ms] : __ldcg(P.k + (dst + c) * S + g));
+            }
+            double mnow[GEO == GEO_NODAL ? 9 : 1];
+            if constexpr (GEO == GEO_NODAL) {
+#pragma unroll
+                for (int c = 0; c < 9; ++c) mnow[c] = mnext[c];
+                if (k + 1 < N) {
+#pragma unroll
+                    for (int c = 0; c < 9; ++c) mnext[c] = __ldg(P.met_n + c * S + g + N2);
+                }
             }
             double rhs[3];
             if constexpr (GEO == GEO_BOX) {
@@ -1132,11 +1153,9 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
                 }
                 TX rx, sx, tx, ry, sy, ty, rz, sz, tz;
                 if constexpr (GEO == GEO_NODAL) {
-                    rx = static_cast<TX>(P.met_n[0 * S + g]); sx = static_cast<TX>(P.met_n[1 * S + g]);
-                    tx = static_cast<TX>(P.met_n[2 * S + g]); ry = static_cast<TX>(P.met_n[3 * S + g]);
-                    sy = static_cast<TX>(P.met_n[4 * S + g]); ty = static_cast<TX>(P.met_n[5 * S + g]);
-                    rz = static_cast<TX>(P.met_n[6 * S + g]); sz = static_cast<TX>(P.met_n[7 * S + g]);
-                    tz = static_cast<TX>(P.met_n[8 * S + g]);
+                    rx = static_cast<TX>(mnow[0]); sx = static_cast<TX>(mnow[1]); tx = static_cast<TX>(mnow[2]);
+                    ry = static_cast<TX>(mnow[3]); sy = static_cast<TX>(mnow[4]); ty = static_cast<TX>(mnow[5]);
+                    rz = static_cast<TX>(mnow[6]); sz = static_cast<TX>(mnow[7]); tz = static_cast<TX>(mnow[8]);
                 } else {
                     rx = met(0); sx = met(1); tx = met(2); ry = met(3); sy = met(4);
                     ty = met(5); rz = met(6); sz = met(7); tz = met(8);
