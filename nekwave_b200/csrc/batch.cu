@@ -159,9 +159,12 @@ batch_stage_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
 
 // What a per-N launch knows of its stage: the LSRK coefficients are kernel parameters
 // (constant-bank operands, no registers); dry: a = b = dt = 0 (timing only).
+// The stages of one N follow each other on one stream: all but the first may start
+// early (launch_overlapped; the slot table does not change within a step).
 struct BatchStage {
     double a, b;
     int stage, dry;
+    bool overlap() const { return stage > 0; }
 };
 
 // Stage parameters of one tile's slot.
@@ -211,8 +214,13 @@ batch_stage_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restri
     extern __shared__ __align__(16) unsigned char smem[];
     const WorkItem w = work[blockIdx.x];
     const SlotDev& S = slots[w.slot];
-    if (!S.active) return;
+    if (!S.active) {
+        stage::grid_wait();
+        return;
+    }
     const StageParams P = slot_params(S, bs);
+    stage::grid_launch_dependents();
+    stage::grid_wait();
     if constexpr (ALG == 0)
         stage_tile<N, GEO_BOX, F32, KS, EPB, KSMEM, true>(P, w.e0, smem, threadIdx.x);
     else
@@ -228,7 +236,10 @@ batch_dmma8_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
     extern __shared__ __align__(16) unsigned char smem[];
     const WorkItem w = work[blockIdx.x];
     const SlotDev& S = slots[w.slot];
-    if (!S.active) return;
+    if (!S.active) {
+        stage::grid_wait();
+        return;
+    }
     const StageParams P = slot_params(S, bs);
     stage::dmma8_tile<2>(P, w.e0, smem, threadIdx.x,
                          CD ? dp.d : reinterpret_cast<const double*>(smem + stage::DmmaLayout8::D));
@@ -242,8 +253,7 @@ cudaError_t launch_dmma8_n(const BatchStage& bs, const SlotDev* slots, const Wor
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    kern<<<ntiles, 128, smem, st>>>(slots, work, bs, dp);
-    return cudaGetLastError();
+    return launch_overlapped(kern, ntiles, 128, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
 // Per-N shapes of the per-N mode: the single-mesh defaults (stage_variants.h entry
@@ -300,7 +310,10 @@ batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restric
     extern __shared__ __align__(16) unsigned char smem[];
     const WorkItem w = work[blockIdx.x];
     const SlotDev& S = slots[w.slot];
-    if (!S.active) return;
+    if (!S.active) {
+        stage::grid_wait();
+        return;
+    }
     const StageParams P = slot_params(S, bs);
     if constexpr (NBulk<N>::AHEAD > 0)
         stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, true, NBulk<N>::EARLY, NBulk<N>::VROW>(
@@ -319,8 +332,7 @@ cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const Work
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    kern<<<ntiles, threads, smem, st>>>(slots, work, bs, dp);
-    return cudaGetLastError();
+    return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
 template <int N, bool F32, int ALG>
@@ -336,8 +348,7 @@ cudaError_t launch_n_alg(const BatchStage& bs, const SlotDev* slots, const WorkI
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    kern<<<ntiles, threads, smem, st>>>(slots, work, bs, dp);
-    return cudaGetLastError();
+    return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
 // Dh: this N's D on the host when every resident cavity of this N uses it (the

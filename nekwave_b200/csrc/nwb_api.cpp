@@ -20,6 +20,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -96,6 +97,57 @@ int wall_code(const nwb_mesh_desc* m, long long fp, bool true_pmc) {
     if (true_pmc && m->bc_type[fp] == 2) return nwb::kConnPMC;
     if (m->bc_type[fp] != 0 || m->vol_idx_plus[fp] < 0) return nwb::kConnPEC;
     return 0;
+}
+
+namespace {
+struct HostSlab {
+    char* base = nullptr;
+    std::vector<int> free;  // block numbers
+};
+constexpr int kSlabBlocks = 256;
+std::mutex g_slab_mu;
+std::vector<HostSlab> g_slabs;
+}  // namespace
+
+void* host_block_alloc() {
+    std::lock_guard<std::mutex> lock(g_slab_mu);
+    for (HostSlab& s : g_slabs)
+        if (!s.free.empty()) {
+            const int b = s.free.back();
+            s.free.pop_back();
+            return s.base + b * kHostBlock;
+        }
+    HostSlab s;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&s.base), kSlabBlocks * kHostBlock,
+                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    try {
+        s.free.reserve(kSlabBlocks);
+        for (int b = kSlabBlocks - 1; b > 0; --b) s.free.push_back(b);
+        g_slabs.push_back(std::move(s));
+    } catch (const std::bad_alloc&) {
+        cudaFreeHost(s.base);
+        return nullptr;
+    }
+    return g_slabs.back().base;
+}
+
+void host_block_free(void* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(g_slab_mu);
+    for (size_t i = 0; i < g_slabs.size(); ++i) {
+        HostSlab& s = g_slabs[i];
+        const ptrdiff_t off = static_cast<char*>(p) - s.base;
+        if (off < 0 || off >= static_cast<ptrdiff_t>(kSlabBlocks * kHostBlock)) continue;
+        s.free.push_back(static_cast<int>(off / static_cast<ptrdiff_t>(kHostBlock)));  // within its reserve
+        if (s.free.size() == kSlabBlocks && g_slabs.size() > 1) {
+            cudaFreeHost(s.base);
+            g_slabs.erase(g_slabs.begin() + static_cast<ptrdiff_t>(i));
+        }
+        return;
+    }
 }
 
 bool snap_axis_normals(std::vector<ElemGeo>& geo) {
@@ -265,7 +317,10 @@ struct nwb_solver {
     double* dw3 = nullptr;
     double* dpartial = nullptr;
     double* denergy = nullptr;
-    int* derr = nullptr;  // kernels record an expired bounded wait here
+    // kernels record an expired bounded wait here: mapped host memory (host_block_alloc),
+    // so nwb_sync reads it without a copy
+    int* herr = nullptr;
+    int* derr = nullptr;
     int eblocks = 1;
     void* dflush = nullptr;
     size_t flush_bytes = 0;
@@ -297,7 +352,7 @@ struct nwb_solver {
         P.c0 = c0;
         P.a = kRK4A[stage];
         P.b = kRK4B[stage];
-        P.kio = nwb::stage_kio(stage);
+        P.kio = nwb::stage_kio(stage) | nwb::kOverlap;
         P.dt = dt;
         for (int x = 0; x < N * N; ++x) P.Dc[x] = hD[x];
         for (int x = 0; x < N; ++x) P.zl[x] = hzl[x];
@@ -387,9 +442,11 @@ struct nwb_solver {
         drop_graphs();
         void* ptrs[] = {u[0], u[1], k, dD, dgeo, dconn, djac_e, dmet_n, dfnrm, dflift,
                         dfplus, djac_n, dw3, dpartial, denergy, dflush, dprobe_off, dprobe_w, dprobe_out, dsnap,
-                        derr, dstage};
+                        dstage};
         for (void* p : ptrs)
             if (p) cudaFree(p);
+        nwb::host_block_free(herr);
+        herr = derr = nullptr;
         if (st) cudaStreamDestroy(st);
         st = nullptr;
         if (snap_st) cudaStreamDestroy(snap_st);
@@ -580,14 +637,16 @@ nwb_status create_solver(const nwb_mesh_desc* m, int N, int nelt, const double* 
     NWB_TRY(dalloc(&s->u[0], 6 * static_cast<size_t>(s->stride), &tot));
     NWB_TRY(dalloc(&s->u[1], 6 * static_cast<size_t>(s->stride), &tot));
     NWB_TRY(dalloc(&s->k, 6 * static_cast<size_t>(s->stride), &tot));
-    NWB_TRY(dalloc(&s->dD, static_cast<size_t>(N2), &tot));
+    NWB_TRY(dalloc(&s->dD, static_cast<size_t>(N2) + 1, &tot));  // bulk copies: 16 bytes at a time
     NWB_TRY(dalloc(&s->dw3, static_cast<size_t>(N3), &tot));
     // partial sums of the energy, or (max|E|, max|H|) pairs; energy, max|E|, max|H|
     NWB_TRY(dalloc(&s->dpartial, 2 * static_cast<size_t>(s->eblocks), &tot));
     NWB_TRY(dalloc(&s->denergy, 3, &tot));
-    NWB_TRY(dalloc(&s->derr, 1, &tot));
-    ce = cudaMemset(s->derr, 0, sizeof(int));
-    if (ce != cudaSuccess) return bail(fail(NWB_ECUDA, "memset: %s", cudaGetErrorString(ce)));
+    s->herr = static_cast<int*>(nwb::host_block_alloc());
+    ce = s->herr ? cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->derr), s->herr, 0)
+                 : cudaErrorMemoryAllocation;
+    if (s->herr) *s->herr = 0;
+    if (ce != cudaSuccess) return bail(fail(NWB_ENOMEM, "status word: %s", cudaGetErrorString(ce)));
 #define NWB_H2D(dst, src, bytes) \
     do { ce = cudaMemcpy((dst), (src), (bytes), cudaMemcpyHostToDevice); \
          if (ce != cudaSuccess) return bail(fail(NWB_ECUDA, "upload: %s", cudaGetErrorString(ce))); } while (0)
@@ -759,11 +818,10 @@ nwb_status nwb_step(nwb_solver* s, double dt, int nsteps) {
 nwb_status nwb_sync(nwb_solver* s) {
     if (!s) return fail(NWB_EINVAL, "nwb_sync: null solver");
     NWB_CU(cudaStreamSynchronize(s->st));
-    // a bounded wait inside a stage kernel that expired (the warp-specialised form)
-    int err = 0;
-    NWB_CU(cudaMemcpy(&err, s->derr, sizeof(int), cudaMemcpyDeviceToHost));
+    // a bounded wait inside a stage kernel that expired
+    const int err = *const_cast<volatile int*>(s->herr);
     if (err != 0) {
-        NWB_CU(cudaMemset(s->derr, 0, sizeof(int)));
+        *s->herr = 0;
         return fail(NWB_ETIMEOUT, "nwb_sync: a stage kernel's bounded wait expired (code %d); the "
                                   "state of the steps since the last sync is not valid", err);
     }

@@ -33,6 +33,41 @@ cudaError_t set_smem_once(K kern, int smem, std::atomic<int>* flags) {
     return cudaSuccess;
 }
 
+// Launch of a stage kernel.  overlap: as a programmatic dependent of the kernel before
+// it on the stream: its blocks may become resident once every block of that kernel
+// has started, set up their barriers and read the constant tables (D, geometry,
+// connections) and wait in grid_wait() for that kernel's completion.  A stage of a
+// small mesh is mostly launch and set-up latency, and on a large one the slots of a
+// draining last wave are otherwise empty.  B200, per step of five stages: 64
+// elements of 5 points 20.5 -> 16.4 us, 792 of 7 points 67.8 -> 66.0, 512 of 8 points 52.6 ->
+// 49.7; large meshes the same (32^3 elements of 8 points 2910 -> 2820 us with the copies
+// now issued before a block's other work).
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, bool overlap,
+                              const A&... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = a;
+    c.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kern, args...);
+}
+
+// Mapped host memory for the few words a solver's kernels hand to the host (its status
+// word and diagnostics): 1 KB blocks cut from 256 KB pinned slabs that all solvers of
+// the process share, since pinning costs the driver 1 to 3 ms a call (B200 host) and a
+// solver's whole set-up of a small cavity is 6 ms.  Thread-safe; memory visible to
+// every device; a slab is given back when its last block is, but for one, which stays.
+// nullptr when no pinned memory can be had.
+constexpr size_t kHostBlock = 1024;
+void* host_block_alloc();
+void host_block_free(void* p);
+
 // Geometry classes the mesh analysis sorts a mesh into (nwb_api.cpp).
 enum GeoKind : int {
     GEO_BOX = 0,     // affine, axis-aligned: metrics diag(rx, sy, tz) per element
@@ -72,6 +107,10 @@ constexpr int kConnPMC = -2;
 // 1923 at 7, 1944 -> 1860 at 9; 64x64x32 elements of 6 points 6710 -> 6460 us.
 constexpr int kKRead = 1;
 constexpr int kKWrite = 2;
+// A stage launch that may overlap the tail of the launch before it on its stream
+// (launch_overlapped): every stage kernel reads and writes states only behind
+// grid_wait().
+constexpr int kOverlap = 4;
 __host__ __device__ constexpr int stage_kio(int stage) {
     return (stage > 0 ? kKRead : 0) | (stage < 4 ? kKWrite : 0);
 }
@@ -82,7 +121,7 @@ struct StageParams {
     double* k;              // [6][stride], updated in place (kio)
     long long stride;       // component stride (doubles)
     int nelt;
-    int kio;                // kKRead | kKWrite
+    int kio;                // kKRead | kKWrite | kOverlap
     const double* D;        // [N*N] column-major
     const ElemGeo* geo;     // [nelt]       (GEO_BOX, GEO_AFFINE)
     const int* conn;        // [nelt*6]     (GEO_BOX, GEO_AFFINE)

@@ -18,7 +18,8 @@
 // doubles) into a component slot with two doubles of slack, and read from
 // offset (first node & 1).  Connections are copied the same way (the solver pads
 // its connection table to a multiple of four entries; a pool cavity's table
-// lies in a 256-byte-rounded range of its arena).
+// lies in a 256-byte-rounded range of its arena), and D (N^2 doubles, rounded up to 16
+// bytes) likewise.
 //
 // The wait is bounded (kWaitNs of the global timer, about a thousand times a
 // normal stage).  When it expires the block records a code in *P.err (when the
@@ -87,7 +88,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void report(const StageParams& P, int code) {
-    if (P.err) atomicCAS(P.err, 0, code);
+    if (P.err) *reinterpret_cast<volatile int*>(P.err) = code;
 }
 
 // Shared-memory layout of one tile: u_in (and with KSM k) [6][CSR] doubles with
@@ -112,7 +113,8 @@ struct BulkLayout {
 
 // Thread 0's part of a tile load: the tile's u_in (and with KSM its k; otherwise k's
 // lines are prefetched into L2), geometry and connections as bulk copies that
-// complete on the mbarrier at smem + L::bar, which must be initialised.
+// complete on the mbarrier at smem + L::bar, which must be initialised.  Waits for the
+// launches before this one (grid_wait) ahead of the first access to u and k.
 template <int N, int EPB, bool KSM, int GEO>
 __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, unsigned char* smem) {
     using L = BulkLayout<N, EPB, KSM, GEO>;
@@ -127,7 +129,19 @@ __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, u
     const unsigned cb = static_cast<unsigned>((ca1 - ca0) * 4);
     const unsigned gb = static_cast<unsigned>(nvalid * sizeof(ElemGeo));
     const bool kread = (P.kio & kKRead) != 0;
-    mbar_arrive_expect_tx(bar, (KSM && kread ? 12 : 6) * ub + (GEO == GEO_NODAL ? 0 : gb + cb));
+    constexpr unsigned db = (L::N2 * 8 + 15) / 16 * 16;  // D, to the 16-byte boundary (its array is padded)
+    mbar_arrive_expect_tx(bar, (KSM && kread ? 12 : 6) * ub + db + (GEO == GEO_NODAL ? 0 : gb + cb));
+    // constant data before grid_wait()
+    bulk_g2s(smem + L::D, P.D, db, bar);
+    if constexpr (GEO == GEO_NODAL) {
+        // the column phase reads the metrics plane by plane: into L2 meanwhile
+#pragma unroll
+        for (int c = 0; c < 9; ++c) bulk_prefetch_l2(P.met_n + c * S + a0, ub);
+    } else {
+        bulk_g2s(smem + L::geo0, P.geo + e0, gb, bar);
+        bulk_g2s(smem + L::conn0, P.conn + ca0, cb, bar);
+    }
+    grid_wait();
     double* su = reinterpret_cast<double*>(smem + L::u0);
 #pragma unroll
     for (int c = 0; c < 6; ++c) bulk_g2s(su + c * L::CSR, P.u_in + c * S + a0, ub, bar);
@@ -140,14 +154,6 @@ __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, u
     } else {
 #pragma unroll
         for (int c = 0; c < 6; ++c) bulk_prefetch_l2(P.k + c * S + a0, ub);
-    }
-    if constexpr (GEO == GEO_NODAL) {
-        // the column phase reads the metrics plane by plane: into L2 meanwhile
-#pragma unroll
-        for (int c = 0; c < 9; ++c) bulk_prefetch_l2(P.met_n + c * S + a0, ub);
-    } else {
-        bulk_g2s(smem + L::geo0, P.geo + e0, gb, bar);
-        bulk_g2s(smem + L::conn0, P.conn + ca0, cb, bar);
     }
 }
 
@@ -185,23 +191,23 @@ template <int N, int GEO, int KS, int EPB, bool CONSTD, bool DSMEM, bool KSM, bo
 __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, unsigned char* smem,
                                           const int tid, const double* Dc, const Pull& pull = Pull()) {
     using L = BulkLayout<N, EPB, KSM, GEO>;
-    constexpr int NT = EPB * KS * N * N;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     double* sD = reinterpret_cast<double*>(smem + L::D);
+    grid_launch_dependents();
+    // the copies first (a block of a large grid waits for nothing before them): only
+    // thread 0 touches the mbarrier before the block's next barrier
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_fence_init();
-    }
-    for (int x = tid; x < L::N2; x += NT) sD[x] = P.D[x];
-    __syncthreads();
-    const long long g0 = static_cast<long long>(e0) * L::N3;
-    FaceRegs<N, GEO, KS, true> G;
-    if (tid == 0) {
         bulk_issue<N, EPB, KSM, GEO>(P, e0, smem);
         pull();
     }
-    if constexpr (EARLY && GEO == GEO_BOX) gather_box<N, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
-    else if constexpr (EARLY) gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
+    const long long g0 = static_cast<long long>(e0) * L::N3;
+    FaceRegs<N, GEO, KS, true> G;
+    if constexpr (EARLY && GEO == GEO_BOX) gather_box_nodes<N, KS, EPB, false>(P, e0, nullptr, tid, G);
+    if constexpr (EARLY && GEO != GEO_BOX) gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
+    grid_wait();
+    if constexpr (EARLY && GEO == GEO_BOX) gather_box_values<N, KS, EPB, false, false>(P, e0, nullptr, tid, G);
     if (!bulk_wait_tile<N, EPB, KSM, GEO>(P, smem, tid)) return;
     const int off = static_cast<int>(g0 & 1);
     const double* su = reinterpret_cast<const double*>(smem + L::u0) + off;
@@ -274,8 +280,7 @@ cudaError_t launch_bulk(const StageParams* p, cudaStream_t st, StageConfig* cfg)
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, L::total, attr_set); e != cudaSuccess) return e;
     if (!p) return cudaSuccess;
-    kern<<<(p->nelt + EPB - 1) / EPB, threads, L::total, st>>>(*p);
-    return cudaGetLastError();
+    return launch_overlapped(kern, (p->nelt + EPB - 1) / EPB, threads, L::total, st, (p->kio & kOverlap) != 0, *p);
 }
 
 // Shapes of the general classes (affine and per-node geometry) in FP64: the bulk-copy

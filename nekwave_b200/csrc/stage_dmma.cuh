@@ -194,9 +194,11 @@ __device__ __forceinline__ void dmma8_tile(const StageParams& P, const int e, un
     double* sD = reinterpret_cast<double*>(smem + L::D);
     double* sflux = reinterpret_cast<double*>(smem + L::flux);
 
+    grid_launch_dependents();
+    if (tid < 64) cp_async8(sD + tid, P.D + tid);
+    grid_wait();
     if (tid < NT) {
         issue2<N, GEO_BOX, 1, NT, false>(P, e, su, sg, sc, tid);
-        if (tid < 64) cp_async8(sD + tid, P.D + tid);
         if (tid == 0 && e_ahead >= 0) prefetch_tile_l2<N3>(P, e_ahead, 1);
     }
     cp_async_commit();
@@ -211,7 +213,8 @@ __device__ __forceinline__ void dmma8_tile(const StageParams& P, const int e, un
     // neighbour traces while the tile's copies fly: the thread's points of faces 0..3,
     // and of its two node columns across t (a part of four planes holds one end)
     BoxFaces<box_points<WPF>()> G;
-    gather_box<N, WPF, 1, false, false, 0, false>(P, e, nullptr, nullptr, tid, G);
+    gather_box_nodes<N, WPF, 1, false, false>(P, e, nullptr, tid, G);
+    gather_box_values<N, WPF, 1, false, false, 0, false>(P, e, nullptr, tid, G);
     constexpr int NZ = WPF == 1 ? 2 : 1;
     double zn[NZ][4][2];
     int zv[NZ];
@@ -282,8 +285,7 @@ cudaError_t launch_dmma8(const StageParams* p, cudaStream_t st, StageConfig* cfg
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (!p) return cudaSuccess;
-    kern<<<p->nelt, 64 * WPF, smem, st>>>(*p);
-    return cudaGetLastError();
+    return launch_overlapped(kern, p->nelt, 64 * WPF, smem, st, (p->kio & kOverlap) != 0, *p);
 }
 
 }  // namespace stage

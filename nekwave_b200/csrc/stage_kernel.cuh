@@ -33,6 +33,15 @@
 namespace nwb {
 namespace stage {
 
+// Lets the next launch of the stream start its blocks (launch_overlapped), and waits
+// until the launches this one depends on have completed and their writes are visible
+// (both do nothing where the launch has no such dependents or dependency).  Every
+// block of a kernel that can be launched that way waits before it ends.
+__device__ __forceinline__ void grid_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc) {
     unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
@@ -426,6 +435,8 @@ template <int N, int GEO, bool F32, int KS, int EPB, bool KSMEM, int MINB>
 __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     stage_kernel(const StageParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
+    grid_launch_dependents();
+    grid_wait();
     stage_tile<N, GEO, F32, KS, EPB, KSMEM>(P, blockIdx.x * EPB, smem, threadIdx.x);
 }
 
@@ -441,8 +452,7 @@ cudaError_t launch_cfg(const StageParams* p, cudaStream_t st, StageConfig* cfg) 
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (!p) return cudaSuccess;
     const int blocks = (p->nelt + EPB - 1) / EPB;
-    kern<<<blocks, threads, smem, st>>>(*p);
-    return cudaGetLastError();
+    return launch_overlapped(kern, blocks, threads, smem, st, (p->kio & kOverlap) != 0, *p);
 }
 
 }  // namespace stage

@@ -243,6 +243,8 @@ __device__ __forceinline__ void stage_tile_mma8(const StageParams& P, const int 
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) stage_kernel_mma8(const StageParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
+    grid_launch_dependents();
+    grid_wait();
     stage_tile_mma8(P, blockIdx.x, smem, threadIdx.x);
 }
 
@@ -254,8 +256,7 @@ cudaError_t launch_mma8(const StageParams* p, cudaStream_t st, StageConfig* cfg)
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (!p) return cudaSuccess;
-    kern<<<p->nelt, 128, smem, st>>>(*p);
-    return cudaGetLastError();
+    return launch_overlapped(kern, p->nelt, 128, smem, st, (p->kio & kOverlap) != 0, *p);
 }
 
 }  // namespace stage

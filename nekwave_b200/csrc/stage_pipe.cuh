@@ -346,7 +346,6 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
             const int f = fp / N2;
             const int pq = fp - f * N2;
             const int p = pq % N, qq = pq / N;
-            int eB = -1;
             if constexpr (GEO == GEO_NODAL) {
                 const long long g = (static_cast<long long>(e) * 6 + f) * N2 + pq;
                 vB = __ldg(P.fplus + g);
@@ -354,9 +353,8 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
                 G.nl[q][1] = __ldg(P.fnrm + P.nfp + g);
                 G.nl[q][2] = __ldg(P.fnrm + 2 * P.nfp + g);
                 G.nl[q][3] = __ldg(P.flift + g);
-                if (vB >= 0) eB = static_cast<int>(vB / N3);
             } else if (structured) {
-                eB = struct_neighbour(P, ex, ey, ez, e, f);
+                const int eB = struct_neighbour(P, ex, ey, ez, e, f);
                 if (eB >= 0) {
                     vB = static_cast<long long>(eB) * N3 + face_local<N>(opposite_face(f), p, qq);
                 }
@@ -367,7 +365,7 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
                 vB = cd;
                 if (cd >= 0) {
                     const int fB = (cd >> 3) & 7, o = cd & 7;
-                    eB = cd >> 6;
+                    const int eB = cd >> 6;
                     int a = (o & 4) ? qq : p;
                     int b = (o & 4) ? p : qq;
                     if (o & 1) a = N - 1 - a;
@@ -375,22 +373,28 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
                     vB = static_cast<long long>(eB) * N3 + face_local<N>(fB, a, b);
                 }
             }
-            if (vB >= 0) {
-                bool in_tile = false;
-                if constexpr (FROM_SMEM) in_tile = eB >= e0 && eB < e0 + nvalid;
-                if (in_tile) {
-                    const int el = eB - e0;
-                    constexpr int EN3 = PAD ? N2 * (N + 1) : N3;  // element stride in the tile
-                    const int sidx = el * EN3 + pidx<N, PAD>(static_cast<int>(vB - static_cast<long long>(eB) * N3));
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) G.nb[q][c] = su[c * CS + sidx];
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) G.nb[q][c] = __ldg(P.u_in + c * S + vB);
-                }
-            }
         }
         G.vB[q] = vB;
+    }
+    // the connections, normals and lifts above are constant; the state is not
+    grid_wait();
+#pragma unroll
+    for (int q = 0; q < FPT; ++q) {
+        const long long vB = G.vB[q];
+        if (vB < 0) continue;
+        if constexpr (FROM_SMEM) {
+            const int l = static_cast<int>(vB - static_cast<long long>(e0) * N3);
+            if (l >= 0 && l < nvalid * N3) {
+                const int el = l / N3;
+                constexpr int EN3 = PAD ? N2 * (N + 1) : N3;  // element stride in the tile
+                const int sidx = el * EN3 + pidx<N, PAD>(l - el * N3);
+#pragma unroll
+                for (int c = 0; c < 6; ++c) G.nb[q][c] = su[c * CS + sidx];
+                continue;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) G.nb[q][c] = __ldg(P.u_in + c * S + vB);
     }
 }
 
@@ -579,26 +583,21 @@ __device__ __forceinline__ int conn_node(int cd, int p, int q) {
     return (cd >> 6) * (N * N * N) + face_local<N>((cd >> 3) & 7, a, b);
 }
 
-// Fill a BoxFaces.  FROM_SMEM: the tile is resident (connections from sc, neighbours
-// inside the tile from su); otherwise only global memory is read (and neighbours follow
-// from the box structure where there is one), so it may run while the tile's copies
-// are in flight.
-// ZF: the points across t as well.
-template <int N, int KS, int EPB, bool PAD, bool FROM_SMEM, int CSX = 0, bool ZF = true>
-__device__ __forceinline__ void gather_box(const StageParams& P, const int e0, const double* su,
-                                           const int* sc, const int tid, BoxFaces<box_points<KS>()>& G) {
+// The neighbour nodes of a BoxFaces, from the box structure where there is one or from the
+// connections (FROM_SMEM: sc of the resident tile): constant data, which may be read
+// before grid_wait().  ZF: the points across t as well.
+template <int N, int KS, int EPB, bool FROM_SMEM, bool ZF = true>
+__device__ __forceinline__ void gather_box_nodes(const StageParams& P, const int e0, const int* sc,
+                                                 const int tid, BoxFaces<box_points<KS>()>& G) {
     constexpr int N2 = N * N, N3 = N2 * N;
     constexpr int TPE = KS * N2;
-    constexpr int CS = CSX ? CSX : EPB * (PAD ? N2 * (N + 1) : N3);
     constexpr int FPT = box_points<KS>();
     const int team = tid / TPE;
     const int lt = tid - team * TPE;
     const int h = lt / N2, pq = lt - h * N2;
     const int p = pq % N, q = pq / N;
-    const int nvalid = min(EPB, P.nelt - e0);
     const int e = e0 + team;
-    const long long S = P.stride;
-    if (team >= nvalid) {
+    if (team >= min(EPB, P.nelt - e0)) {
 #pragma unroll
         for (int x = 0; x < FPT; ++x) G.vB[x] = kConnPEC;
         G.zv[0] = G.zv[1] = kConnPEC;
@@ -622,6 +621,30 @@ __device__ __forceinline__ void gather_box(const StageParams& P, const int e0, c
         else cd = __ldg(P.conn + e * 6 + f);
         return conn_node<N>(cd, p, q);
     };
+#pragma unroll
+    for (int x = 0; x < FPT; ++x) {
+        const int f = x * KS + h;  // odd: across r, even: across s
+        G.vB[x] = (KS * FPT == 4 || f < 4) ? node(f) : kConnPEC;
+    }
+    if constexpr (ZF) {
+        G.zv[0] = node(4);
+        G.zv[1] = node(5);
+    }
+}
+
+// The neighbour values of a BoxFaces whose nodes are known.  FROM_SMEM: the tile is
+// resident (neighbours inside it from su); otherwise only global memory is read, so it
+// may run while the tile's copies are in flight.
+template <int N, int KS, int EPB, bool PAD, bool FROM_SMEM, int CSX = 0, bool ZF = true>
+__device__ __forceinline__ void gather_box_values(const StageParams& P, const int e0, const double* su,
+                                                  const int tid, BoxFaces<box_points<KS>()>& G) {
+    constexpr int N2 = N * N, N3 = N2 * N;
+    constexpr int CS = CSX ? CSX : EPB * (PAD ? N2 * (N + 1) : N3);
+    constexpr int FPT = box_points<KS>();
+    const int lt = tid % (KS * N2);
+    const int h = lt / N2;
+    const int nvalid = min(EPB, P.nelt - e0);
+    const long long S = P.stride;
     auto fetch = [&](int vB, int ca, int cb, double (&v)[4]) {
         if constexpr (FROM_SMEM) {
             const int l = vB - e0 * N3;
@@ -644,19 +667,20 @@ __device__ __forceinline__ void gather_box(const StageParams& P, const int e0, c
 #pragma unroll
     for (int x = 0; x < FPT; ++x) {
         const int f = x * KS + h;  // odd: across r (a, b = y, z), even: across s (z, x)
-        G.vB[x] = kConnPEC;
-        if (KS * FPT == 4 || f < 4) {
-            G.vB[x] = node(f);
-            if (G.vB[x] >= 0) fetch(G.vB[x], (f & 1) ? 1 : 2, (f & 1) ? 2 : 0, G.nb[x]);
-        }
+        if (G.vB[x] >= 0) fetch(G.vB[x], (f & 1) ? 1 : 2, (f & 1) ? 2 : 0, G.nb[x]);
     }
     if constexpr (ZF) {
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            G.zv[s] = node(4 + s);
+        for (int s = 0; s < 2; ++s)
             if (G.zv[s] >= 0) fetch(G.zv[s], 0, 1, G.zn[s]);
-        }
     }
+}
+
+template <int N, int KS, int EPB, bool PAD, bool FROM_SMEM, int CSX = 0>
+__device__ __forceinline__ void gather_box(const StageParams& P, const int e0, const double* su,
+                                           const int* sc, const int tid, BoxFaces<box_points<KS>()>& G) {
+    gather_box_nodes<N, KS, EPB, FROM_SMEM>(P, e0, sc, tid, G);
+    gather_box_values<N, KS, EPB, PAD, FROM_SMEM, CSX>(P, e0, su, tid, G);
 }
 
 // Jumps of the four components of one face point: nb - own, or the wall's mirror (PEC:
@@ -1303,6 +1327,8 @@ __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     const int tid = threadIdx.x;
     const int ntiles = (P.nelt + EPB - 1) / EPB;
     int t = blockIdx.x;
+    grid_launch_dependents();
+    grid_wait();
     if (t >= ntiles) return;
     double* sD = reinterpret_cast<double*>(smem + L::D);
     double* sflux = reinterpret_cast<double*>(smem + L::flux);
@@ -1368,8 +1394,7 @@ cudaError_t launch2(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
     if (!p) return cudaSuccess;
     const int tiles = (p->nelt + EPB - 1) / EPB;
     const int blocks = PIPE ? (tiles < res ? tiles : res) : tiles;
-    kern<<<blocks, threads, smem, st>>>(*p);
-    return cudaGetLastError();
+    return launch_overlapped(kern, blocks, threads, smem, st, (p->kio & kOverlap) != 0, *p);
 }
 
 }  // namespace stage
