@@ -1,6 +1,14 @@
 // diag_kernels.cu -- device diagnostics: the FP64 discrete energy of
-// Case::computeTotalEnergy (src/case.cpp:733-766) as a deterministic two-pass
-// reduction, and an L2-evicting buffer write used between timed iterations.
+// Case::computeTotalEnergy (src/case.cpp:733-766) and the largest |E| and |H| of
+// Case::getMaxE / getMaxH (src/case.cpp:768-794) as deterministic two-pass reductions,
+// the probe values of ProbeManager::record (src/probe.cpp:192-216), and an L2-evicting
+// buffer write used between timed iterations.
+//
+// The reductions are bound by HBM on large states (48 bytes a node, read two nodes
+// per 16-byte load) and by latency on small ones, so the second pass sums its at most
+// 1184 partials with a block, and results go to mapped host memory (no copy).
+// B200, 792 elements of 7 points: ten steps with a probe read after each, then the energy
+// and the norms, 1275 -> 901 us.
 #include "nwb_internal.h"
 
 namespace nwb {
@@ -8,28 +16,46 @@ namespace {
 
 constexpr int kEnergyThreads = 256;
 
-// Block b sums 1/2 (|E|^2 + |H|^2) J w3 over a contiguous range of nodes with a
+// Contiguous range of nodes of this block, starting at an even node (the states'
+// component rows are 512-byte aligned, so node pairs are 16-byte aligned).
+__device__ __forceinline__ void node_range(int npts, int* lo, int* hi) {
+    const int pairs = (npts + 1) / 2;
+    const int per = (pairs + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+    *lo = min(pairs, per * static_cast<int>(blockIdx.x));
+    *hi = min(pairs, *lo + per);
+}
+
+// Block b sums 1/2 (|E|^2 + |H|^2) J w3 over a contiguous range of node pairs with a
 // fixed per-thread order and a fixed shuffle tree, so repeated calls agree bit
-// for bit.  jac_e (per element) or jac_n (per node) supplies J.
+// for bit.  jac_e (per element) or jac_n (per node) supplies J.  Node indices fit an
+// int (at most 2^31 - 1 nodes); a row's padding holds the odd last pair's partner.
 __global__ void __launch_bounds__(kEnergyThreads)
-energy_partials_kernel(const double* __restrict__ u, long long stride, int N3,
-                       long long npts, const double* __restrict__ jac_e,
-                       const double* __restrict__ jac_n, const double* __restrict__ w3,
-                       double* __restrict__ partial) {
-    const long long per = (npts + gridDim.x - 1) / gridDim.x;
-    const long long lo = per * blockIdx.x;
-    const long long hi = min(npts, lo + per);
+energy_partials_kernel(const double* __restrict__ u, long long stride, int N3, int npts,
+                       const double* __restrict__ jac_e, const double* __restrict__ jac_n,
+                       const double* __restrict__ w3, double* __restrict__ partial) {
+    int lo, hi;
+    node_range(npts, &lo, &hi);
     double acc = 0.0;
-    for (long long p = lo + threadIdx.x; p < hi; p += blockDim.x) {
-        const long long e = p / N3;
-        const int m = static_cast<int>(p - e * N3);
-        const double J = jac_n ? jac_n[p] : jac_e[e];
-        const double dV = J * w3[m];
-        const double ex = u[p], ey = u[stride + p], ez = u[2 * stride + p];
-        const double hx = u[3 * stride + p], hy = u[4 * stride + p], hz = u[5 * stride + p];
-        const double eSq = ex * ex + ey * ey + ez * ez;
-        const double hSq = hx * hx + hy * hy + hz * hz;
-        acc += 0.5 * (eSq + hSq) * dV;
+    for (int x = lo + static_cast<int>(threadIdx.x); x < hi; x += kEnergyThreads) {
+        const int p = 2 * x;
+        double2 v[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) v[c] = __ldg(reinterpret_cast<const double2*>(u + c * stride + p));
+        const unsigned e = static_cast<unsigned>(p) / static_cast<unsigned>(N3);
+        const int m = p - static_cast<int>(e) * N3;
+        const double dV = (jac_n ? jac_n[p] : jac_e[e]) * w3[m];
+        acc += 0.5 *
+               ((v[0].x * v[0].x + v[1].x * v[1].x + v[2].x * v[2].x) +
+                (v[3].x * v[3].x + v[4].x * v[4].x + v[5].x * v[5].x)) *
+               dV;
+        if (p + 1 < npts) {
+            const bool next = m + 1 == N3;
+            const double dW = (jac_n ? jac_n[p + 1] : jac_e[next ? e + 1 : e]) * w3[next ? 0 : m + 1];
+            acc += 0.5 *
+                   ((v[0].y * v[0].y + v[1].y * v[1].y + v[2].y * v[2].y) +
+                    (v[3].y * v[3].y + v[4].y * v[4].y + v[5].y * v[5].y)) *
+                   dW;
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
@@ -43,37 +69,54 @@ energy_partials_kernel(const double* __restrict__ u, long long stride, int N3,
     }
 }
 
-__global__ void energy_final_kernel(const double* __restrict__ partial, int n,
-                                    double* __restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < n; ++b) s += partial[b];
-        *out = s;
+// One block: strided sums in a fixed order, then a fixed tree.  (One thread summing them
+// one after the other waited for L2 at every fourth: about 100 us for 1184.)
+__global__ void __launch_bounds__(kEnergyThreads)
+energy_final_kernel(const double* __restrict__ partial, int n, double* __restrict__ out) {
+    __shared__ double s[kEnergyThreads];
+    double acc = 0.0;
+    for (int b = threadIdx.x; b < n; b += kEnergyThreads) acc += partial[b];
+    s[threadIdx.x] = acc;
+    __syncthreads();
+#pragma unroll
+    for (int w = kEnergyThreads / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *out = s[0];
 }
 
-// Largest |E| and |H| over the nodes of a contiguous range per block, as
-// Case::getMaxE / getMaxH (src/case.cpp:768-794) form them on the host:
-// sqrt((x*x + y*y) + z*z) with separate multiply, add and square-root roundings
-// (no contraction), kept when larger than the running maximum (a NaN node never
-// is).  The maximum does not depend on the order, so the result equals the
-// host's bit for bit.  partial[2b] = max|E|, partial[2b+1] = max|H| of block b.
-__device__ __forceinline__ double norm3_rn(double x, double y, double z) {
-    return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
+// Largest |E|^2 and |H|^2 over the nodes of a contiguous range per block, the squares
+// formed as Case::getMaxE / getMaxH (src/case.cpp:768-794) form them on the host:
+// (x*x + y*y) + z*z with separate multiply and add roundings (no contraction), kept when
+// larger than the running maximum (a NaN node never is).  The correctly rounded
+// square root is monotone, so the root of the largest square, taken once at the end, is
+// the host's largest root bit for bit, in any order.
+// partial[2b] = max |E|^2, partial[2b+1] = max |H|^2 of block b.
+__device__ __forceinline__ double square3_rn(double x, double y, double z) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
 }
 
 __global__ void __launch_bounds__(kEnergyThreads)
-maxnorm_partials_kernel(const double* __restrict__ u, long long stride, long long npts,
+maxnorm_partials_kernel(const double* __restrict__ u, long long stride, int npts,
                         double* __restrict__ partial) {
-    const long long per = (npts + gridDim.x - 1) / gridDim.x;
-    const long long lo = per * blockIdx.x;
-    const long long hi = min(npts, lo + per);
+    int lo, hi;
+    node_range(npts, &lo, &hi);
     double me = 0.0, mh = 0.0;
-    for (long long p = lo + threadIdx.x; p < hi; p += blockDim.x) {
-        const double e = norm3_rn(u[p], u[stride + p], u[2 * stride + p]);
-        const double h = norm3_rn(u[3 * stride + p], u[4 * stride + p], u[5 * stride + p]);
+    for (int x = lo + static_cast<int>(threadIdx.x); x < hi; x += kEnergyThreads) {
+        const int p = 2 * x;
+        double2 v[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) v[c] = __ldg(reinterpret_cast<const double2*>(u + c * stride + p));
+        double e = square3_rn(v[0].x, v[1].x, v[2].x), h = square3_rn(v[3].x, v[4].x, v[5].x);
         if (e > me) me = e;
         if (h > mh) mh = h;
+        if (p + 1 < npts) {
+            e = square3_rn(v[0].y, v[1].y, v[2].y);
+            h = square3_rn(v[3].y, v[4].y, v[5].y);
+            if (e > me) me = e;
+            if (h > mh) mh = h;
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -96,30 +139,49 @@ maxnorm_partials_kernel(const double* __restrict__ u, long long stride, long lon
     }
 }
 
-__global__ void maxnorm_final_kernel(const double* __restrict__ partial, int n,
-                                     double* __restrict__ out) {
-    if (blockIdx.x == 0 && threadIdx.x < 2) {
-        double m = 0.0;
-        for (int b = 0; b < n; ++b)
-            if (partial[2 * b + threadIdx.x] > m) m = partial[2 * b + threadIdx.x];
-        out[threadIdx.x] = m;
+// One warp per field over the blocks' maxima.
+__global__ void __launch_bounds__(64)
+maxnorm_final_kernel(const double* __restrict__ partial, int n, double* __restrict__ out) {
+    const int field = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double m = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < n; b += 32) {
+        const double v = partial[2 * b + field];
+        if (v > m) m = v;
     }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const double o = __shfl_down_sync(0xffffffffu, m, off);
+        if (o > m) m = o;
+    }
+    if (lane == 0) out[field] = __dsqrt_rn(m);
 }
 
-// ProbeManager::record (src/probe.cpp:192-216): thread (probe, component) sums
-// w[p] * u[offset + p] over the probe element's N^3 nodes in node order, with
-// separate multiply and add roundings as on the host, so the values equal the
-// reference's bit for bit on the same state and weights.
-__global__ void probe_kernel(const double* __restrict__ u, long long stride, int N3,
-                             const long long* __restrict__ offset, const double* __restrict__ w,
-                             int nprobes, double* __restrict__ out) {
+// ProbeManager::record (src/probe.cpp:192-216): warp c of block pr forms the N^3 products
+// w[p] * u[offset + p] of component c with coalesced loads, then its first lane adds
+// them in node order, with separate multiply and add roundings as on the host, so the
+// values equal the reference's bit for bit on the same state and weights.  (One thread
+// per component loading as it adds waited for L2 at every fourth node.)  The weights are
+// loaded before grid_wait(): the launch may overlap the stage before it.
+constexpr int kProbeThreads = 192;
+__global__ void __launch_bounds__(kProbeThreads)
+probe_kernel(const double* __restrict__ u, long long stride, int N3,
+             const long long* __restrict__ offset, const double* __restrict__ w, int nprobes,
+             double* __restrict__ out) {
+    __shared__ double prod[6][1000];
     const int pr = blockIdx.x;
-    const int c = threadIdx.x;
-    if (pr >= nprobes || c >= 6) return;
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double* wp = w + static_cast<long long>(pr) * N3;
     const double* up = u + c * stride + offset[pr];
+    for (int p = lane; p < N3; p += 32) prod[c][p] = wp[p];
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+#pragma unroll 4
+    for (int p = lane; p < N3; p += 32) prod[c][p] = __dmul_rn(prod[c][p], up[p]);
+    __syncwarp();
+    if (lane != 0) return;
     double acc = 0.0;
-    for (int p = 0; p < N3; ++p) acc = __dadd_rn(acc, __dmul_rn(wp[p], up[p]));
+#pragma unroll 16
+    for (int p = 0; p < N3; ++p) acc = __dadd_rn(acc, prod[c][p]);
     out[pr * 6 + c] = acc;
 }
 
@@ -140,29 +202,29 @@ cudaError_t launch_energy(const double* u, long long stride, int N, int nelt,
                           const double* jac_e, const double* jac_n, const double* w3,
                           double* partial, int nblocks, double* out, cudaStream_t st) {
     const int N3 = N * N * N;
-    const long long npts = static_cast<long long>(nelt) * N3;
+    const int npts = nelt * N3;
     energy_partials_kernel<<<nblocks, kEnergyThreads, 0, st>>>(u, stride, N3, npts, jac_e, jac_n,
                                                                w3, partial);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    energy_final_kernel<<<1, 32, 0, st>>>(partial, nblocks, out);
+    energy_final_kernel<<<1, kEnergyThreads, 0, st>>>(partial, nblocks, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_max_norms(const double* u, long long stride, long long npts, double* partial,
                              int nblocks, double* out, cudaStream_t st) {
-    maxnorm_partials_kernel<<<nblocks, kEnergyThreads, 0, st>>>(u, stride, npts, partial);
+    maxnorm_partials_kernel<<<nblocks, kEnergyThreads, 0, st>>>(u, stride, static_cast<int>(npts), partial);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    maxnorm_final_kernel<<<1, 32, 0, st>>>(partial, nblocks, out);
+    maxnorm_final_kernel<<<1, 64, 0, st>>>(partial, nblocks, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_probes(const double* u, long long stride, int N3, const long long* offset,
                           const double* w, int nprobes, double* out, cudaStream_t st) {
     if (nprobes <= 0) return cudaSuccess;
-    probe_kernel<<<nprobes, 32, 0, st>>>(u, stride, N3, offset, w, nprobes, out);
-    return cudaGetLastError();
+    return launch_overlapped(probe_kernel, nprobes, kProbeThreads, 0, st, true, u, stride, N3, offset, w, nprobes,
+                             out);
 }
 
 cudaError_t launch_l2_flush(void* buf, size_t bytes, cudaStream_t st) {

@@ -276,6 +276,10 @@ nwb_status dalloc(T** p, size_t count, size_t* total) {
 
 extern "C" void nwb_set_error_(const char* msg) { g_err = msg ? msg : ""; }
 
+// Probes whose values fit a solver's block of mapped host memory; more go through a
+// device buffer and a copy.
+constexpr int kHostProbes = 20;
+
 struct nwb_solver {
     int device = 0;
     cudaStream_t st = nullptr;
@@ -316,11 +320,16 @@ struct nwb_solver {
     double* djac_n = nullptr;
     double* dw3 = nullptr;
     double* dpartial = nullptr;
-    double* denergy = nullptr;
-    // kernels record an expired bounded wait here: mapped host memory (host_block_alloc),
-    // so nwb_sync reads it without a copy
-    int* herr = nullptr;
-    int* derr = nullptr;
+    // A block of mapped host memory (host_block_alloc): kernels record an expired bounded
+    // wait and write the energy, the largest norms and the probe values there, so reading
+    // them needs no copy.
+    struct HostWords {
+        double energy, norms[2];
+        int err;
+        double probes[6 * kHostProbes];
+    };
+    HostWords* hw = nullptr;
+    HostWords* dw = nullptr;
     int eblocks = 1;
     void* dflush = nullptr;
     size_t flush_bytes = 0;
@@ -348,7 +357,7 @@ struct nwb_solver {
         P.flift = dflift;
         P.fplus = dfplus;
         P.nfp = nfp;
-        P.err = derr;
+        P.err = &dw->err;
         P.c0 = c0;
         P.a = kRK4A[stage];
         P.b = kRK4B[stage];
@@ -441,12 +450,12 @@ struct nwb_solver {
     void release() {
         drop_graphs();
         void* ptrs[] = {u[0], u[1], k, dD, dgeo, dconn, djac_e, dmet_n, dfnrm, dflift,
-                        dfplus, djac_n, dw3, dpartial, denergy, dflush, dprobe_off, dprobe_w, dprobe_out, dsnap,
+                        dfplus, djac_n, dw3, dpartial, dflush, dprobe_off, dprobe_w, dprobe_out, dsnap,
                         dstage};
         for (void* p : ptrs)
             if (p) cudaFree(p);
-        nwb::host_block_free(herr);
-        herr = derr = nullptr;
+        nwb::host_block_free(hw);
+        hw = dw = nullptr;
         if (st) cudaStreamDestroy(st);
         st = nullptr;
         if (snap_st) cudaStreamDestroy(snap_st);
@@ -639,13 +648,13 @@ nwb_status create_solver(const nwb_mesh_desc* m, int N, int nelt, const double* 
     NWB_TRY(dalloc(&s->k, 6 * static_cast<size_t>(s->stride), &tot));
     NWB_TRY(dalloc(&s->dD, static_cast<size_t>(N2) + 1, &tot));  // bulk copies: 16 bytes at a time
     NWB_TRY(dalloc(&s->dw3, static_cast<size_t>(N3), &tot));
-    // partial sums of the energy, or (max|E|, max|H|) pairs; energy, max|E|, max|H|
+    // partial sums of the energy, or (max|E|^2, max|H|^2) pairs
     NWB_TRY(dalloc(&s->dpartial, 2 * static_cast<size_t>(s->eblocks), &tot));
-    NWB_TRY(dalloc(&s->denergy, 3, &tot));
-    s->herr = static_cast<int*>(nwb::host_block_alloc());
-    ce = s->herr ? cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->derr), s->herr, 0)
-                 : cudaErrorMemoryAllocation;
-    if (s->herr) *s->herr = 0;
+    static_assert(sizeof(nwb_solver::HostWords) <= nwb::kHostBlock, "one block of host memory");
+    s->hw = static_cast<nwb_solver::HostWords*>(nwb::host_block_alloc());
+    ce = s->hw ? cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->dw), s->hw, 0)
+               : cudaErrorMemoryAllocation;
+    if (s->hw) *s->hw = {};
     if (ce != cudaSuccess) return bail(fail(NWB_ENOMEM, "status word: %s", cudaGetErrorString(ce)));
 #define NWB_H2D(dst, src, bytes) \
     do { ce = cudaMemcpy((dst), (src), (bytes), cudaMemcpyHostToDevice); \
@@ -819,9 +828,9 @@ nwb_status nwb_sync(nwb_solver* s) {
     if (!s) return fail(NWB_EINVAL, "nwb_sync: null solver");
     NWB_CU(cudaStreamSynchronize(s->st));
     // a bounded wait inside a stage kernel that expired
-    const int err = *const_cast<volatile int*>(s->herr);
+    const int err = *const_cast<volatile int*>(&s->hw->err);
     if (err != 0) {
-        *s->herr = 0;
+        s->hw->err = 0;
         return fail(NWB_ETIMEOUT, "nwb_sync: a stage kernel's bounded wait expired (code %d); the "
                                   "state of the steps since the last sync is not valid", err);
     }
@@ -851,11 +860,11 @@ nwb_status nwb_eval_rhs(nwb_solver* s, double* h, size_t n) {
 nwb_status nwb_energy(nwb_solver* s, double* out) {
     if (!s || !out) return fail(NWB_EINVAL, "nwb_energy: null argument");
     cudaError_t e = nwb::launch_energy(s->u[s->cur], s->stride, s->N, s->nelt, s->djac_e, s->djac_n,
-                                       s->dw3, s->dpartial, s->eblocks, s->denergy, s->st);
+                                       s->dw3, s->dpartial, s->eblocks, &s->dw->energy, s->st);
     if (e != cudaSuccess) return fail(NWB_ECUDA, "energy kernel: %s", cudaGetErrorString(e));
     s->launches += 2;
-    NWB_CU(cudaMemcpyAsync(out, s->denergy, sizeof(double), cudaMemcpyDeviceToHost, s->st));
     NWB_CU(cudaStreamSynchronize(s->st));
+    *out = *const_cast<volatile double*>(&s->hw->energy);
     if (!std::isfinite(*out)) return fail(NWB_ENONFINITE, "nwb_energy: state holds NaN/Inf");
     return NWB_OK;
 }
@@ -863,12 +872,12 @@ nwb_status nwb_energy(nwb_solver* s, double* out) {
 nwb_status nwb_max_norms(nwb_solver* s, double* max_e, double* max_h) {
     if (!s || !max_e || !max_h) return fail(NWB_EINVAL, "nwb_max_norms: null argument");
     cudaError_t e = nwb::launch_max_norms(s->u[s->cur], s->stride, s->npts, s->dpartial, s->eblocks,
-                                          s->denergy + 1, s->st);
+                                          s->dw->norms, s->st);
     if (e != cudaSuccess) return fail(NWB_ECUDA, "max-norm kernel: %s", cudaGetErrorString(e));
     s->launches += 2;
-    double h[2];
-    NWB_CU(cudaMemcpyAsync(h, s->denergy + 1, 2 * sizeof(double), cudaMemcpyDeviceToHost, s->st));
     NWB_CU(cudaStreamSynchronize(s->st));
+    const volatile double* const w = s->hw->norms;
+    const double h[2] = {w[0], w[1]};
     *max_e = h[0];
     *max_h = h[1];
     if (!std::isfinite(h[0]) || !std::isfinite(h[1]))
@@ -897,7 +906,7 @@ nwb_status nwb_probe_setup(nwb_solver* s, int nprobes, const long long* node_off
     if (nprobes == 0) return NWB_OK;
     NWB_CU(cudaMalloc(&s->dprobe_off, sizeof(long long) * nprobes));
     NWB_CU(cudaMalloc(&s->dprobe_w, sizeof(double) * N3 * static_cast<size_t>(nprobes)));
-    NWB_CU(cudaMalloc(&s->dprobe_out, sizeof(double) * 6 * nprobes));
+    if (nprobes > kHostProbes) NWB_CU(cudaMalloc(&s->dprobe_out, sizeof(double) * 6 * nprobes));
     NWB_CU(cudaMemcpy(s->dprobe_off, node_offset, sizeof(long long) * nprobes, cudaMemcpyHostToDevice));
     NWB_CU(cudaMemcpy(s->dprobe_w, weights, sizeof(double) * N3 * static_cast<size_t>(nprobes),
                       cudaMemcpyHostToDevice));
@@ -909,12 +918,14 @@ nwb_status nwb_probe_read(nwb_solver* s, double* out) {
     if (!s || !out) return fail(NWB_EINVAL, "nwb_probe_read: null argument");
     if (s->nprobes == 0) return fail(NWB_EINVAL, "nwb_probe_read: no probes set up");
     cudaError_t e = nwb::launch_probes(s->u[s->cur], s->stride, s->N * s->N * s->N, s->dprobe_off,
-                                       s->dprobe_w, s->nprobes, s->dprobe_out, s->st);
+                                       s->dprobe_w, s->nprobes,
+                                       s->dprobe_out ? s->dprobe_out : s->dw->probes, s->st);
     if (e != cudaSuccess) return fail(NWB_ECUDA, "probe kernel: %s", cudaGetErrorString(e));
     ++s->launches;
-    NWB_CU(cudaMemcpyAsync(out, s->dprobe_out, sizeof(double) * 6 * s->nprobes, cudaMemcpyDeviceToHost,
-                           s->st));
+    const size_t bytes = sizeof(double) * 6 * s->nprobes;
+    if (s->dprobe_out) NWB_CU(cudaMemcpyAsync(out, s->dprobe_out, bytes, cudaMemcpyDeviceToHost, s->st));
     NWB_CU(cudaStreamSynchronize(s->st));
+    if (!s->dprobe_out) std::memcpy(out, s->hw->probes, bytes);
     return NWB_OK;
 }
 
