@@ -411,13 +411,14 @@ __device__ __forceinline__ bool wants_energy(const SlotDev& S, int post) {
 
 // Energy partial of each tile, fixed order within the tile.
 __global__ void __launch_bounds__(256)
-batch_diag_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
-                  const int* __restrict__ ntiles_p, int post, int only_slot) {
-    const int ntiles = *ntiles_p;
+batch_diag_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work, int ntiles_v,
+                  const int* __restrict__ ntiles_p, int post) {
+    stage::grid_launch_dependents();
+    stage::grid_wait();
+    const int ntiles = ntiles_p ? *ntiles_p : ntiles_v;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int t = blockIdx.x * 8 + warp; t < ntiles; t += gridDim.x * 8) {
         const WorkItem w = work[t];
-        if (only_slot >= 0 && w.slot != only_slot) continue;
         const SlotDev& S = slots[w.slot];
         if (!(S.active || !post) || !wants_energy(S, post)) continue;
         const double* u = S.u[post ? (S.par ^ 1) : S.par];
@@ -447,12 +448,11 @@ batch_diag_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict_
 // the element's nodes, as ProbeManager::record does on the host,
 // src/probe.cpp:192-216), then thread 0 advances the slot's step bookkeeping.
 __global__ void __launch_bounds__(32 * (kMaxProbes + 1))
-batch_epilogue_kernel(SlotDev* __restrict__ slots, int nslots, int post, int only_slot,
+batch_epilogue_kernel(SlotDev* __restrict__ slots, const int* __restrict__ slot_list, int first_slot, int post,
                       int* __restrict__ counters) {
-    if (blockIdx.x == 0 && threadIdx.x < 8 && post) counters[threadIdx.x] = 0;
-    const int s = blockIdx.x;
-    if (s >= nslots || (only_slot >= 0 && s != only_slot)) return;
-    SlotDev& S = slots[s];
+    stage::grid_wait();
+    if (blockIdx.x == 0 && threadIdx.x < 8 && counters) counters[threadIdx.x] = 0;
+    SlotDev& S = slots[slot_list ? slot_list[blockIdx.x] : first_slot + static_cast<int>(blockIdx.x)];
     if (post && !S.active) return;
     if (!post && !S.u[0]) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -624,18 +624,16 @@ cudaError_t launch_box_pulse(const BoxPulse& b, double* u, long long stride, cud
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_diag(SlotDev* slots, const WorkItem* work, const int* ntiles, int post,
-                              int only_slot, int grid, cudaStream_t st) {
-    batch_diag_kernel<<<grid, 256, 0, st>>>(slots, work, ntiles, post, only_slot);
-    return cudaGetLastError();
+cudaError_t launch_batch_diag(SlotDev* slots, const WorkItem* work, int ntiles, const int* ntiles_p, int post,
+                              int grid, bool overlap, cudaStream_t st) {
+    return launch_overlapped(batch_diag_kernel, grid, 256, 0, st, overlap, slots, work, ntiles, ntiles_p, post);
 }
 
-cudaError_t launch_batch_epilogue(SlotDev* slots, int nslots, int post, int only_slot,
-                                  int* counters, cudaStream_t st) {
+cudaError_t launch_batch_epilogue(SlotDev* slots, const int* slot_list, int first_slot, int nslots, int post,
+                                  int* counters, bool overlap, cudaStream_t st) {
     if (nslots < 1) return cudaSuccess;
-    batch_epilogue_kernel<<<nslots, 32 * (kMaxProbes + 1), 0, st>>>(slots, nslots, post, only_slot,
-                                                                  counters);
-    return cudaGetLastError();
+    return launch_overlapped(batch_epilogue_kernel, nslots, 32 * (kMaxProbes + 1), 0, st, overlap, slots, slot_list,
+                             first_slot, post, counters);
 }
 
 }  // namespace nwb

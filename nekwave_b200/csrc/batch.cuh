@@ -61,15 +61,16 @@ cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots
                                  const WorkItem* work, int ntiles, int dry, const double* Dh,
                                  cudaStream_t st);
 int batch_epb_n(int N, int f32);
-// Diagnostics after a step (post = 1) or of the initial state (post = 0):
-// energy partials per tile and probe values into the slots' history buffers.
-// only_slot >= 0 restricts the work to one slot (initial-state diagnostics).
-cudaError_t launch_batch_diag(SlotDev* slots, const WorkItem* work, const int* ntiles, int post,
-                              int only_slot, int grid, cudaStream_t st);
-// End of step: per-slot energy sum (fixed order), parity flip, step count,
-// completion; resets the stage counters.
-cudaError_t launch_batch_epilogue(SlotDev* slots, int nslots, int post, int only_slot,
-                                  int* counters, cudaStream_t st);
+// Diagnostics after a step (post = 1) or of the initial state (post = 0): energy
+// partials per tile of the work items [work, work + ntiles) (ntiles_p, when given: their
+// number on the device).  overlap: see launch_overlapped.
+cudaError_t launch_batch_diag(SlotDev* slots, const WorkItem* work, int ntiles, const int* ntiles_p, int post,
+                              int grid, bool overlap, cudaStream_t st);
+// End of step of nslots slots (slot_list[0..nslots), or first_slot..): per-slot energy sum
+// (fixed order), probe values, parity flip, step count, completion; resets the stage
+// counters (when given).
+cudaError_t launch_batch_epilogue(SlotDev* slots, const int* slot_list, int first_slot, int nslots, int post,
+                                  int* counters, bool overlap, cudaStream_t st);
 // Gaussian pulses on the nodes of an axis-aligned box cavity: component c gets
 // pulse[c*5+0] * exp(-|x - (pulse[c*5+1..3])|^2 / pulse[c*5+4]^2) (zero where
 // pulse[c*5+4] <= 0), node positions from the box's uniform element grid.
