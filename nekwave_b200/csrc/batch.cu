@@ -199,7 +199,18 @@ __device__ __forceinline__ StageParams slot_params(const SlotDev& S, const Batch
 // D of one N by value, for the constant-bank form of the per-N kernels.
 struct DParam {
     double d[100];
+    float f[100];  // rounded to FP32 (FP32-bulk)
 };
+
+// D of one N by value (null: zeros, for kernels that take it from shared memory).
+DParam d_param(int N, const double* Dh) {
+    DParam dp{};
+    for (int x = 0; Dh && x < N * N; ++x) {
+        dp.d[x] = Dh[x];
+        dp.f[x] = static_cast<float>(Dh[x]);
+    }
+    return dp;
+}
 
 // One block per tile of one N: the single-mesh kernel's tuned shape for that N,
 // fully unrolled, reading its slot from the work item (per-N mode).  ALG 0 is the
@@ -256,20 +267,15 @@ cudaError_t launch_dmma8_n(const BatchStage& bs, const SlotDev* slots, const Wor
     return launch_overlapped(kern, ntiles, 128, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
-// Per-N shapes of the per-N mode: the single-mesh defaults (stage_variants.h entry
-// 0), with the persistent form of N = 4 replaced by its one-tile-per-block form.
-// N = 8 in FP64 runs batch_dmma8_kernel instead (NShape<8> is its FP32-bulk shape).
-// An ALG with CONSTD runs without it for an N whose cavities do not all share the
-// pool's D for that N (same arithmetic, D from shared memory).
+// Per-N shapes of the per-N mode where neither the bulk-copy form (NBulk, F32Shape) nor the
+// tensor-core tile runs: the single-mesh defaults (stage_variants.h entry 0) at 2, 3 and 10
+// points, and at 4 points in FP64 with the persistent form replaced by its
+// one-tile-per-block form.  An ALG with CONSTD runs without it for an N whose cavities do
+// not all share the pool's D for that N (same arithmetic, D from shared memory).
 template <int N> struct NShape;
 template <> struct NShape<2> { static constexpr int KS = 2, EPB = 16, KSM = 1, MINB = 1, ALG = 0; };
 template <> struct NShape<3> { static constexpr int KS = 1, EPB = 16, KSM = 0, MINB = 4, ALG = 0; };
 template <> struct NShape<4> { static constexpr int KS = 2, EPB = 4, KSM = 0, MINB = 4, ALG = 12; };
-template <> struct NShape<5> { static constexpr int KS = 2, EPB = 2, KSM = 0, MINB = 4, ALG = 4; };
-template <> struct NShape<6> { static constexpr int KS = 2, EPB = 2, KSM = 0, MINB = 3, ALG = 4; };
-template <> struct NShape<7> { static constexpr int KS = 2, EPB = 1, KSM = 0, MINB = 4, ALG = 12; };
-template <> struct NShape<8> { static constexpr int KS = 2, EPB = 1, KSM = 0, MINB = 4, ALG = 12; };
-template <> struct NShape<9> { static constexpr int KS = 2, EPB = 1, KSM = 0, MINB = 2, ALG = 12; };
 template <> struct NShape<10> { static constexpr int KS = 2, EPB = 1, KSM = 0, MINB = 2, ALG = 0; };
 
 // FP64 per-N shapes that run the bulk-copy one-tile form (the single-mesh default
@@ -335,6 +341,37 @@ cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const Work
     return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
+// FP32-bulk, per-N mode: the single-mesh form (stage::F32Shape), D from dp (CD) or from
+// shared memory.
+template <int N, bool CD>
+__global__ void __launch_bounds__(stage::F32Shape<N>::EPB * 2 * N * N, stage::F32Shape<N>::MINB)
+batch_f32_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
+                   const __grid_constant__ BatchStage bs, const __grid_constant__ DParam dp) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    using Sh = stage::F32Shape<N>;
+    const WorkItem w = work[blockIdx.x];
+    const SlotDev& S = slots[w.slot];
+    if (!S.active) {
+        stage::grid_wait();
+        return;
+    }
+    const StageParams P = slot_params(S, bs);
+    stage::bulk_tile<N, GEO_BOX, 2, Sh::EPB, CD && Sh::CD != 0, false, Sh::KSM != 0, true, false, false, true>(
+        P, w.e0, smem, threadIdx.x, dp.d, stage::NoPull(), dp.f);
+}
+
+template <int N, bool CD>
+cudaError_t launch_f32_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                         const DParam& dp, cudaStream_t st) {
+    using Sh = stage::F32Shape<N>;
+    constexpr int smem = stage::BulkLayout<N, Sh::EPB, Sh::KSM != 0, GEO_BOX, true>::total;
+    auto kern = batch_f32_n_kernel<N, CD>;
+    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
+    if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
+    if (ntiles <= 0) return cudaSuccess;
+    return launch_overlapped(kern, ntiles, Sh::EPB * 2 * N * N, smem, st, bs.overlap(), slots, work, bs, dp);
+}
+
 template <int N, bool F32, int ALG>
 cudaError_t launch_n_alg(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                          const DParam& dp, cudaStream_t st) {
@@ -355,50 +392,48 @@ cudaError_t launch_n_alg(const BatchStage& bs, const SlotDev* slots, const WorkI
 // constant-bank form then applies), else null.
 template <int N, bool F32>
 cudaError_t launch_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
-                     const double* Dh, cudaStream_t st, int* epb_out) {
-    using Sh = NShape<N>;
-    if (epb_out) *epb_out = (NBulk<N>::on && !F32) ? NBulk<N>::EPB : Sh::EPB;
-    if constexpr (NBulk<N>::on && !F32) {
-        DParam dp{};
+                     const double* Dh, cudaStream_t st) {
+    if constexpr (stage::F32Shape<N>::on && F32) {
+        const DParam dp = d_param(N, Dh);
+        if (Dh) return launch_f32_n<N, true>(bs, slots, work, ntiles, dp, st);
+        if (ntiles <= 0) {  // set-up call: prepare both forms
+            cudaError_t e = launch_f32_n<N, true>(bs, slots, work, 0, dp, st);
+            if (e != cudaSuccess) return e;
+        }
+        return launch_f32_n<N, false>(bs, slots, work, ntiles, dp, st);
+    } else if constexpr (NBulk<N>::on && !F32) {
+        const DParam dp = d_param(N, Dh);
         if constexpr (NBulk<N>::CD) {
-            if (Dh) {
-                for (int x = 0; x < N * N; ++x) dp.d[x] = Dh[x];
-                return launch_bulk_n<N, true>(bs, slots, work, ntiles, dp, st);
-            }
+            if (Dh) return launch_bulk_n<N, true>(bs, slots, work, ntiles, dp, st);
             if (ntiles <= 0) {  // set-up call: prepare both forms
                 cudaError_t e = launch_bulk_n<N, true>(bs, slots, work, 0, dp, st);
                 if (e != cudaSuccess) return e;
             }
         }
         return launch_bulk_n<N, false>(bs, slots, work, ntiles, dp, st);
-    }
-    if constexpr (dmma_tile<N, F32>()) {
-        DParam dp{};
-        if (Dh) {
-            for (int x = 0; x < N * N; ++x) dp.d[x] = Dh[x];
-            return launch_dmma8_n<true>(bs, slots, work, ntiles, dp, st);
-        }
+    } else if constexpr (dmma_tile<N, F32>()) {
+        const DParam dp = d_param(N, Dh);
+        if (Dh) return launch_dmma8_n<true>(bs, slots, work, ntiles, dp, st);
         if (ntiles <= 0) {  // set-up call: prepare both forms
             cudaError_t e = launch_dmma8_n<true>(bs, slots, work, 0, dp, st);
             if (e != cudaSuccess) return e;
         }
         return launch_dmma8_n<false>(bs, slots, work, ntiles, dp, st);
-    }
-    constexpr bool cd_bit = Sh::ALG >= 2 && ((Sh::ALG - 2) & 8) != 0;
-    constexpr bool has_cd = cd_bit && !F32;  // the constant-bank D is an FP64 form
-    constexpr int ALG_PLAIN = cd_bit ? Sh::ALG - 8 : Sh::ALG;
-    DParam dp{};
-    if constexpr (has_cd) {
-        if (Dh) {
-            for (int x = 0; x < N * N; ++x) dp.d[x] = Dh[x];
-            return launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, ntiles, dp, st);
+    } else {
+        using Sh = NShape<N>;
+        constexpr bool cd_bit = Sh::ALG >= 2 && ((Sh::ALG - 2) & 8) != 0;
+        constexpr bool has_cd = cd_bit && !F32;  // the constant-bank D is an FP64 form
+        constexpr int ALG_PLAIN = cd_bit ? Sh::ALG - 8 : Sh::ALG;
+        const DParam dp = d_param(N, Dh);
+        if constexpr (has_cd) {
+            if (Dh) return launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, ntiles, dp, st);
+            if (ntiles <= 0) {  // set-up call: prepare both forms
+                cudaError_t e = launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, 0, dp, st);
+                if (e != cudaSuccess) return e;
+            }
         }
-        if (ntiles <= 0) {  // set-up call: prepare both forms
-            cudaError_t e = launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, 0, dp, st);
-            if (e != cudaSuccess) return e;
-        }
+        return launch_n_alg<N, F32, ALG_PLAIN>(bs, slots, work, ntiles, dp, st);
     }
-    return launch_n_alg<N, F32, ALG_PLAIN>(bs, slots, work, ntiles, dp, st);
 }
 
 // Does this slot record energy after the step it is taking now (post = 1), or
@@ -544,8 +579,8 @@ cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots
     const BatchStage bs{dry ? 0.0 : kRk4a[stage], dry ? 0.0 : kRk4b[stage], stage, dry};
     switch (N) {
 #define NWB_CASE(n) \
-        case n: return f32 ? launch_n<n, true>(bs, slots, work, ntiles, Dh, st, nullptr) \
-                           : launch_n<n, false>(bs, slots, work, ntiles, Dh, st, nullptr);
+        case n: return f32 ? launch_n<n, true>(bs, slots, work, ntiles, Dh, st) \
+                           : launch_n<n, false>(bs, slots, work, ntiles, Dh, st);
         NWB_CASE(2) NWB_CASE(3) NWB_CASE(4) NWB_CASE(5) NWB_CASE(6) NWB_CASE(7) NWB_CASE(8)
         NWB_CASE(9) NWB_CASE(10)
 #undef NWB_CASE
@@ -556,7 +591,10 @@ cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots
 namespace {
 template <int N>
 int epb_n(int f32) {
-    return (NBulk<N>::on && !f32) ? NBulk<N>::EPB : NShape<N>::EPB;
+    if constexpr (N == 8) return f32 ? stage::F32Shape<N>::EPB : 1;  // FP64: one element per block
+    else if constexpr (NBulk<N>::on) return f32 ? stage::F32Shape<N>::EPB : NBulk<N>::EPB;
+    else if constexpr (stage::F32Shape<N>::on) return f32 ? stage::F32Shape<N>::EPB : NShape<N>::EPB;
+    else return NShape<N>::EPB;
 }
 }  // namespace
 

@@ -363,7 +363,10 @@ struct nwb_solver {
         P.b = kRK4B[stage];
         P.kio = nwb::stage_kio(stage) | nwb::kOverlap;
         P.dt = dt;
-        for (int x = 0; x < N * N; ++x) P.Dc[x] = hD[x];
+        for (int x = 0; x < N * N; ++x) {
+            P.Dc[x] = hD[x];
+            P.Dcf[x] = static_cast<float>(hD[x]);
+        }
         for (int x = 0; x < N; ++x) P.zl[x] = hzl[x];
         for (int d = 0; d < 3; ++d) P.snel[d] = snel[d];
         P.spmask = spmask;

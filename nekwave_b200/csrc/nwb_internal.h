@@ -136,6 +136,7 @@ struct StageParams {
     double a, b, dt;        // LSRK45 stage coefficients and step
     int snel[3];            // structured box mesh: elements per axis (x fastest), or 0
     int spmask;             // structured box mesh: periodic axes (bit 0 x, 1 y, 2 z)
+    float Dcf[100];         // D rounded to FP32, by value (FP32-bulk)
     double Dc[100];         // D again, by value: kernels that index it with constants
                             // read it as an operand from the parameter bank
     double zl[10];          // line coordinates: D zl = 1, zl[0] = -1 (the GLL nodes for

@@ -93,7 +93,7 @@ __device__ __forceinline__ void report(const StageParams& P, int code) {
 
 // Shared-memory layout of one tile: u_in (and with KSM k) [6][CSR] doubles with
 // slack, geometry, connections, D, the lifted fluxes, the mbarrier and a flag.
-template <int N, int EPB, bool KSM, int GEO = GEO_BOX>
+template <int N, int EPB, bool KSM, int GEO = GEO_BOX, bool F32 = false>
 struct BulkLayout {
     static constexpr int N2 = N * N, N3 = N2 * N;
     static constexpr int CSR = (EPB * N3 + 2 + 1) / 2 * 2;
@@ -106,7 +106,9 @@ struct BulkLayout {
     static constexpr int conn_b = align16((EPB * 6 + 6) * 4);
     static constexpr int D = conn0 + conn_b;
     static constexpr int flux0 = D + align16(N2 * 8);
-    static constexpr int bar = flux0 + EPB * flux_planes<GEO, true>() * N2 * 8;
+    // FP32-bulk: the deviations, the fit and the maxima (as Layout2::uc)
+    static constexpr int uc = flux0 + EPB * flux_planes<GEO, true>() * N2 * 8;
+    static constexpr int bar = uc + (F32 ? align16(6 * CSR * 4) + align16((EPB * 30 + 10) * 8) + align16(EPB * 8) : 0);
     static constexpr int flag = bar + 8;
     static constexpr int total = flag + 16;
 };
@@ -115,9 +117,9 @@ struct BulkLayout {
 // lines are prefetched into L2), geometry and connections as bulk copies that
 // complete on the mbarrier at smem + L::bar, which must be initialised.  Waits for the
 // launches before this one (grid_wait) ahead of the first access to u and k.
-template <int N, int EPB, bool KSM, int GEO>
+template <int N, int EPB, bool KSM, int GEO, bool F32>
 __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, unsigned char* smem) {
-    using L = BulkLayout<N, EPB, KSM, GEO>;
+    using L = BulkLayout<N, EPB, KSM, GEO, F32>;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     const long long S = P.stride;
     const long long g0 = static_cast<long long>(e0) * L::N3;
@@ -160,9 +162,9 @@ __device__ __forceinline__ void bulk_issue(const StageParams& P, const int e0, u
 // Every thread's wait for the tile issued by bulk_issue: true when it is resident.
 // On expiry thread 0 records the code, waits once more (bounded) for the copies so
 // that none lands in a finished block, and every thread gets false.
-template <int N, int EPB, bool KSM, int GEO>
+template <int N, int EPB, bool KSM, int GEO, bool F32>
 __device__ __forceinline__ bool bulk_wait_tile(const StageParams& P, unsigned char* smem, const int tid) {
-    using L = BulkLayout<N, EPB, KSM, GEO>;
+    using L = BulkLayout<N, EPB, KSM, GEO, F32>;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     int* flag = reinterpret_cast<int*>(smem + L::flag);
     if (tid == 0) *flag = mbar_wait(bar, 0) ? 1 : 0;
@@ -187,10 +189,11 @@ __device__ __forceinline__ bool bulk_wait_tile(const StageParams& P, unsigned ch
 // right after it has issued the tile's copies (NoPull, or a functor that pulls a
 // later block's tile into L2).
 template <int N, int GEO, int KS, int EPB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
-          bool VROW = false, bool ILP2 = false, class Pull = NoPull>
+          bool VROW = false, bool ILP2 = false, bool F32 = false, class Pull = NoPull>
 __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, unsigned char* smem,
-                                          const int tid, const double* Dc, const Pull& pull = Pull()) {
-    using L = BulkLayout<N, EPB, KSM, GEO>;
+                                          const int tid, const double* Dc, const Pull& pull = Pull(),
+                                          const float* Dcf = nullptr) {
+    using L = BulkLayout<N, EPB, KSM, GEO, F32>;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::bar);
     double* sD = reinterpret_cast<double*>(smem + L::D);
     grid_launch_dependents();
@@ -199,7 +202,7 @@ __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, un
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_fence_init();
-        bulk_issue<N, EPB, KSM, GEO>(P, e0, smem);
+        bulk_issue<N, EPB, KSM, GEO, F32>(P, e0, smem);
         pull();
     }
     const long long g0 = static_cast<long long>(e0) * L::N3;
@@ -208,16 +211,16 @@ __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, un
     if constexpr (EARLY && GEO != GEO_BOX) gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
     grid_wait();
     if constexpr (EARLY && GEO == GEO_BOX) gather_box_values<N, KS, EPB, false, false>(P, e0, nullptr, tid, G);
-    if (!bulk_wait_tile<N, EPB, KSM, GEO>(P, smem, tid)) return;
+    if (!bulk_wait_tile<N, EPB, KSM, GEO, F32>(P, smem, tid)) return;
     const int off = static_cast<int>(g0 & 1);
     const double* su = reinterpret_cast<const double*>(smem + L::u0) + off;
     const double* sk = KSM ? reinterpret_cast<const double*>(smem + L::k0) + off : nullptr;
     const ElemGeo* sg = reinterpret_cast<const ElemGeo*>(smem + L::geo0);
     const int* sc = reinterpret_cast<const int*>(smem + L::conn0) + ((e0 * 6) & 3);
     double* sflux = reinterpret_cast<double*>(smem + L::flux0);
-    compute2<N, GEO, false, KS, EPB, true, false, CONSTD, EARLY, false, DSMEM, CtaBar, L::CSR, KSM, VROW,
+    compute2<N, GEO, F32, KS, EPB, true, false, CONSTD, EARLY, false, DSMEM, CtaBar, L::CSR, KSM, VROW,
              ILP2>(
-        P, e0, su, sg, sc, sD, sflux, nullptr, tid, G, Dc, CtaBar(), sk);
+        P, e0, su, sg, sc, sD, sflux, smem + L::uc, tid, G, Dc, CtaBar(), sk, Dcf);
 }
 
 // Tile taken by block b.  ZCOL on a structured box whose rows hold whole tiles:
@@ -258,24 +261,25 @@ struct MeshPull {
 // instead of DRAM; 0: no pull.  On B200 this pays where few blocks are resident
 // (6 and 9 points: 3 and 2 per SM), whose tile waits the other blocks hide least.
 template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
-          bool ZCOL, bool VROW, bool ILP2, int AHEAD>
+          bool ZCOL, bool VROW, bool ILP2, int AHEAD, bool F32>
 __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     stage_bulk_kernel(const __grid_constant__ StageParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int t = bulk_tile_index<EPB, ZCOL>(P, blockIdx.x);
     if constexpr (AHEAD > 0)
-        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2>(
-            P, t * EPB, smem, threadIdx.x, P.Dc, MeshPull<N * N * N, EPB, MINB, AHEAD, ZCOL>{P});
+        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2, F32>(
+            P, t * EPB, smem, threadIdx.x, P.Dc, MeshPull<N * N * N, EPB, MINB, AHEAD, ZCOL>{P}, P.Dcf);
     else
-        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2>(P, t * EPB, smem, threadIdx.x, P.Dc);
+        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2, F32>(P, t * EPB, smem, threadIdx.x, P.Dc,
+                                                                              NoPull(), P.Dcf);
 }
 
 template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
-          bool ZCOL, bool VROW, bool ILP2, int AHEAD = 0>
+          bool ZCOL, bool VROW, bool ILP2, int AHEAD = 0, bool F32 = false>
 cudaError_t launch_bulk(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
-    using L = BulkLayout<N, EPB, KSM, GEO>;
+    using L = BulkLayout<N, EPB, KSM, GEO, F32>;
     constexpr int threads = EPB * KS * N * N;
-    auto kern = stage_bulk_kernel<N, GEO, KS, EPB, MINB, CONSTD, DSMEM, KSM, EARLY, ZCOL, VROW, ILP2, AHEAD>;
+    auto kern = stage_bulk_kernel<N, GEO, KS, EPB, MINB, CONSTD, DSMEM, KSM, EARLY, ZCOL, VROW, ILP2, AHEAD, F32>;
     if (cfg) *cfg = StageConfig{KS, EPB, threads, L::total, KSM ? 1 : 0, MINB};
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, L::total, attr_set); e != cudaSuccess) return e;
@@ -311,6 +315,30 @@ cudaError_t launch_general(const StageParams* p, cudaStream_t st, StageConfig* c
     using Sh = GeneralShape<N>;
     constexpr bool cd = (GEO == GEO_NODAL ? Sh::CDN : Sh::CDA) != 0;
     return launch_bulk<N, GEO, 2, Sh::EPB, Sh::MINB, cd, false, true, true, false, false, false>(p, st, cfg);
+}
+
+// Shapes of the axis-aligned class in FP32-bulk at 4 to 9 points (on): the bulk-copy tile
+// with the same arithmetic as before.  Beside u_in the tile holds its FP32 copy; the column
+// phase's FP64 loop serves the elements that fall back, most of them in the benchmark's
+// fields, so it takes its D rows in registers and (CD) the unrolled loop of the FP64 class
+// (with its D rows read from shared memory at each use it did more than twice the shared
+// loads of the FP64 class).  k in shared memory (KSM) only at 5 points: elsewhere it costs
+// a resident block.  From a sweep of four shapes per N.  B200, per step, before -> now:
+// 25^3 elements of 8 points 1917 -> 1623 us, 34^3 of 6 points 2452 -> 2019 us, 22^3 of 9 points
+// 2631 -> 1750 us, 40^3 of 5 points 2569 -> 2122 us.
+template <int N> struct F32Shape { static constexpr bool on = false; static constexpr int EPB = 1, MINB = 1, KSM = 0, CD = 0; };
+template <> struct F32Shape<4> { static constexpr bool on = true; static constexpr int EPB = 2, MINB = 8, KSM = 0, CD = 1; };
+template <> struct F32Shape<5> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 8, KSM = 1, CD = 1; };
+template <> struct F32Shape<6> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 5, KSM = 0, CD = 1; };
+template <> struct F32Shape<7> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 4, KSM = 0, CD = 1; };
+template <> struct F32Shape<8> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 4, KSM = 0, CD = 0; };
+template <> struct F32Shape<9> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 2, KSM = 0, CD = 1; };
+
+template <int N>
+cudaError_t launch_f32(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
+    using Sh = F32Shape<N>;
+    return launch_bulk<N, GEO_BOX, 2, Sh::EPB, Sh::MINB, Sh::CD != 0, false, Sh::KSM != 0, true, false, false, false, 0,
+                       true>(p, st, cfg);
 }
 
 }  // namespace stage

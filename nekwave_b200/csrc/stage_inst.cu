@@ -64,7 +64,9 @@ cudaError_t launch_variant(int vid, const StageParams* p, cudaStream_t st, Stage
     } else if constexpr (I < kNumShapes) {
         if (vid == I) {
             constexpr Shape v = kShapes[I];
-            if constexpr (v.alg == 1) {
+            if constexpr (GEO == GEO_BOX && F32 && I == kFirstGeneral && F32Shape<NWB_N>::on) {
+                return launch_f32<NWB_N>(p, st, cfg);  // variant 0 in FP32-bulk
+            } else if constexpr (v.alg == 1) {
                 if constexpr (GEO == GEO_BOX && !F32 && NWB_N == 8)
                     return launch_mma8<v.minb>(p, st, cfg);
                 else

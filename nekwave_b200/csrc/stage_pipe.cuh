@@ -848,7 +848,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
                                          double* sflux, unsigned char* smem_uc, const int tid,
                                          FaceRegs<N, GEO, KS, SPLIT>& G,
                                          const double* __restrict__ Dc = nullptr, Bar bar = Bar(),
-                                         const double* sk = nullptr) {
+                                         const double* sk = nullptr, const float* Dcf = nullptr) {
     using TC = typename std::conditional<F32, float, double>::type;
     constexpr int N2 = N * N, N3 = N2 * N;
     constexpr int RP = PAD ? N + 1 : N;              // row pitch in shared memory
@@ -859,10 +859,9 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     constexpr int KPT = (N + KS - 1) / KS;
     constexpr int CS = CSX ? CSX : EPB * EN3;
     constexpr bool BOXF = box_faces<GEO, SPLIT>();
-    static_assert(CSX == 0 || !F32, "tiles with slack: FP64 only");
-    static_assert(!KSM || (!PAD && !F32), "k in shared memory: unpadded FP64 tiles");
+    static_assert(!KSM || !PAD, "k in shared memory: unpadded tiles");
     static_assert(!SPLIT || KS == 1 || KS == 2, "the field split: one or two threads per column");
-    static_assert(!CONSTD || (SPLIT && !F32), "constant-bank D: FP64 field split only");
+    static_assert(!CONSTD || SPLIT, "constant-bank D: field split only");
     static_assert(!VROW || (SPLIT && !F32 && !PAD && CSX % 2 == 0), "row pairs: FP64 split, unpadded");
 
     const int team = tid / TPE;
@@ -910,7 +909,6 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         s_fb = reinterpret_cast<unsigned*>(szl + 10);
         if (tid < 2 * EPB) s_fb[tid] = 0u;  // formed in (c), after the face phase's barrier
         constexpr int ic = N / 2;
-        const double inv = 1.0 / (P.zl[N - 1] - P.zl[0]);
         const int nlin = tid < NT ? nvalid * 6 : 0;
         if (tid == 0) {
             // constant indices: a runtime index would move a caller's local P into
@@ -920,6 +918,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         }
         // (a) centre value and slopes of each component
         for (int x = tid; x < nlin; x += NT) {
+            const double inv = 1.0 / (P.zl[N - 1] - P.zl[0]);
             const int el = x / 6, c = x - 6 * el;
             const double* U = su + c * CS + el * EN3;
             double* Lc = lin + el * LIN + 4 * c;
@@ -931,6 +930,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         // (b) curl of L with the residual's sign: +curl H_L for E, -curl E_L for H
         // (physical gradient = J^-T applied to the slopes; met = rx,sx,tx,ry,...,tz)
         for (int x = tid; x < nlin; x += NT) {
+            const double inv = 1.0 / (P.zl[N - 1] - P.zl[0]);
             const int el = x / 6, rc = x - 6 * el;
             const int fld = rc / 3, q = rc - 3 * fld;
             const int o = fld == 0 ? 3 : 0;  // the differentiated field
@@ -963,16 +963,64 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     }
     bar.sync();
 
+    // FP32-bulk: does this thread's element run the FP64 column arithmetic?
+    bool fb64 = false;
     if constexpr (F32 && GEO != GEO_NODAL) {
-        // (c) FP32-bulk deviations w = u - L: each thread takes its own node column
-        // (i, j) of its element, planes h, h + KS, ... (the fit is complete: it was
-        // formed before the face phase's barrier)
+        // (c) The largest deviation |u - L| and the largest variation |u - centre| of the
+        // element, each thread over its node column (i, j), planes h, h + KS, ... (the fit
+        // is complete: it was formed before the face phase's barrier).  Both maxima are
+        // taken in FP64 and rounded to FP32 once (rounding is monotone).  An element whose
+        // deviations are not small against its variation (a field resolved within one or
+        // two elements, where the fit removes little; in the benchmark's fields most
+        // elements, as the tails of a pulse are exponentials) runs the FP64 arithmetic on
+        // u itself: its FP32 rounding would not shrink with the deviations there.  The
+        // FP32 copy is made after that decision, for the elements that use it.
+        const double* szl = s_lin + EPB * LIN;
+        constexpr int ic = N / 2;
+        const double zi = szl[i] - szl[ic], zj = szl[j] - szl[ic];
         if (active) {
+            double wm = 0.0, vm = 0.0;
+            double dz[KPT];
+#pragma unroll
+            for (int k = 0; k < N; k += KS) dz[k / KS] = szl[min(k + h, N - 1)] - szl[ic];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                const double* Lc = s_lin + team * LIN + 4 * c;
+                const double centre = Lc[0], at = Lc[3];
+                const double base = Lc[0] + Lc[1] * zi + Lc[2] * zj;
+                const int col = c * CS + team * EN3 + i + RP * j;
+#pragma unroll
+                for (int k = 0; k < N; k += KS) {
+                    if (k + h >= N) break;
+                    const double uv = su[col + PP * (k + h)];
+                    const double Lv = base + at * dz[k / KS];
+                    const double w = fabs(uv - Lv), v = fabs(uv - centre);
+                    if (w > wm) wm = w;
+                    if (v > vm) vm = v;
+                }
+            }
+            // non-negative floats order as their bit patterns
+            unsigned wb = __float_as_uint(static_cast<float>(wm)), vb = __float_as_uint(static_cast<float>(vm));
+            if constexpr (EPB == 1) {  // a warp's threads share the element: one atomic a warp
+                const unsigned lanes = __activemask();
+                wb = __reduce_max_sync(lanes, wb);
+                vb = __reduce_max_sync(lanes, vb);
+                if ((tid & 31) == __ffs(lanes) - 1) {
+                    atomicMax(s_fb, wb);
+                    atomicMax(s_fb + 1, vb);
+                }
+            } else {
+                atomicMax(s_fb + 2 * team, wb);
+                atomicMax(s_fb + 2 * team + 1, vb);
+            }
+        }
+        bar.sync();
+        const int tm = EPB == 1 ? 0 : (active ? team : 0);
+        fb64 = __uint_as_float(s_fb[2 * tm]) > kFp64Fallback * __uint_as_float(s_fb[2 * tm + 1]);
+        // the deviations w = u - L in FP32
+        if constexpr (!SPLIT) fb64 = false;  // the forms without the split have no FP64 loop
+        if (active && !fb64) {
             TC* w = reinterpret_cast<TC*>(smem_uc);
-            const double* szl = s_lin + EPB * LIN;
-            constexpr int ic = N / 2;
-            const double zi = szl[i] - szl[ic], zj = szl[j] - szl[ic];
-            float wmax = 0.f, vmax = 0.f;
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 const double* Lc = s_lin + team * LIN + 4 * c;
@@ -981,17 +1029,11 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
                 const int col = c * CS + team * EN3 + i + RP * j;
                 for (int k = h; k < N; k += KS) {
                     const double Lv = base + at * (szl[k] - szl[ic]);
-                    const float wv = static_cast<float>(su[col + PP * k] - Lv);
-                    w[col + PP * k] = wv;
-                    wmax = fmaxf(wmax, fabsf(wv));
-                    vmax = fmaxf(vmax, fabsf(static_cast<float>(su[col + PP * k] - Lc[0])));
+                    w[col + PP * k] = static_cast<float>(su[col + PP * k] - Lv);
                 }
             }
-            // non-negative floats order as their bit patterns
-            atomicMax(s_fb + 2 * team, __float_as_uint(wmax));
-            atomicMax(s_fb + 2 * team + 1, __float_as_uint(vmax));
         }
-        bar.sync();
+        if (EPB > 1 || !fb64) bar.sync();  // one element per block: a uniform choice
     }
 
     // ---- column phase: volume curl + face terms + LSRK update ------------------
@@ -999,40 +1041,38 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     const TC* U = s_uc + team * EN3;
     const double* Uf = su + team * EN3;
     const double* Fl = sflux + team * flux_planes<GEO, SPLIT>() * N2;
-    TC Dr[N], Ds[N];
-#pragma unroll
-    for (int l = 0; l < N; ++l) {
-        Dr[l] = static_cast<TC>(sD[i + l * N]);
-        Ds[l] = static_cast<TC>(sD[j + l * N]);
-    }
-    TC m_[9];
-    if constexpr (GEO != GEO_NODAL) {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) m_[c] = static_cast<TC>(sg[team].met[c]);
-    }
     const double A = P.a, B = P.b, DT = P.dt;
     const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
     const long long ebase = static_cast<long long>(e) * N3;
 
     if constexpr (SPLIT) {
-        // FP32-bulk: an element whose deviations from its linear fit are not small
-        // against its variation (a field resolved within one or two elements, where
-        // the fit removes little) runs the FP64 arithmetic on u itself: its FP32
-        // rounding would not shrink with the deviations there.
-        bool fb64 = false;
-        if constexpr (F32 && GEO != GEO_NODAL)
-            fb64 = __uint_as_float(s_fb[2 * team]) > kFp64Fallback * __uint_as_float(s_fb[2 * team + 1]);
         // the column work in arithmetic type TX (TC, or FP64 for a fallback element)
         auto columns = [&](auto zero) {
         using TX = decltype(zero);
         constexpr bool SAME = std::is_same<TX, TC>::value;
+        // the FP64 arithmetic of either class takes the unrolled loop, FP32's stays rolled
+        constexpr bool CD = CONSTD && std::is_same<TX, double>::value;
+        // D(k, l) of the t-derivative
+        auto dtc = [&](int k, int l) -> TX {
+            if constexpr (CONSTD && F32 && SAME) return Dcf[k + l * N];
+            else if constexpr (CONSTD) return static_cast<TX>(Dc[k + l * N]);
+            else return static_cast<TX>(sD[k + l * N]);
+        };
         const TX* ubase;
         if constexpr (SAME) ubase = U;
         else ubase = Uf;
-        auto met = [&](int c) -> TX {
-            if constexpr (SAME) return m_[c];
-            else return static_cast<TX>(sg[team].met[c]);
-        };
+        TX Dr[N], Ds[N];
+#pragma unroll
+        for (int l = 0; l < N; ++l) {
+            Dr[l] = static_cast<TX>(sD[i + l * N]);
+            Ds[l] = static_cast<TX>(sD[j + l * N]);
+        }
+        TX m_[9];
+        if constexpr (GEO != GEO_NODAL) {
+#pragma unroll
+            for (int c = 0; c < 9; ++c) m_[c] = static_cast<TX>(sg[team].met[c]);
+        }
+        auto met = [&](int c) -> TX { return m_[c]; };
         // field hf = 0: E residual from V = H (+curl H); hf = 1: H residual from V = E
         // (-curl E).  KS = 2: thread h takes field h; KS = 1: one thread takes both,
         // one after the other, with the same arithmetic per node.
@@ -1087,20 +1127,20 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         }
         // KSM: k staged in shared memory with the tile's layout (unpadded)
         const double* Kf = KSM ? sk + team * EN3 : nullptr;
-        if constexpr (CONSTD) {
+        if constexpr (CD) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
                 knext[c] = !kread ? 0.0
                          : (KSM ? Kf[(dst + c) * CS + i + RP * j]
                                 : __ldcg(P.k + (dst + c) * S + ebase + i + N * j));
         }
-#pragma unroll (CONSTD ? N : 1)
+#pragma unroll (CD ? N : 1)
         for (int k = 0; k < N; ++k) {
             const int mn = i + N * j + N2 * k;           // node in natural numbering
             const int ms = i + RP * j + PP * k;          // node in shared memory
             const long long g = ebase + mn;
             double kold[3];
-            if constexpr (CONSTD) {
+            if constexpr (CD) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) kold[c] = knext[c];
                 if (k + 1 < N) {
@@ -1135,9 +1175,9 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
                 TX Wz_r = 0, Wy_r = 0, Wz_s = 0, Wx_s = 0, Wy_t = 0, Wx_t = 0;
 #pragma unroll
                 for (int l = 0; l < N; ++l) {
-                    const TX dr = (DSMEM || !SAME) ? static_cast<TX>(sD[i + l * N]) : static_cast<TX>(Dr[l]);
-                    const TX ds = (DSMEM || !SAME) ? static_cast<TX>(sD[j + l * N]) : static_cast<TX>(Ds[l]);
-                    const TX dt = CONSTD ? static_cast<TX>(Dc[k + l * N]) : static_cast<TX>(sD[k + l * N]);
+                    const TX dr = DSMEM ? static_cast<TX>(sD[i + l * N]) : Dr[l];
+                    const TX ds = DSMEM ? static_cast<TX>(sD[j + l * N]) : Ds[l];
+                    const TX dt = dtc(k, l);
                     const int is = PP * k + RP * l + i;
                     const bool odd = ILP2 && (l & 1);
                     TX& az_r = odd ? Wz_r : Vz_r; TX& ay_r = odd ? Wy_r : Vy_r;
@@ -1163,9 +1203,9 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
                 TX dr_[3] = {0, 0, 0}, ds_[3] = {0, 0, 0}, dt_[3] = {0, 0, 0};
 #pragma unroll
                 for (int l = 0; l < N; ++l) {
-                    const TX dr = (DSMEM || !SAME) ? static_cast<TX>(sD[i + l * N]) : static_cast<TX>(Dr[l]);
-                    const TX ds = (DSMEM || !SAME) ? static_cast<TX>(sD[j + l * N]) : static_cast<TX>(Ds[l]);
-                    const TX dt = CONSTD ? static_cast<TX>(Dc[k + l * N]) : static_cast<TX>(sD[k + l * N]);
+                    const TX dr = DSMEM ? static_cast<TX>(sD[i + l * N]) : Dr[l];
+                    const TX ds = DSMEM ? static_cast<TX>(sD[j + l * N]) : Ds[l];
+                    const TX dt = dtc(k, l);
                     const int ir = PP * k + RP * j + l;
                     const int is = PP * k + RP * l + i;
 #pragma unroll
@@ -1220,6 +1260,17 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
             columns(TC(0));
         }
     } else {
+        TC Dr[N], Ds[N];
+#pragma unroll
+        for (int l = 0; l < N; ++l) {
+            Dr[l] = static_cast<TC>(sD[i + l * N]);
+            Ds[l] = static_cast<TC>(sD[j + l * N]);
+        }
+        TC m_[9];
+        if constexpr (GEO != GEO_NODAL) {
+#pragma unroll
+            for (int c = 0; c < 9; ++c) m_[c] = static_cast<TC>(sg[team].met[c]);
+        }
         // one plane at a time: the register budget goes to the batched loads
 #pragma unroll 1
         for (int kk = 0; kk < KPT; ++kk) {
