@@ -26,27 +26,32 @@ using stage::stage_tile;
 // FP64 runs the field-split tensor-core tile (stage_dmma.cuh, 128 threads) as the
 // single-mesh default does; ALG below is its FP32-bulk shape.
 template <int N> struct BShape;
-template <> struct BShape<2> { static constexpr int KS = 2, EPB = 16, ALG = 0; };
-template <> struct BShape<3> { static constexpr int KS = 1, EPB = 14, ALG = 0; };
+template <> struct BShape<2> { static constexpr int KS = 2, EPB = 16, ALG = 4; };
+template <> struct BShape<3> { static constexpr int KS = 1, EPB = 14, ALG = 4; };
 template <> struct BShape<4> { static constexpr int KS = 2, EPB = 4, ALG = 4; };
 template <> struct BShape<5> { static constexpr int KS = 2, EPB = 2, ALG = 4; };
 template <> struct BShape<6> { static constexpr int KS = 2, EPB = 1, ALG = 4; };
 template <> struct BShape<7> { static constexpr int KS = 2, EPB = 1, ALG = 4; };
 template <> struct BShape<8> { static constexpr int KS = 2, EPB = 1, ALG = 8; };
 template <> struct BShape<9> { static constexpr int KS = 1, EPB = 1, ALG = 4; };
-template <> struct BShape<10> { static constexpr int KS = 1, EPB = 1, ALG = 0; };
+template <> struct BShape<10> { static constexpr int KS = 1, EPB = 1, ALG = 4; };
 
 // N = 8 in FP64: the single-mesh default is the field-split tensor-core tile
 template <int N, bool F32>
 __host__ __device__ constexpr bool dmma_tile() { return N == 8 && !F32; }
 
+// the family of an N in the mixed launch: FP32-bulk keeps the first at 2, 3 and 10 points
+template <int N, bool F32>
+__host__ __device__ constexpr int balg() { return F32 && (N == 2 || N == 3 || N == 10) ? 0 : BShape<N>::ALG; }
+
 template <int N, bool F32>
 constexpr int bsmem() {
     using B = BShape<N>;
+    constexpr int ALG = balg<N, F32>();
     if constexpr (dmma_tile<N, F32>()) return stage::DmmaLayout8::total;
-    else if constexpr (B::ALG == 0) return SmemLayout<N, F32, B::EPB, false>::total;
-    else return stage::Layout2<N, F32, B::EPB, false, (((B::ALG - 2) & 4) != 0),
-                               stage::flux_planes<GEO_BOX, (((B::ALG - 2) & 2) != 0)>()>::total;
+    else if constexpr (ALG == 0) return SmemLayout<N, F32, B::EPB, false>::total;
+    else return stage::Layout2<N, F32, B::EPB, false, (((ALG - 2) & 4) != 0),
+                               stage::flux_planes<GEO_BOX, (((ALG - 2) & 2) != 0)>()>::total;
 }
 
 // One tile of the second family without the persistent loop: stage u_in (and D,
@@ -84,10 +89,10 @@ __device__ __forceinline__ void run_tile(const StageParams& P, int e0, unsigned 
     if constexpr (dmma_tile<N, F32>())
         stage::dmma8_tile<2>(P, e0, smem, tid,
                              reinterpret_cast<const double*>(smem + stage::DmmaLayout8::D));
-    else if constexpr (B::ALG == 0)
+    else if constexpr (balg<N, F32>() == 0)
         stage_tile<N, GEO_BOX, F32, B::KS, B::EPB, false, false>(P, e0, smem, tid);
     else
-        tile2<N, F32, B::KS, B::EPB, B::ALG>(P, e0, smem, tid);
+        tile2<N, F32, B::KS, B::EPB, balg<N, F32>()>(P, e0, smem, tid);
 }
 
 // Carpenter-Kennedy LSRK45 (src/dg_solver.cpp:58-69), for the host and the device.
@@ -212,32 +217,6 @@ DParam d_param(int N, const double* Dh) {
     return dp;
 }
 
-// One block per tile of one N: the single-mesh kernel's tuned shape for that N,
-// fully unrolled, reading its slot from the work item (per-N mode).  ALG 0 is the
-// first-family tile (stage_kernel.cuh); ALG 2 + flags (SPLIT = 2, PAD = 4,
-// CONSTD = 8 with D from dp; no PIPE: the work list is walked one tile per block)
-// the second (stage_pipe.cuh).
-template <int N, bool F32, int KS, int EPB, bool KSMEM, int MINB, int ALG>
-__global__ void __launch_bounds__(EPB * KS * N * N, MINB)
-batch_stage_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
-                     const __grid_constant__ BatchStage bs,
-                     const __grid_constant__ DParam dp) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const WorkItem w = work[blockIdx.x];
-    const SlotDev& S = slots[w.slot];
-    if (!S.active) {
-        stage::grid_wait();
-        return;
-    }
-    const StageParams P = slot_params(S, bs);
-    stage::grid_launch_dependents();
-    stage::grid_wait();
-    if constexpr (ALG == 0)
-        stage_tile<N, GEO_BOX, F32, KS, EPB, KSMEM, true>(P, w.e0, smem, threadIdx.x);
-    else
-        tile2<N, F32, KS, EPB, ALG>(P, w.e0, smem, threadIdx.x, dp.d);
-}
-
 // N = 8 in FP64, per-N mode: the single-mesh default's field-split tensor-core tile
 // (128 threads, one element per block), D from dp (CD) or from shared memory.
 template <int MINB, bool CD>
@@ -267,27 +246,42 @@ cudaError_t launch_dmma8_n(const BatchStage& bs, const SlotDev* slots, const Wor
     return launch_overlapped(kern, ntiles, 128, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
-// Per-N shapes of the per-N mode where neither the bulk-copy form (NBulk, F32Shape) nor the
-// tensor-core tile runs: the single-mesh defaults (stage_variants.h entry 0) at 2, 3 and 10
-// points, and at 4 points in FP64 with the persistent form replaced by its
-// one-tile-per-block form.  An ALG with CONSTD runs without it for an N whose cavities do
-// not all share the pool's D for that N (same arithmetic, D from shared memory).
+// FP32-bulk per-N shapes at 2, 3 and 10 points: the first family's tile, the single-mesh
+// default there.
 template <int N> struct NShape;
-template <> struct NShape<2> { static constexpr int KS = 2, EPB = 16, KSM = 1, MINB = 1, ALG = 0; };
-template <> struct NShape<3> { static constexpr int KS = 1, EPB = 16, KSM = 0, MINB = 4, ALG = 0; };
-template <> struct NShape<4> { static constexpr int KS = 2, EPB = 4, KSM = 0, MINB = 4, ALG = 12; };
-template <> struct NShape<10> { static constexpr int KS = 2, EPB = 1, KSM = 0, MINB = 2, ALG = 0; };
+template <> struct NShape<2> { static constexpr int KS = 2, EPB = 16, KSM = 1, MINB = 1; };
+template <> struct NShape<3> { static constexpr int KS = 1, EPB = 16, KSM = 0, MINB = 4; };
+template <> struct NShape<10> { static constexpr int KS = 2, EPB = 1, KSM = 0, MINB = 2; };
 
-// FP64 per-N shapes that run the bulk-copy one-tile form (the single-mesh default
-// at these N): k staged in shared memory, CD = t-derivative D from the parameters.
-// EARLY = neighbour traces requested while the tile's copies fly.  VROW = the
-// r-derivative's node rows read with 16-byte loads.  AHEAD = 1: each block pulls
-// into L2 the tile of the block half a wave of resident blocks after it (PoolPull).
-template <int N> struct NBulk { static constexpr bool on = false, VROW = false, CD = false, EARLY = false; static constexpr int EPB = 1, MINB = 1, AHEAD = 0; };
-template <> struct NBulk<5> { static constexpr bool on = true, VROW = false, CD = true, EARLY = true; static constexpr int EPB = 1, MINB = 8, AHEAD = 0; };
-template <> struct NBulk<6> { static constexpr bool on = true, VROW = false, CD = true, EARLY = true; static constexpr int EPB = 2, MINB = 3, AHEAD = 1; };
-template <> struct NBulk<7> { static constexpr bool on = true, VROW = false, CD = true, EARLY = true; static constexpr int EPB = 1, MINB = 4, AHEAD = 0; };
-template <> struct NBulk<9> { static constexpr bool on = true, VROW = false, CD = true, EARLY = true; static constexpr int EPB = 1, MINB = 2, AHEAD = 1; };
+template <int N>
+__global__ void __launch_bounds__(NShape<N>::EPB * NShape<N>::KS * N * N, NShape<N>::MINB)
+batch_first_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
+                     const __grid_constant__ BatchStage bs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    using Sh = NShape<N>;
+    const WorkItem w = work[blockIdx.x];
+    const SlotDev& S = slots[w.slot];
+    stage::grid_launch_dependents();
+    stage::grid_wait();
+    if (!S.active) return;
+    const StageParams P = slot_params(S, bs);
+    stage_tile<N, GEO_BOX, true, Sh::KS, Sh::EPB, (Sh::KSM != 0), true>(P, w.e0, smem, threadIdx.x);
+}
+
+// FP64 per-N shapes: the single-mesh default at every N but 8, the bulk-copy one-tile form
+// with the t-derivative's D from the parameters (CD of the kernels below) and neighbour
+// traces requested while the tile's copies fly.  KSM: k staged in shared memory.  AHEAD = 1:
+// each block pulls into L2 the tile of the block half a wave of resident blocks after it
+// (PoolPull).
+template <int N> struct NBulk;
+template <> struct NBulk<2> { static constexpr int EPB = 16, MINB = 4, KSM = 1, AHEAD = 0; };
+template <> struct NBulk<3> { static constexpr int EPB = 8, MINB = 4, KSM = 1, AHEAD = 0; };
+template <> struct NBulk<4> { static constexpr int EPB = 4, MINB = 4, KSM = 0, AHEAD = 0; };
+template <> struct NBulk<5> { static constexpr int EPB = 1, MINB = 8, KSM = 1, AHEAD = 0; };
+template <> struct NBulk<6> { static constexpr int EPB = 2, MINB = 3, KSM = 1, AHEAD = 1; };
+template <> struct NBulk<7> { static constexpr int EPB = 1, MINB = 4, KSM = 1, AHEAD = 0; };
+template <> struct NBulk<9> { static constexpr int EPB = 1, MINB = 2, KSM = 1, AHEAD = 0; };
+template <> struct NBulk<10> { static constexpr int EPB = 1, MINB = 2, KSM = 0, AHEAD = 0; };
 
 // Thread 0's L2 pull in a per-N bulk kernel: the tile of the work item about AHEAD/2
 // waves of resident blocks after this block's (that N's tiles are the grid, one per
@@ -322,17 +316,17 @@ batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restric
     }
     const StageParams P = slot_params(S, bs);
     if constexpr (NBulk<N>::AHEAD > 0)
-        stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, true, NBulk<N>::EARLY, NBulk<N>::VROW>(
+        stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, NBulk<N>::KSM != 0, true>(
             P, w.e0, smem, threadIdx.x, dp.d, PoolPull<N>{slots, work, bs.stage});
     else
-        stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, true, NBulk<N>::EARLY, NBulk<N>::VROW>(
+        stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, NBulk<N>::KSM != 0, true>(
             P, w.e0, smem, threadIdx.x, dp.d);
 }
 
 template <int N, bool CD>
 cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                           const DParam& dp, cudaStream_t st) {
-    constexpr int smem = stage::BulkLayout<N, NBulk<N>::EPB, true>::total;
+    constexpr int smem = stage::BulkLayout<N, NBulk<N>::EPB, NBulk<N>::KSM != 0>::total;
     constexpr int threads = NBulk<N>::EPB * 2 * N * N;
     auto kern = batch_bulk_n_kernel<N, CD>;
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
@@ -372,20 +366,17 @@ cudaError_t launch_f32_n(const BatchStage& bs, const SlotDev* slots, const WorkI
     return launch_overlapped(kern, ntiles, Sh::EPB * 2 * N * N, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
-template <int N, bool F32, int ALG>
-cudaError_t launch_n_alg(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
-                         const DParam& dp, cudaStream_t st) {
+template <int N>
+cudaError_t launch_n_first(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                           cudaStream_t st) {
     using Sh = NShape<N>;
     constexpr int threads = Sh::EPB * Sh::KS * N * N;
-    constexpr int smem = ALG == 0
-        ? SmemLayout<N, F32, Sh::EPB, (Sh::KSM != 0)>::total
-        : stage::Layout2<N, F32, Sh::EPB, false, (((ALG - 2) & 4) != 0),
-                         stage::flux_planes<GEO_BOX, (((ALG - 2) & 2) != 0)>()>::total;
-    auto kern = batch_stage_n_kernel<N, F32, Sh::KS, Sh::EPB, (Sh::KSM != 0), Sh::MINB, ALG>;
+    constexpr int smem = SmemLayout<N, true, Sh::EPB, (Sh::KSM != 0)>::total;
+    auto kern = batch_first_n_kernel<N>;
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs, dp);
+    return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs);
 }
 
 // Dh: this N's D on the host when every resident cavity of this N uses it (the
@@ -401,17 +392,9 @@ cudaError_t launch_n(const BatchStage& bs, const SlotDev* slots, const WorkItem*
             if (e != cudaSuccess) return e;
         }
         return launch_f32_n<N, false>(bs, slots, work, ntiles, dp, st);
-    } else if constexpr (NBulk<N>::on && !F32) {
-        const DParam dp = d_param(N, Dh);
-        if constexpr (NBulk<N>::CD) {
-            if (Dh) return launch_bulk_n<N, true>(bs, slots, work, ntiles, dp, st);
-            if (ntiles <= 0) {  // set-up call: prepare both forms
-                cudaError_t e = launch_bulk_n<N, true>(bs, slots, work, 0, dp, st);
-                if (e != cudaSuccess) return e;
-            }
-        }
-        return launch_bulk_n<N, false>(bs, slots, work, ntiles, dp, st);
-    } else if constexpr (dmma_tile<N, F32>()) {
+    } else if constexpr (F32) {
+        return launch_n_first<N>(bs, slots, work, ntiles, st);
+    } else if constexpr (N == 8) {
         const DParam dp = d_param(N, Dh);
         if (Dh) return launch_dmma8_n<true>(bs, slots, work, ntiles, dp, st);
         if (ntiles <= 0) {  // set-up call: prepare both forms
@@ -420,19 +403,13 @@ cudaError_t launch_n(const BatchStage& bs, const SlotDev* slots, const WorkItem*
         }
         return launch_dmma8_n<false>(bs, slots, work, ntiles, dp, st);
     } else {
-        using Sh = NShape<N>;
-        constexpr bool cd_bit = Sh::ALG >= 2 && ((Sh::ALG - 2) & 8) != 0;
-        constexpr bool has_cd = cd_bit && !F32;  // the constant-bank D is an FP64 form
-        constexpr int ALG_PLAIN = cd_bit ? Sh::ALG - 8 : Sh::ALG;
         const DParam dp = d_param(N, Dh);
-        if constexpr (has_cd) {
-            if (Dh) return launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, ntiles, dp, st);
-            if (ntiles <= 0) {  // set-up call: prepare both forms
-                cudaError_t e = launch_n_alg<N, F32, Sh::ALG>(bs, slots, work, 0, dp, st);
-                if (e != cudaSuccess) return e;
-            }
+        if (Dh) return launch_bulk_n<N, true>(bs, slots, work, ntiles, dp, st);
+        if (ntiles <= 0) {  // set-up call: prepare both forms
+            cudaError_t e = launch_bulk_n<N, true>(bs, slots, work, 0, dp, st);
+            if (e != cudaSuccess) return e;
         }
-        return launch_n_alg<N, F32, ALG_PLAIN>(bs, slots, work, ntiles, dp, st);
+        return launch_bulk_n<N, false>(bs, slots, work, ntiles, dp, st);
     }
 }
 
@@ -591,10 +568,12 @@ cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots
 namespace {
 template <int N>
 int epb_n(int f32) {
-    if constexpr (N == 8) return f32 ? stage::F32Shape<N>::EPB : 1;  // FP64: one element per block
-    else if constexpr (NBulk<N>::on) return f32 ? stage::F32Shape<N>::EPB : NBulk<N>::EPB;
-    else if constexpr (stage::F32Shape<N>::on) return f32 ? stage::F32Shape<N>::EPB : NShape<N>::EPB;
-    else return NShape<N>::EPB;
+    if (f32) {
+        if constexpr (stage::F32Shape<N>::on) return stage::F32Shape<N>::EPB;
+        else return NShape<N>::EPB;
+    }
+    if constexpr (N == 8) return 1;
+    else return NBulk<N>::EPB;
 }
 }  // namespace
 

@@ -49,11 +49,15 @@ constexpr int nth_general(int v) {
     return -1;
 }
 constexpr int kFirstGeneral = nth_general(0);
-// Variant numbers: the axis-aligned class in FP64 has every shape in list order;
+constexpr int kDefault = NWB_DEFAULT(NWB_N);
+static_assert(kDefault < kNumShapes && (NWB_N != 9 || kShapes[kDefault].alg == 1058), "the default's entry");
+// Variant numbers: the axis-aligned class in FP64 has every shape in list order (the
+// default first: it swaps its number with entry 0's);
 // the axis-aligned class in FP32-bulk has the shapes that are not FP64-only, in
 // order; the other classes have one variant, the first such shape.
 inline int shape_index(int geo, int f32, int variant) {
-    return (geo == GEO_BOX && !f32) ? variant : nth_general(variant);
+    if (geo == GEO_BOX && !f32) return variant == 0 ? kDefault : (variant == kDefault ? 0 : variant);
+    return nth_general(variant);
 }
 
 // vid: shape index (shape_index)
