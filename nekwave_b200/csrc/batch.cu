@@ -487,11 +487,25 @@ batch_epilogue_kernel(SlotDev* __restrict__ slots, const int* __restrict__ slot_
         const double* wt = ws + N;
         const long long base = static_cast<long long>(S.probe_elem[pr]) * N3;
         double acc[6] = {0, 0, 0, 0, 0, 0};
-        for (int m = lane; m < N3; m += 32) {
-            const int i = m % N, j = (m / N) % N, k = m / N2;
-            const double wgt = wr[i] * ws[j] * wt[k];
+        // four nodes of a lane in flight (one at a time the loop waited for L2 at each)
+        const double* up = u + base;
+        const long long st = S.stride;
+        for (int m0 = lane; m0 < N3; m0 += 128) {
+            double w[4], v[4][6];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) acc[c] += wgt * u[c * S.stride + base + m];
+            for (int q = 0; q < 4; ++q) {
+                const int m = min(m0 + 32 * q, N3 - 1);
+                const int i = m % N, j = (m / N) % N, k = m / N2;
+                w[q] = wr[i] * ws[j] * wt[k];
+#pragma unroll
+                for (int c = 0; c < 6; ++c) v[q][c] = __ldcg(up + c * st + m);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (m0 + 32 * q < N3) {
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) acc[c] += w[q] * v[q][c];
+                }
         }
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
