@@ -87,7 +87,7 @@ __device__ __forceinline__ void run_tile(const StageParams& P, int e0, unsigned 
     using B = BShape<N>;
     static_assert(B::KS * B::EPB * N * N <= kBatchThreads, "shape too large");
     if constexpr (dmma_tile<N, F32>())
-        stage::dmma8_tile<2>(P, e0, smem, tid,
+        stage::dmma8_tile(P, e0, smem, tid,
                              reinterpret_cast<const double*>(smem + stage::DmmaLayout8::D));
     else if constexpr (balg<N, F32>() == 0)
         stage_tile<N, GEO_BOX, F32, B::KS, B::EPB, false, false>(P, e0, smem, tid);
@@ -231,7 +231,7 @@ batch_dmma8_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
         return;
     }
     const StageParams P = slot_params(S, bs);
-    stage::dmma8_tile<2>(P, w.e0, smem, threadIdx.x,
+    stage::dmma8_tile(P, w.e0, smem, threadIdx.x,
                          CD ? dp.d : reinterpret_cast<const double*>(smem + stage::DmmaLayout8::D));
 }
 

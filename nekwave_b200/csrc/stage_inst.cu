@@ -30,7 +30,7 @@ constexpr Shape kShapes[] = {NWB_VLIST(NWB_X)};
 constexpr int kNumShapes = static_cast<int>(sizeof(kShapes) / sizeof(Shape));
 // FP64 tensor-core shapes and the bulk-copy form: axis-aligned class, FP64 only
 constexpr bool fp64_only(int alg) {
-    return alg == 1 || alg == 200 || alg == 201 || alg == 211 || alg == 212 || alg >= 1000;
+    return alg == 1 || alg == 201 || alg == 211 || alg == 212 || alg >= 1000;
 }
 constexpr int count_simt() {
     int n = 0;
@@ -75,16 +75,16 @@ cudaError_t launch_variant(int vid, const StageParams* p, cudaStream_t st, Stage
                     return launch_mma8<v.minb>(p, st, cfg);
                 else
                     return cudaErrorInvalidValue;
-            } else if constexpr (v.alg == 200 || v.alg == 201) {
+            } else if constexpr (v.alg == 201) {
                 if constexpr (GEO == GEO_BOX && !F32 && NWB_N == 8)
-                    return launch_dmma8<v.minb, v.alg - 199>(p, st, cfg);
+                    return launch_dmma8<v.minb>(p, st, cfg);
                 else
                     return cudaErrorInvalidValue;
             } else if constexpr (v.alg == 211 || v.alg == 212) {
-                // two warps per field, each block pulling a later block's element into
+                // each block pulling a later block's element into
                 // L2 half (211) or one (212) wave of resident blocks ahead
                 if constexpr (GEO == GEO_BOX && !F32 && NWB_N == 8)
-                    return launch_dmma8<v.minb, 2, v.alg - 210>(p, st, cfg);
+                    return launch_dmma8<v.minb, v.alg - 210>(p, st, cfg);
                 else
                     return cudaErrorInvalidValue;
             } else if constexpr (v.alg >= 2 && v.alg <= 129) {
