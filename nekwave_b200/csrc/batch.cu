@@ -12,6 +12,8 @@
 #include "stage_pipe.cuh"
 #include "stage_dmma.cuh"
 #include "stage_bulk.cuh"
+#include "stage_quad.cuh"
+#include "stage_variants.h"
 
 namespace nwb {
 namespace {
@@ -272,16 +274,24 @@ batch_first_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restri
 // with the t-derivative's D from the parameters (CD of the kernels below) and neighbour
 // traces requested while the tile's copies fly.  KSM: k staged in shared memory.  AHEAD = 1:
 // each block pulls into L2 the tile of the block half a wave of resident blocks after it
-// (PoolPull).
+// (PoolPull).  4 points: the four-thread form (NQuad) at every size.
 template <int N> struct NBulk;
 template <> struct NBulk<2> { static constexpr int EPB = 16, MINB = 4, KSM = 1, AHEAD = 0; };
 template <> struct NBulk<3> { static constexpr int EPB = 8, MINB = 4, KSM = 1, AHEAD = 0; };
-template <> struct NBulk<4> { static constexpr int EPB = 4, MINB = 4, KSM = 0, AHEAD = 0; };
 template <> struct NBulk<5> { static constexpr int EPB = 1, MINB = 8, KSM = 1, AHEAD = 0; };
 template <> struct NBulk<6> { static constexpr int EPB = 2, MINB = 3, KSM = 1, AHEAD = 1; };
 template <> struct NBulk<7> { static constexpr int EPB = 1, MINB = 4, KSM = 1, AHEAD = 0; };
 template <> struct NBulk<9> { static constexpr int EPB = 1, MINB = 2, KSM = 1, AHEAD = 0; };
 template <> struct NBulk<10> { static constexpr int EPB = 1, MINB = 2, KSM = 0, AHEAD = 0; };
+
+// The four-threads-per-column form, for launches over few elements (NWB_SMALL): form 1.
+template <int N> struct NQuad { static constexpr int EPB = 1, MINB = 2, KSM = 1; };
+template <> struct NQuad<2> { static constexpr int EPB = 8, MINB = 4, KSM = 1; };
+template <> struct NQuad<3> { static constexpr int EPB = 2, MINB = 8, KSM = 1; };
+template <> struct NQuad<4> { static constexpr int EPB = 2, MINB = 8, KSM = 1; };
+template <> struct NQuad<5> { static constexpr int EPB = 1, MINB = 6, KSM = 1; };
+template <> struct NQuad<9> { static constexpr int EPB = 1, MINB = 1, KSM = 1; };
+template <> struct NQuad<10> { static constexpr int EPB = 1, MINB = 1, KSM = 0; };
 
 // Thread 0's L2 pull in a per-N bulk kernel: the tile of the work item about AHEAD/2
 // waves of resident blocks after this block's (that N's tiles are the grid, one per
@@ -303,8 +313,8 @@ struct PoolPull {
     }
 };
 
-template <int N, bool CD>
-__global__ void __launch_bounds__(NBulk<N>::EPB * 2 * N * N, NBulk<N>::MINB)
+template <int N, int EPB, int MINB, bool KSM, bool PULL, bool CD>
+__global__ void __launch_bounds__(EPB * 2 * N * N, MINB)
 batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
                     const __grid_constant__ BatchStage bs, const __grid_constant__ DParam dp) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -315,24 +325,71 @@ batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restric
         return;
     }
     const StageParams P = slot_params(S, bs);
-    if constexpr (NBulk<N>::AHEAD > 0)
-        stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, NBulk<N>::KSM != 0, true>(
-            P, w.e0, smem, threadIdx.x, dp.d, PoolPull<N>{slots, work, bs.stage});
+    if constexpr (PULL)
+        stage::bulk_tile<N, GEO_BOX, 2, EPB, CD, false, KSM, true>(P, w.e0, smem, threadIdx.x, dp.d,
+                                                                   PoolPull<N>{slots, work, bs.stage});
     else
-        stage::bulk_tile<N, GEO_BOX, 2, NBulk<N>::EPB, CD, false, NBulk<N>::KSM != 0, true>(
-            P, w.e0, smem, threadIdx.x, dp.d);
+        stage::bulk_tile<N, GEO_BOX, 2, EPB, CD, false, KSM, true>(P, w.e0, smem, threadIdx.x, dp.d);
 }
 
-template <int N, bool CD>
-cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
-                          const DParam& dp, cudaStream_t st) {
-    constexpr int smem = stage::BulkLayout<N, NBulk<N>::EPB, NBulk<N>::KSM != 0>::total;
-    constexpr int threads = NBulk<N>::EPB * 2 * N * N;
-    auto kern = batch_bulk_n_kernel<N, CD>;
-    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
+template <int N, int EPB, int MINB, bool KSM, bool CD>
+__global__ void __launch_bounds__(stage::Quad<N, EPB>::threads, MINB)
+batch_quad_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
+                    const __grid_constant__ BatchStage bs, const __grid_constant__ DParam dp) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const WorkItem w = work[blockIdx.x];
+    const SlotDev& S = slots[w.slot];
+    if (!S.active) {
+        stage::grid_wait();
+        return;
+    }
+    const StageParams P = slot_params(S, bs);
+    stage::quad_tile<N, EPB, KSM, CD>(P, w.e0, smem, threadIdx.x, dp.d);
+}
+
+template <int N, int EPB, bool KSM, class K>
+cudaError_t launch_tiles(K kern, int threads, std::atomic<int>* attr_set, const BatchStage& bs, const SlotDev* slots,
+                         const WorkItem* work, int ntiles, const DParam& dp, cudaStream_t st) {
+    constexpr int smem = stage::BulkLayout<N, EPB, KSM>::total;
     if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
     return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs, dp);
+}
+
+template <int N, int EPB, int MINB, bool KSM, bool PULL, bool CD>
+cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                          const DParam& dp, cudaStream_t st) {
+    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
+    return launch_tiles<N, EPB, KSM>(batch_bulk_n_kernel<N, EPB, MINB, KSM, PULL, CD>, EPB * 2 * N * N, attr_set, bs,
+                                     slots, work, ntiles, dp, st);
+}
+
+template <int N, bool CD>
+cudaError_t launch_quad_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                          const DParam& dp, cudaStream_t st) {
+    using Q = NQuad<N>;
+    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
+    return launch_tiles<N, Q::EPB, Q::KSM != 0>(batch_quad_n_kernel<N, Q::EPB, Q::MINB, Q::KSM != 0, CD>,
+                                                stage::Quad<N, Q::EPB>::threads, attr_set, bs, slots, work, ntiles,
+                                                dp, st);
+}
+
+// The form of a per-N launch (batch_form_n): 0 large, 1 four threads per column, 2 (6 points)
+// one element per block.
+template <int N, bool CD>
+cudaError_t launch_form_n(int form, const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                          const DParam& dp, cudaStream_t st) {
+    if constexpr (N == 4) return launch_quad_n<N, CD>(bs, slots, work, ntiles, dp, st);
+    else {
+        if (form == 1) return launch_quad_n<N, CD>(bs, slots, work, ntiles, dp, st);
+        if constexpr (N == 6)
+            if (form == 2) return launch_bulk_n<N, 1, 5, true, false, CD>(bs, slots, work, ntiles, dp, st);
+        if constexpr (N == 8) return launch_dmma8_n<CD>(bs, slots, work, ntiles, dp, st);
+        else {
+            using B = NBulk<N>;
+            return launch_bulk_n<N, B::EPB, B::MINB, B::KSM != 0, (B::AHEAD > 0), CD>(bs, slots, work, ntiles, dp, st);
+        }
+    }
 }
 
 // FP32-bulk, per-N mode: the single-mesh form (stage::F32Shape), D from dp (CD) or from
@@ -382,7 +439,7 @@ cudaError_t launch_n_first(const BatchStage& bs, const SlotDev* slots, const Wor
 // Dh: this N's D on the host when every resident cavity of this N uses it (the
 // constant-bank form then applies), else null.
 template <int N, bool F32>
-cudaError_t launch_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+cudaError_t launch_n(int form, const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                      const double* Dh, cudaStream_t st) {
     if constexpr (stage::F32Shape<N>::on && F32) {
         const DParam dp = d_param(N, Dh);
@@ -394,22 +451,18 @@ cudaError_t launch_n(const BatchStage& bs, const SlotDev* slots, const WorkItem*
         return launch_f32_n<N, false>(bs, slots, work, ntiles, dp, st);
     } else if constexpr (F32) {
         return launch_n_first<N>(bs, slots, work, ntiles, st);
-    } else if constexpr (N == 8) {
-        const DParam dp = d_param(N, Dh);
-        if (Dh) return launch_dmma8_n<true>(bs, slots, work, ntiles, dp, st);
-        if (ntiles <= 0) {  // set-up call: prepare both forms
-            cudaError_t e = launch_dmma8_n<true>(bs, slots, work, 0, dp, st);
-            if (e != cudaSuccess) return e;
-        }
-        return launch_dmma8_n<false>(bs, slots, work, ntiles, dp, st);
     } else {
         const DParam dp = d_param(N, Dh);
-        if (Dh) return launch_bulk_n<N, true>(bs, slots, work, ntiles, dp, st);
-        if (ntiles <= 0) {  // set-up call: prepare both forms
-            cudaError_t e = launch_bulk_n<N, true>(bs, slots, work, 0, dp, st);
-            if (e != cudaSuccess) return e;
+        if (ntiles <= 0) {  // set-up call: prepare every form
+            for (int f = 0; f < kBatchForms; ++f) {
+                cudaError_t e = launch_form_n<N, true>(f, bs, slots, work, 0, dp, st);
+                if (e == cudaSuccess) e = launch_form_n<N, false>(f, bs, slots, work, 0, dp, st);
+                if (e != cudaSuccess) return e;
+            }
+            return cudaSuccess;
         }
-        return launch_bulk_n<N, false>(bs, slots, work, ntiles, dp, st);
+        return Dh ? launch_form_n<N, true>(form, bs, slots, work, ntiles, dp, st)
+                  : launch_form_n<N, false>(form, bs, slots, work, ntiles, dp, st);
     }
 }
 
@@ -564,14 +617,14 @@ int max_batch_smem() {
 
 }  // namespace
 
-cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots,
+cudaError_t launch_batch_stage_n(int N, int f32, int form, int stage, const SlotDev* slots,
                                  const WorkItem* work, int ntiles, int dry, const double* Dh,
                                  cudaStream_t st) {
     const BatchStage bs{dry ? 0.0 : kRk4a[stage], dry ? 0.0 : kRk4b[stage], stage, dry};
     switch (N) {
 #define NWB_CASE(n) \
-        case n: return f32 ? launch_n<n, true>(bs, slots, work, ntiles, Dh, st) \
-                           : launch_n<n, false>(bs, slots, work, ntiles, Dh, st);
+        case n: return f32 ? launch_n<n, true>(form, bs, slots, work, ntiles, Dh, st) \
+                           : launch_n<n, false>(form, bs, slots, work, ntiles, Dh, st);
         NWB_CASE(2) NWB_CASE(3) NWB_CASE(4) NWB_CASE(5) NWB_CASE(6) NWB_CASE(7) NWB_CASE(8)
         NWB_CASE(9) NWB_CASE(10)
 #undef NWB_CASE
@@ -581,21 +634,40 @@ cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots
 
 namespace {
 template <int N>
-int epb_n(int f32) {
+int epb_n(int f32, int form) {
     if (f32) {
         if constexpr (stage::F32Shape<N>::on) return stage::F32Shape<N>::EPB;
         else return NShape<N>::EPB;
     }
-    if constexpr (N == 8) return 1;
-    else return NBulk<N>::EPB;
+    if constexpr (N == 4) return NQuad<N>::EPB;
+    else {
+        if (form == 1) return NQuad<N>::EPB;
+        if (form == 2 || N == 8) return 1;
+        if constexpr (N != 8) return NBulk<N>::EPB;
+        else return 1;
+    }
 }
 }  // namespace
 
-int batch_epb_n(int N, int f32) {
+int batch_form_n(int N, int f32, long long nelt) {
+    if (f32) return 0;
+#define NWB_X(n, i) if (nelt <= (n)) return form; ++form;
+    int form = 1;
     switch (N) {
-        case 2: return epb_n<2>(f32); case 3: return epb_n<3>(f32); case 4: return epb_n<4>(f32);
-        case 5: return epb_n<5>(f32); case 6: return epb_n<6>(f32); case 7: return epb_n<7>(f32);
-        case 8: return epb_n<8>(f32); case 9: return epb_n<9>(f32); case 10: return epb_n<10>(f32);
+#define NWB_CASE(k) case k: { NWB_SMALL_##k(NWB_X) break; }
+        NWB_CASE(2) NWB_CASE(3) NWB_CASE(4) NWB_CASE(5) NWB_CASE(6) NWB_CASE(7) NWB_CASE(8) NWB_CASE(9) NWB_CASE(10)
+#undef NWB_CASE
+        default: break;
+    }
+#undef NWB_X
+    return 0;
+}
+
+int batch_epb_n(int N, int f32, int form) {
+    switch (N) {
+        case 2: return epb_n<2>(f32, form); case 3: return epb_n<3>(f32, form); case 4: return epb_n<4>(f32, form);
+        case 5: return epb_n<5>(f32, form); case 6: return epb_n<6>(f32, form); case 7: return epb_n<7>(f32, form);
+        case 8: return epb_n<8>(f32, form); case 9: return epb_n<9>(f32, form); case 10: return epb_n<10>(f32, form);
         default: return 1;
     }
 }

@@ -57,10 +57,15 @@ cudaError_t launch_batch_stage(int f32, int stage, const SlotDev* slots, const W
 // which must have been cut with batch_epb_n(N, f32) elements each).  Dh: that N's D on
 // the host when every resident cavity of that N shares it (lets the kernel take D
 // from its parameters), else null.
-cudaError_t launch_batch_stage_n(int N, int f32, int stage, const SlotDev* slots,
+// form: batch_form_n of that N's resident elements, also when the tiles were cut.
+cudaError_t launch_batch_stage_n(int N, int f32, int form, int stage, const SlotDev* slots,
                                  const WorkItem* work, int ntiles, int dry, const double* Dh,
                                  cudaStream_t st);
-int batch_epb_n(int N, int f32);
+// Kernel form of a per-N launch over nelt elements in all (0: the large one), as the
+// single solver's default follows its mesh's size; elements per block of a form.
+constexpr int kBatchForms = 3;
+int batch_form_n(int N, int f32, long long nelt);
+int batch_epb_n(int N, int f32, int form);
 // Diagnostics after a step (post = 1) or of the initial state (post = 0): energy
 // partials per tile of the work items [work, work + ntiles) (ntiles_p, when given: their
 // number on the device).  overlap: see launch_overlapped.

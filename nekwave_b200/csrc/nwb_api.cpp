@@ -338,6 +338,7 @@ struct nwb_solver {
     size_t flush_bytes = 0;
     nwb::StageConfig cfg{};
     int variant = 0;
+    int dflt = 0;  // what variant 0 stands for on this mesh (nwb::stage_default_variant)
     long long launches = 0;
     size_t device_bytes = 0;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
@@ -345,6 +346,8 @@ struct nwb_solver {
     double gdt = 0.0;
     bool is_box = false;
     nwb::BoxPulse box{};
+
+    int shape(int v) const { return v == 0 ? dflt : v; }
 
     nwb::StageParams params(int stage, double dt) const {
         nwb::StageParams P{};
@@ -379,7 +382,7 @@ struct nwb_solver {
 
     nwb_status launch_stage(int stage, double dt) {
         nwb::StageParams P = params(stage, dt);
-        cudaError_t e = nwb::launch_stage(N, geo, f32, variant, &P, st, nullptr);
+        cudaError_t e = nwb::launch_stage(N, geo, f32, shape(variant), &P, st, nullptr);
         if (e != cudaSuccess) return fail(NWB_ECUDA, "stage kernel launch: %s", cudaGetErrorString(e));
         cur ^= 1;
         ++launches;
@@ -663,7 +666,8 @@ nwb_status create_solver(const nwb_mesh_desc* m, int N, int nelt, const double* 
     ce = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
     if (ce != cudaSuccess) return bail(fail(NWB_ECUDA, "cudaStreamCreate: %s", cudaGetErrorString(ce)));
 
-    ce = nwb::launch_stage(N, s->geo, s->f32, s->variant, nullptr, nullptr, &s->cfg);
+    s->dflt = nwb::stage_default_variant(N, s->geo, s->f32, nelt);
+    ce = nwb::launch_stage(N, s->geo, s->f32, s->shape(s->variant), nullptr, nullptr, &s->cfg);
     if (ce != cudaSuccess)
         return bail(fail(NWB_ECUDA, "stage kernel set-up: %s", cudaGetErrorString(ce)));
 
@@ -879,7 +883,7 @@ nwb_status nwb_eval_rhs(nwb_solver* s, double* h, size_t n) {
     P.a = 0.0;
     P.b = 0.0;
     P.kio = nwb::kKWrite;
-    cudaError_t e = nwb::launch_stage(s->N, s->geo, s->f32, s->variant, &P, s->st, nullptr);
+    cudaError_t e = nwb::launch_stage(s->N, s->geo, s->f32, s->shape(s->variant), &P, s->st, nullptr);
     if (e != cudaSuccess) return fail(NWB_ECUDA, "stage kernel launch: %s", cudaGetErrorString(e));
     ++s->launches;
     NWB_CU(cudaMemcpy2DAsync(h, sizeof(double) * s->npts, s->k, sizeof(double) * s->stride,
@@ -1077,7 +1081,7 @@ nwb_status nwb_solver_set_variant(nwb_solver* s, int variant) {
     if (variant < 0 || variant >= nwb::stage_variant_count(s->N, s->geo, s->f32))
         return fail(NWB_EINVAL, "nwb_solver_set_variant: variant %d out of range", variant);
     nwb::StageConfig c{};
-    cudaError_t e = nwb::launch_stage(s->N, s->geo, s->f32, variant, nullptr, nullptr, &c);
+    cudaError_t e = nwb::launch_stage(s->N, s->geo, s->f32, s->shape(variant), nullptr, nullptr, &c);
     if (e != cudaSuccess)
         return fail(NWB_ECUDA, "variant %d set-up: %s", variant, cudaGetErrorString(e));
     NWB_CU(cudaStreamSynchronize(s->st));
@@ -1101,7 +1105,7 @@ nwb_status nwb_solver_autotune(nwb_solver* s, int reps, int* best, float* ms_out
     float bestt = 1e30f, t0 = 1e30f;
     for (int v = 0; v < nv; ++v) {
         nwb::StageConfig c{};
-        cudaError_t e = nwb::launch_stage(s->N, s->geo, s->f32, v, nullptr, nullptr, &c);
+        cudaError_t e = nwb::launch_stage(s->N, s->geo, s->f32, s->shape(v), nullptr, nullptr, &c);
         if (e != cudaSuccess) return fail(NWB_ECUDA, "variant %d set-up: %s", v, cudaGetErrorString(e));
         nwb::StageParams P = s->params(0, 0.0);
         P.a = 0.0;
@@ -1109,12 +1113,12 @@ nwb_status nwb_solver_autotune(nwb_solver* s, int reps, int* best, float* ms_out
         P.kio = nwb::kKRead | nwb::kKWrite;  // timed as the inner stages are
         P.u_out = s->u[s->cur ^ 1];
         for (int w = 0; w < 2; ++w) {
-            e = nwb::launch_stage(s->N, s->geo, s->f32, v, &P, s->st, nullptr);
+            e = nwb::launch_stage(s->N, s->geo, s->f32, s->shape(v), &P, s->st, nullptr);
             if (e != cudaSuccess) return fail(NWB_ECUDA, "autotune launch: %s", cudaGetErrorString(e));
         }
         NWB_CU(cudaEventRecord(a, s->st));
         for (int r = 0; r < reps; ++r) {
-            e = nwb::launch_stage(s->N, s->geo, s->f32, v, &P, s->st, nullptr);
+            e = nwb::launch_stage(s->N, s->geo, s->f32, s->shape(v), &P, s->st, nullptr);
             if (e != cudaSuccess) return fail(NWB_ECUDA, "autotune launch: %s", cudaGetErrorString(e));
         }
         NWB_CU(cudaEventRecord(b, s->st));

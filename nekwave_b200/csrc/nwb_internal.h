@@ -201,6 +201,10 @@ nwb_status set_error(nwb_status s, const char* fmt, ...);
 cudaError_t launch_stage(int N, int geo, int f32, int variant, const StageParams* p,
                          cudaStream_t st, StageConfig* cfg_out);
 int stage_variant_count(int N, int geo, int f32);
+// The variant that stands for variant 0 on a mesh of nelt elements (stage_variants.h).
+int stage_default_variant(int N, int geo, int f32, int nelt);
+template <int N>
+int stage_default_variant_n(int geo, int f32, int nelt);
 template <int N>
 cudaError_t launch_stage_n(int geo, int f32, int variant, const StageParams* p, cudaStream_t st,
                            StageConfig* cfg);

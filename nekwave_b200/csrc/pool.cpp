@@ -193,6 +193,7 @@ struct nwb_pool {
     nwb::WorkItem* d_work_n = nullptr;
     int work_n_cap = 0;
     int n_off[11] = {}, n_cnt[11] = {};
+    int n_form[11] = {};  // kernel form of that N's launches (nwb::batch_form_n)
     // that N's range of the work list (energy tiles) and its slots (d_slot_list)
     int w_off[11] = {}, w_cnt[11] = {}, s_off[11] = {}, s_cnt[11] = {};
     int* d_slot_list = nullptr;
@@ -287,7 +288,11 @@ struct nwb_pool {
         std::vector<nwb::WorkItem> wn;
         for (int N = 2; N <= 10; ++N) {
             n_off[N] = static_cast<int>(wn.size());
-            const int epb = nwb::batch_epb_n(N, f32);
+            long long total = 0;
+            for (const SlotHost& h : slots)
+                if (h.used && h.N == N) total += h.nelt;
+            n_form[N] = nwb::batch_form_n(N, f32, total);
+            const int epb = nwb::batch_epb_n(N, f32, n_form[N]);
             for (int s = 0; s < max_slots; ++s) {
                 const SlotHost& h = slots[s];
                 if (!h.used || h.N != N) continue;
@@ -342,7 +347,7 @@ struct nwb_pool {
             cudaError_t e = cudaSuccess;
             for (int n = 0; n < nsteps && e == cudaSuccess; ++n) {
                 for (int s = 0; s < 5 && e == cudaSuccess; ++s)
-                    e = nwb::launch_batch_stage_n(N, f32, s, d_slots, d_work_n + n_off[N], n_cnt[N], dry,
+                    e = nwb::launch_batch_stage_n(N, f32, n_form[N], s, d_slots, d_work_n + n_off[N], n_cnt[N], dry,
                                                   all_canon ? canonD[N] : nullptr, c);
                 if (dry) continue;
                 if (e == cudaSuccess && diag)
@@ -390,7 +395,7 @@ struct nwb_pool {
         grid = sms * std::min(3, by_smem);  // the kernel is built for 3 resident blocks
         diag_grid = sms * 4;
         for (int N = 2; N <= 10; ++N) {  // one-time kernel attribute set-up, outside capture
-            cudaError_t e = nwb::launch_batch_stage_n(N, f32, 0, nullptr, nullptr, 0, 0, nullptr, st);
+            cudaError_t e = nwb::launch_batch_stage_n(N, f32, 0, 0, nullptr, nullptr, 0, 0, nullptr, st);
             if (e != cudaSuccess) return set_error(NWB_ECUDA, "per-N set-up: %s", cudaGetErrorString(e));
         }
         return NWB_OK;
@@ -518,10 +523,13 @@ nwb_status nwb_pool_create(size_t hbm_budget_bytes, int max_slots, nwb_precision
     if (e == cudaSuccess) {
         double min_tile = 1e300;
         for (int N = 2; N <= 10; ++N) {
-            const int epb = std::min(nwb::batch_shape(N, p->f32).epb, nwb::batch_epb_n(N, p->f32));
+            const int epb = std::min(nwb::batch_shape(N, p->f32).epb, nwb::batch_epb_n(N, p->f32, 0));
             min_tile = std::min(min_tile, 144.0 * N * N * N * epb);
         }
-        const double cap = static_cast<double>(max_slots) + static_cast<double>(hbm_budget_bytes) / min_tile + 1;
+        // the forms for few elements cut smaller tiles, of at most kSmallTiles elements in all
+        constexpr int kSmallTiles = 9 * 40 * 148;
+        const double cap = static_cast<double>(max_slots) + static_cast<double>(hbm_budget_bytes) / min_tile + 1 +
+                           kSmallTiles;
         if (cap > 0x7fffffff) e = cudaErrorInvalidValue;
         p->work_cap = p->work_n_cap = static_cast<int>(cap);
     }

@@ -19,6 +19,21 @@ cudaError_t launch_stage(int N, int geo, int f32, int variant, const StageParams
     }
 }
 
+int stage_default_variant(int N, int geo, int f32, int nelt) {
+    switch (N) {
+        case 2: return stage_default_variant_n<2>(geo, f32, nelt);
+        case 3: return stage_default_variant_n<3>(geo, f32, nelt);
+        case 4: return stage_default_variant_n<4>(geo, f32, nelt);
+        case 5: return stage_default_variant_n<5>(geo, f32, nelt);
+        case 6: return stage_default_variant_n<6>(geo, f32, nelt);
+        case 7: return stage_default_variant_n<7>(geo, f32, nelt);
+        case 8: return stage_default_variant_n<8>(geo, f32, nelt);
+        case 9: return stage_default_variant_n<9>(geo, f32, nelt);
+        case 10: return stage_default_variant_n<10>(geo, f32, nelt);
+        default: return 0;
+    }
+}
+
 int stage_variant_count(int N, int geo, int f32) {
     switch (N) {
         case 2: return stage_variant_count_n<2>(geo, f32);

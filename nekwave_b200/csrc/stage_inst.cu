@@ -5,6 +5,7 @@
 #include "stage_pipe.cuh"
 #include "stage_dmma.cuh"
 #include "stage_bulk.cuh"
+#include "stage_quad.cuh"
 #include "stage_variants.h"
 
 #ifndef NWB_N
@@ -98,6 +99,12 @@ cudaError_t launch_variant(int vid, const StageParams* p, cudaStream_t st, Stage
                                    (fl & 64) != 0>(p, st, cfg);
                 else
                     return cudaErrorInvalidValue;
+            } else if constexpr (v.alg >= 2024) {
+                // four threads per column (stage_quad.cuh); + 32: k staged in shared memory
+                if constexpr (GEO == GEO_BOX && !F32)
+                    return launch_quad<NWB_N, v.epb, v.minb, v.alg == 2056>(p, st, cfg);
+                else
+                    return cudaErrorInvalidValue;
             } else if constexpr (v.alg >= 1000) {
                 // the bulk-copy one-tile form (stage_bulk.cuh), second-family flags
                 // ALG - 1000: 2 SPLIT (required), 8 CONSTD, 16 EARLY, 32 KSM, 64 DSMEM,
@@ -124,6 +131,13 @@ cudaError_t launch_variant(int vid, const StageParams* p, cudaStream_t st, Stage
         return cudaErrorInvalidValue;
     }
 }
+
+struct Small {
+    int nelt, entry;
+};
+#define NWB_X(n, i) Small{n, i},
+constexpr Small kSmall[] = {NWB_CAT(NWB_SMALL_, NWB_N)(NWB_X) Small{0, kDefault}};
+#undef NWB_X
 
 template <int GEO>
 int count_variants(int f32) {
@@ -153,6 +167,14 @@ cudaError_t launch_stage_n<NWB_N>(int geo, int f32, int variant, const StagePara
         default:
             return cudaErrorInvalidValue;
     }
+}
+
+template <>
+int stage_default_variant_n<NWB_N>(int geo, int f32, int nelt) {
+    if (geo != GEO_BOX || f32) return 0;
+    for (const stage::Small& s : stage::kSmall)
+        if (nelt <= s.nelt) return s.entry;  // variant numbers are list indices but for 0
+    return 0;
 }
 
 template <>

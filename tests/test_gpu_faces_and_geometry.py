@@ -10,6 +10,9 @@ import pytest
 from oracle import oracle as O
 from tests.gpu_helpers import random_state, rel_l2, rel_max, solver_for
 
+from nekwave_b200 import DgSolver
+from nekwave_b200.pool import CavityPool
+
 pytestmark = pytest.mark.gpu
 
 
@@ -97,3 +100,38 @@ def test_the_register_of_an_earlier_run_does_not_enter_a_step(gpu, N, warp):
     s.steps(dt, 2)
     assert rel_l2(s.downloadState(), O.step(m, 1.0, dt, 2, u)[0]) < 1e-12
     s.finalize()
+
+
+# elements up to which an order takes the shapes for few elements, and a size beyond it
+LARGE = {2: (13, 12, 12), 3: (13, 13, 13), 4: (5, 4, 3), 5: (19, 18, 18), 6: (15, 14, 15), 7: (7, 7, 7),
+         8: (5, 4, 3), 9: (6, 5, 5), 10: (11, 11, 10)}
+
+
+@pytest.mark.parametrize("N", range(2, 11))
+def test_few_and_many_elements_give_a_cavity_the_same_bits(gpu, N):
+    """The launch shape follows the number of elements of an order (single solver: of its
+    mesh; pool: of all its cavities).  A small cavity alone, in a pool of its own (shapes
+    for few elements) and beside a large one (the other shape) ends in the same bits."""
+    small, dt = (3, 2, 2), 1e-3
+    pulses = [(0.5 + 0.1 * c, 0.3, 0.4, 0.5, 0.2) for c in range(6)]
+    s = DgSolver("fp64")
+    s.initializeBox(N, small, (0, 0, 0), (1, 1, 1), 1.0)
+    s.initPulse(pulses)
+    s.steps(dt, 3)
+    want = s.downloadState()
+    s.finalize()
+    for nels in ([small], [small, LARGE[N]], [LARGE[N], small]):
+        pool = CavityPool(1 << 30, max_slots=4)
+        slots = [pool.add_box(N, nel, (0, 0, 0), (1, 1, 1), 1.0, dt, 3) for nel in nels]
+        for q in slots:
+            pool.init_pulse(q, pulses)
+        pool.step(3)
+        np.testing.assert_array_equal(pool.results(slots[nels.index(small)])["state"], want)
+        if LARGE[N] in nels:
+            s = DgSolver("fp64")
+            s.initializeBox(N, LARGE[N], (0, 0, 0), (1, 1, 1), 1.0)
+            s.initPulse(pulses)
+            s.steps(dt, 3)
+            np.testing.assert_array_equal(pool.results(slots[nels.index(LARGE[N])])["state"], s.downloadState())
+            s.finalize()
+        pool.close()
