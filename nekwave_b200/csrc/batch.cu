@@ -34,7 +34,7 @@ template <> struct BShape<4> { static constexpr int KS = 2, EPB = 4, ALG = 4; };
 template <> struct BShape<5> { static constexpr int KS = 2, EPB = 2, ALG = 4; };
 template <> struct BShape<6> { static constexpr int KS = 2, EPB = 1, ALG = 4; };
 template <> struct BShape<7> { static constexpr int KS = 2, EPB = 1, ALG = 4; };
-template <> struct BShape<8> { static constexpr int KS = 2, EPB = 1, ALG = 8; };
+template <> struct BShape<8> { static constexpr int KS = 2, EPB = 1, ALG = 4; };
 template <> struct BShape<9> { static constexpr int KS = 1, EPB = 1, ALG = 4; };
 template <> struct BShape<10> { static constexpr int KS = 1, EPB = 1, ALG = 4; };
 

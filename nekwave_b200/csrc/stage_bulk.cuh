@@ -322,16 +322,17 @@ cudaError_t launch_general(const StageParams* p, cudaStream_t st, StageConfig* c
 // phase's FP64 loop serves the elements that fall back, most of them in the benchmark's
 // fields, so it takes its D rows in registers and (CD) the unrolled loop of the FP64 class
 // (with its D rows read from shared memory at each use it did more than twice the shared
-// loads of the FP64 class).  k in shared memory (KSM) only at 5 points: elsewhere it costs
-// a resident block.  From a sweep of four shapes per N.  B200, per step, before -> now:
-// 25^3 elements of 8 points 1917 -> 1623 us, 34^3 of 6 points 2452 -> 2019 us, 22^3 of 9 points
-// 2631 -> 1750 us, 40^3 of 5 points 2569 -> 2122 us.
+// loads of the FP64 class); at 8 points it is the tensor-core column phase of the FP64
+// class.  k in shared memory (KSM) only at 5 points: elsewhere it costs a resident block.
+// From a sweep of four shapes per N.  B200, per step, before -> now: 25^3 elements of 8 points
+// 1917 -> 1406 us, 34^3 of 6 points 2452 -> 2019 us, 22^3 of 9 points 2631 -> 1750 us, 40^3 of 5
+// points 2569 -> 2122 us.
 template <int N> struct F32Shape { static constexpr bool on = false; static constexpr int EPB = 1, MINB = 1, KSM = 0, CD = 0; };
 template <> struct F32Shape<4> { static constexpr bool on = true; static constexpr int EPB = 2, MINB = 8, KSM = 0, CD = 1; };
 template <> struct F32Shape<5> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 8, KSM = 1, CD = 1; };
 template <> struct F32Shape<6> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 5, KSM = 0, CD = 1; };
 template <> struct F32Shape<7> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 4, KSM = 0, CD = 1; };
-template <> struct F32Shape<8> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 4, KSM = 0, CD = 0; };
+template <> struct F32Shape<8> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 4, KSM = 0, CD = 1; };
 template <> struct F32Shape<9> { static constexpr bool on = true; static constexpr int EPB = 1, MINB = 2, KSM = 0, CD = 1; };
 
 template <int N>

@@ -42,6 +42,7 @@
 // face points before it forms any flux, and each node's k is read before the
 // derivative sums that hide its latency.
 #pragma once
+#include "stage_dmma_columns.cuh"
 #include "stage_kernel.cuh"
 
 #include <cstdint>
@@ -1046,6 +1047,26 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     const long long ebase = static_cast<long long>(e) * N3;
 
     if constexpr (SPLIT) {
+        // the lifted fluxes of the faces across t at this column, components x and y of field
+        // hf's residual (box_flux with d = z, a = x, b = y); tr: the differentiated field's
+        // traces where they are in registers already
+        auto z_fluxes = [&](int hf, const double (*tr)[2], double (&zf)[2][2]) {
+            if constexpr (BOXF) {
+                const int src = hf == 0 ? 3 : 0, dst = 3 - src;
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const double* own = Uf + i + RP * j + (s ? PP * (N - 1) : 0);
+                    const double sx = tr ? tr[s][0] : own[src * CS], sy = tr ? tr[s][1] : own[(src + 1) * CS];
+                    const double dx = own[dst * CS], dy = own[(dst + 1) * CS];
+                    double jmp[4], F[4];
+                    box_jumps(G.zv[s], G.zn[s], hf == 0 ? dx : sx, hf == 0 ? dy : sy, hf == 0 ? sx : dx,
+                              hf == 0 ? sy : dy, jmp);
+                    box_flux<TC>(sg[team].nrm[4 + s][2], P.c0, sg[team].lift[4 + s], jmp, F);
+                    zf[s][0] = hf == 0 ? F[0] : F[2];
+                    zf[s][1] = hf == 0 ? F[1] : F[3];
+                }
+            }
+        };
         // the column work in arithmetic type TX (TC, or FP64 for a fallback element)
         auto columns = [&](auto zero) {
         using TX = decltype(zero);
@@ -1088,29 +1109,12 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         for (int c = 0; c < NC; ++c)
 #pragma unroll
             for (int l = 0; l < N; ++l) col[c][l] = V[c * CS + i + RP * j + PP * l];
-        // the lifted fluxes of the faces across t at this column, components x and y of
-        // this residual (box_flux with d = z, a = x, b = y)
         double zf[2][2];
         if constexpr (BOXF) {
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const int m = i + RP * j + (s ? PP * (N - 1) : 0);
-                const double* own = Uf + m;
-                double sx, sy;  // the differentiated field's trace: in registers when FP64
-                if constexpr (F32) {
-                    sx = own[src * CS];
-                    sy = own[(src + 1) * CS];
-                } else {
-                    sx = static_cast<double>(col[0][s ? N - 1 : 0]);
-                    sy = static_cast<double>(col[1][s ? N - 1 : 0]);
-                }
-                const double dx = own[dst * CS], dy = own[(dst + 1) * CS];
-                double jmp[4], F[4];
-                box_jumps(G.zv[s], G.zn[s], hf == 0 ? dx : sx, hf == 0 ? dy : sy, hf == 0 ? sx : dx,
-                          hf == 0 ? sy : dy, jmp);
-                box_flux<TC>(sg[team].nrm[4 + s][2], P.c0, sg[team].lift[4 + s], jmp, F);
-                zf[s][0] = hf == 0 ? F[0] : F[2];
-                zf[s][1] = hf == 0 ? F[1] : F[3];
+            if constexpr (F32) z_fluxes(hf, nullptr, zf);
+            else {
+                const double tr[2][2] = {{col[0][0], col[1][0]}, {col[0][N - 1], col[1][N - 1]}};
+                z_fluxes(hf, tr, zf);
             }
         }
         // CONSTD (plane loop unrolled): k of the next plane is requested before this
@@ -1254,7 +1258,40 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
         }
         };
         if constexpr (F32 && GEO != GEO_NODAL) {
-            if (fb64) columns(0.0);
+            // 8 points: a fallback element's FP64 sums on the tensor cores, as in the FP64
+            // class; the four warps take other nodes than the node columns above, so the
+            // lifted fluxes of the faces across t go through shared memory (where the
+            // FP32 copy would be)
+            constexpr bool DMMA = N == 8 && GEO == GEO_BOX && KS == 2 && EPB == 1 && !PAD && CS % 2 == 0;
+            if constexpr (DMMA) {
+                if (fb64) {
+                    double* sz = reinterpret_cast<double*>(smem_uc);  // [2 faces][4][64]
+                    double zf[2][2];
+                    z_fluxes(h, nullptr, zf);
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) sz[(4 * s + 2 * h + c) * N2 + loc] = zf[s][c];
+                    bar.sync();  // every thread of the block is here: one element
+                    const int role = (tid >> 5) & 1, g = (tid & 31) >> 2, t = tid & 3;
+                    const int src = h == 0 ? 3 : 0;
+                    const double sgn = h == 0 ? 1.0 : -1.0;
+                    const double d0 = sD[g + 8 * t], d1 = sD[g + 8 * (4 + t)];
+                    const double rx = sgn * sg->met[0], sy = sgn * sg->met[4], tz = sgn * sg->met[8];
+                    const double* z = sz + (2 * h + role) * N2 + 8 * g + 2 * t;
+                    const double2* zlo = reinterpret_cast<const double2*>(z);
+                    const double2* zhi = reinterpret_cast<const double2*>(z + 4 * N2);
+                    const double* const D64 = CONSTD ? Dc : sD;
+                    if (role == 0)
+                        dmma8_columns<0, CS>(P, su, su + src * CS, sflux, g, t, 3 - src, d0, d1, rx, sy, tz, ebase,
+                                             D64, zlo, zhi);
+                    else
+                        dmma8_columns<1, CS>(P, su, su + src * CS, sflux, g, t, 3 - src, d0, d1, rx, sy, tz, ebase,
+                                             D64, zlo, zhi);
+                    return;
+                }
+                columns(0.0f);
+            } else if (fb64) columns(0.0);
             else columns(0.0f);
         } else {
             columns(TC(0));
