@@ -313,7 +313,7 @@ struct PoolPull {
     }
 };
 
-template <int N, int EPB, int MINB, bool KSM, bool PULL, bool CD>
+template <int N, int EPB, int MINB, bool KSM, bool PULL, bool CD, int KIO>
 __global__ void __launch_bounds__(EPB * 2 * N * N, MINB)
 batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
                     const __grid_constant__ BatchStage bs, const __grid_constant__ DParam dp) {
@@ -326,10 +326,11 @@ batch_bulk_n_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restric
     }
     const StageParams P = slot_params(S, bs);
     if constexpr (PULL)
-        stage::bulk_tile<N, GEO_BOX, 2, EPB, CD, false, KSM, true>(P, w.e0, smem, threadIdx.x, dp.d,
-                                                                   PoolPull<N>{slots, work, bs.stage});
+        stage::bulk_tile<N, GEO_BOX, 2, EPB, CD, false, KSM, true, false, false, false, KIO>(
+            P, w.e0, smem, threadIdx.x, dp.d, PoolPull<N>{slots, work, bs.stage});
     else
-        stage::bulk_tile<N, GEO_BOX, 2, EPB, CD, false, KSM, true>(P, w.e0, smem, threadIdx.x, dp.d);
+        stage::bulk_tile<N, GEO_BOX, 2, EPB, CD, false, KSM, true, false, false, false, KIO>(P, w.e0, smem, threadIdx.x,
+                                                                                             dp.d);
 }
 
 template <int N, int EPB, int MINB, bool KSM, bool CD>
@@ -356,12 +357,35 @@ cudaError_t launch_tiles(K kern, int threads, std::atomic<int>* attr_set, const 
     return launch_overlapped(kern, ntiles, threads, smem, st, bs.overlap(), slots, work, bs, dp);
 }
 
+template <int N, int EPB, int MINB, bool KSM, bool PULL, bool CD, int KIO>
+cudaError_t launch_bulk_kio(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                            const DParam& dp, cudaStream_t st) {
+    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
+    return launch_tiles<N, EPB, KSM>(batch_bulk_n_kernel<N, EPB, MINB, KSM, PULL, CD, KIO>, EPB * 2 * N * N, attr_set,
+                                     bs, slots, work, ntiles, dp, st);
+}
+
+// A kernel of its own for the first, the inner and the last stage, as in launch_bulk; without
+// the parameters' D (CD), a rare pool, one that tests at run time.
 template <int N, int EPB, int MINB, bool KSM, bool PULL, bool CD>
 cudaError_t launch_bulk_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                           const DParam& dp, cudaStream_t st) {
-    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
-    return launch_tiles<N, EPB, KSM>(batch_bulk_n_kernel<N, EPB, MINB, KSM, PULL, CD>, EPB * 2 * N * N, attr_set, bs,
-                                     slots, work, ntiles, dp, st);
+#define NWB_KIO(x) launch_bulk_kio<N, EPB, MINB, KSM, PULL, CD, x>(bs, slots, work, ntiles, dp, st)
+    if constexpr (!CD) return NWB_KIO(0);
+    else {
+        if (ntiles > 0) {
+            switch (stage_kio(bs.stage)) {
+                case kKWrite: return NWB_KIO(kKWrite);
+                case kKRead: return NWB_KIO(kKRead);
+                default: return NWB_KIO(kKRead | kKWrite);
+            }
+        }
+        cudaError_t e = NWB_KIO(kKWrite);
+        if (e == cudaSuccess) e = NWB_KIO(kKRead);
+        if (e == cudaSuccess) e = NWB_KIO(kKRead | kKWrite);
+        return e;
+    }
+#undef NWB_KIO
 }
 
 template <int N, bool CD>

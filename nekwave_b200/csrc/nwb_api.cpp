@@ -376,6 +376,7 @@ struct nwb_solver {
         }
         for (int x = 0; x < N; ++x) P.zl[x] = hzl[x];
         for (int d = 0; d < 3; ++d) P.snel[d] = snel[d];
+        for (int d = 0; d < 2 && snel[0] > 0; ++d) nwb::set_divider(snel[d], &P.sdiv[d], &P.sshift[d]);
         P.spmask = spmask;
         return P;
     }

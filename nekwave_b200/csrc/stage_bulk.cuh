@@ -189,7 +189,7 @@ __device__ __forceinline__ bool bulk_wait_tile(const StageParams& P, unsigned ch
 // right after it has issued the tile's copies (NoPull, or a functor that pulls a
 // later block's tile into L2).
 template <int N, int GEO, int KS, int EPB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
-          bool VROW = false, bool ILP2 = false, bool F32 = false, class Pull = NoPull>
+          bool VROW = false, bool ILP2 = false, bool F32 = false, int KIO = 0, class Pull = NoPull>
 __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, unsigned char* smem,
                                           const int tid, const double* Dc, const Pull& pull = Pull(),
                                           const float* Dcf = nullptr) {
@@ -218,8 +218,7 @@ __device__ __forceinline__ void bulk_tile(const StageParams& P, const int e0, un
     const ElemGeo* sg = reinterpret_cast<const ElemGeo*>(smem + L::geo0);
     const int* sc = reinterpret_cast<const int*>(smem + L::conn0) + ((e0 * 6) & 3);
     double* sflux = reinterpret_cast<double*>(smem + L::flux0);
-    compute2<N, GEO, F32, KS, EPB, true, false, CONSTD, EARLY, false, DSMEM, CtaBar, L::CSR, KSM, VROW,
-             ILP2>(
+    compute2<N, GEO, F32, KS, EPB, true, false, CONSTD, EARLY, false, DSMEM, CtaBar, L::CSR, KSM, VROW, ILP2, KIO>(
         P, e0, su, sg, sc, sD, sflux, smem + L::uc, tid, G, Dc, CtaBar(), sk, Dcf);
 }
 
@@ -261,30 +260,56 @@ struct MeshPull {
 // instead of DRAM; 0: no pull.  On B200 this pays where few blocks are resident
 // (6 and 9 points: 3 and 2 per SM), whose tile waits the other blocks hide least.
 template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
-          bool ZCOL, bool VROW, bool ILP2, int AHEAD, bool F32>
+          bool ZCOL, bool VROW, bool ILP2, int AHEAD, bool F32, int KIO>
 __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     stage_bulk_kernel(const __grid_constant__ StageParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int t = bulk_tile_index<EPB, ZCOL>(P, blockIdx.x);
     if constexpr (AHEAD > 0)
-        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2, F32>(
+        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2, F32, KIO>(
             P, t * EPB, smem, threadIdx.x, P.Dc, MeshPull<N * N * N, EPB, MINB, AHEAD, ZCOL>{P}, P.Dcf);
     else
-        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2, F32>(P, t * EPB, smem, threadIdx.x, P.Dc,
-                                                                              NoPull(), P.Dcf);
+        bulk_tile<N, GEO, KS, EPB, CONSTD, DSMEM, KSM, EARLY, VROW, ILP2, F32, KIO>(P, t * EPB, smem, threadIdx.x,
+                                                                                   P.Dc, NoPull(), P.Dcf);
 }
 
 template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
-          bool ZCOL, bool VROW, bool ILP2, int AHEAD = 0, bool F32 = false>
-cudaError_t launch_bulk(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
+          bool ZCOL, bool VROW, bool ILP2, int AHEAD, bool F32, int KIO>
+cudaError_t launch_bulk_kio(const StageParams* p, cudaStream_t st) {
     using L = BulkLayout<N, EPB, KSM, GEO, F32>;
-    constexpr int threads = EPB * KS * N * N;
-    auto kern = stage_bulk_kernel<N, GEO, KS, EPB, MINB, CONSTD, DSMEM, KSM, EARLY, ZCOL, VROW, ILP2, AHEAD, F32>;
-    if (cfg) *cfg = StageConfig{KS, EPB, threads, L::total, KSM ? 1 : 0, MINB};
+    auto kern = stage_bulk_kernel<N, GEO, KS, EPB, MINB, CONSTD, DSMEM, KSM, EARLY, ZCOL, VROW, ILP2, AHEAD, F32, KIO>;
     static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
     if (cudaError_t e = set_smem_once(kern, L::total, attr_set); e != cudaSuccess) return e;
     if (!p) return cudaSuccess;
-    return launch_overlapped(kern, (p->nelt + EPB - 1) / EPB, threads, L::total, st, (p->kio & kOverlap) != 0, *p);
+    return launch_overlapped(kern, (p->nelt + EPB - 1) / EPB, EPB * KS * N * N, L::total, st,
+                             (p->kio & kOverlap) != 0, *p);
+}
+
+// SPEC: a kernel of its own for the first, the inner and the last stage of a step, without
+// the tests on the register's accesses in the plane loop (the defaults; the other
+// shapes test at run time).  B200, per step: 64x64x32 elements of 6 points 5393 -> 5260 us,
+// 20^3 of 10 points 1806 -> 1782 us.
+template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
+          bool ZCOL, bool VROW, bool ILP2, int AHEAD = 0, bool F32 = false, bool SPEC = false>
+cudaError_t launch_bulk(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
+    using L = BulkLayout<N, EPB, KSM, GEO, F32>;
+    if (cfg) *cfg = StageConfig{KS, EPB, EPB * KS * N * N, L::total, KSM ? 1 : 0, MINB};
+#define NWB_KIO(x) launch_bulk_kio<N, GEO, KS, EPB, MINB, CONSTD, DSMEM, KSM, EARLY, ZCOL, VROW, ILP2, AHEAD, F32, x>(p, st)
+    if constexpr (!SPEC) return NWB_KIO(0);
+    else {
+        if (p) {
+            switch (p->kio & (kKRead | kKWrite)) {
+                case kKWrite: return NWB_KIO(kKWrite);
+                case kKRead: return NWB_KIO(kKRead);
+                default: return NWB_KIO(kKRead | kKWrite);
+            }
+        }
+        cudaError_t e = NWB_KIO(kKWrite);
+        if (e == cudaSuccess) e = NWB_KIO(kKRead);
+        if (e == cudaSuccess) e = NWB_KIO(kKRead | kKWrite);
+        return e;
+    }
+#undef NWB_KIO
 }
 
 // Shapes of the general classes (affine and per-node geometry) in FP64: the bulk-copy
@@ -314,7 +339,8 @@ template <int N, int GEO>
 cudaError_t launch_general(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
     using Sh = GeneralShape<N>;
     constexpr bool cd = (GEO == GEO_NODAL ? Sh::CDN : Sh::CDA) != 0;
-    return launch_bulk<N, GEO, 2, Sh::EPB, Sh::MINB, cd, false, true, true, false, false, false>(p, st, cfg);
+    return launch_bulk<N, GEO, 2, Sh::EPB, Sh::MINB, cd, false, true, true, false, false, false, 0, false, true>(p, st,
+                                                                                                               cfg);
 }
 
 // Shapes of the axis-aligned class in FP32-bulk at 4 to 9 points (on): the bulk-copy tile
@@ -339,7 +365,7 @@ template <int N>
 cudaError_t launch_f32(const StageParams* p, cudaStream_t st, StageConfig* cfg) {
     using Sh = F32Shape<N>;
     return launch_bulk<N, GEO_BOX, 2, Sh::EPB, Sh::MINB, Sh::CD != 0, false, Sh::KSM != 0, true, false, false, false, 0,
-                       true>(p, st, cfg);
+                       true, true>(p, st, cfg);
 }
 
 }  // namespace stage

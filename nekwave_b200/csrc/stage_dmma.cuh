@@ -59,8 +59,9 @@ __device__ __forceinline__ void dmma8_z_gather(const StageParams& P, int e, int 
     const long long S = P.stride;
     int v0, v1;
     if (P.snel[0] > 0) {
-        const int nx = P.snel[0], r = e / nx;
-        const int eB = struct_neighbour(P, e - r * nx, r % P.snel[1], r / P.snel[1], e, f);
+        int ex, ey, ez;
+        struct_coords(P, e, ex, ey, ez);
+        const int eB = struct_neighbour(P, ex, ey, ez, e, f);
         v0 = eB < 0 ? kConnPEC : eB * 512 + face_local<8>(f == 4 ? 5 : 4, i, j);
         v1 = v0 + 1;
     } else {

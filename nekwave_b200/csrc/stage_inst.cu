@@ -117,7 +117,8 @@ cudaError_t launch_variant(int vid, const StageParams* p, cudaStream_t st, Stage
                 if constexpr (GEO == GEO_BOX && !F32)
                     return launch_bulk<NWB_N, GEO, v.ks, v.epb, v.minb, (fl & 8) != 0, (fl & 64) != 0,
                                        (fl & 32) != 0, (fl & 16) != 0, (fl & 1) != 0, (fl & 4) != 0,
-                                       (fl & 128) != 0, (fl & 512) ? 2 : ((fl & 256) ? 1 : 0)>(p, st, cfg);
+                                       (fl & 128) != 0, (fl & 512) ? 2 : ((fl & 256) ? 1 : 0), false, I == kDefault>(p, st,
+                                                                                                          cfg);
                 else
                     return cudaErrorInvalidValue;
             } else if constexpr (GEO == GEO_BOX || I == kFirstGeneral) {

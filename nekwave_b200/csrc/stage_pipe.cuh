@@ -300,6 +300,14 @@ __device__ __forceinline__ int struct_neighbour(const StageParams& P, int ex, in
     }
 }
 
+// Element coordinates of element e of a structured box mesh.
+__device__ __forceinline__ void struct_coords(const StageParams& P, int e, int& ex, int& ey, int& ez) {
+    const int r = static_cast<int>((static_cast<unsigned long long>(e) * P.sdiv[0]) >> P.sshift[0]);
+    ez = static_cast<int>((static_cast<unsigned long long>(r) * P.sdiv[1]) >> P.sshift[1]);
+    ex = e - r * P.snel[0];
+    ey = r - ez * P.snel[1];
+}
+
 // The face of the neighbour that meets face f on a structured box.
 __device__ __forceinline__ int opposite_face(int f) { return f < 4 ? f ^ 2 : f ^ 1; }
 
@@ -334,10 +342,7 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
     const bool structured = !FROM_SMEM && P.snel[0] > 0;
     int ex = 0, ey = 0, ez = 0;
     if (structured) {
-        ex = e % P.snel[0];
-        const int r = e / P.snel[0];
-        ey = r % P.snel[1];
-        ez = r / P.snel[1];
+        struct_coords(P, e, ex, ey, ez);
     }
 #pragma unroll
     for (int q = 0; q < FPT; ++q) {
@@ -607,10 +612,7 @@ __device__ __forceinline__ void gather_box_nodes(const StageParams& P, const int
     const bool structured = !FROM_SMEM && P.snel[0] > 0;
     int ex = 0, ey = 0, ez = 0;
     if (structured) {
-        ex = e % P.snel[0];
-        const int r = e / P.snel[0];
-        ey = r % P.snel[1];
-        ez = r / P.snel[1];
+        struct_coords(P, e, ex, ey, ez);
     }
     auto node = [&](int f) -> int {
         if (structured) {
@@ -843,7 +845,7 @@ __device__ __forceinline__ void row_pairs(const double* p, double (&r)[N]) {
 // two independent FMA chains per sum instead of one (a different rounding order).
 template <int N, int GEO, bool F32, int KS, int EPB, bool SPLIT, bool PAD, bool CONSTD = false,
           bool EARLY = false, bool FACEDONE = false, bool DSMEM = false, class Bar = CtaBar,
-          int CSX = 0, bool KSM = false, bool VROW = false, bool ILP2 = false>
+          int CSX = 0, bool KSM = false, bool VROW = false, bool ILP2 = false, int KIO = 0>
 __device__ __forceinline__ void compute2(const StageParams& P, const int e0, const double* su,
                                          const ElemGeo* sg, const int* sc, const double* sD,
                                          double* sflux, unsigned char* smem_uc, const int tid,
@@ -1043,7 +1045,8 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
     const double* Uf = su + team * EN3;
     const double* Fl = sflux + team * flux_planes<GEO, SPLIT>() * N2;
     const double A = P.a, B = P.b, DT = P.dt;
-    const bool kread = (P.kio & kKRead) != 0, kwrite = (P.kio & kKWrite) != 0;
+    // KIO: the stage's accesses to k when the kernel was built for them (0: at run time)
+    const bool kread = ((KIO ? KIO : P.kio) & kKRead) != 0, kwrite = ((KIO ? KIO : P.kio) & kKWrite) != 0;
     const long long ebase = static_cast<long long>(e) * N3;
 
     if constexpr (SPLIT) {

@@ -155,8 +155,8 @@ __device__ __forceinline__ void quad_tile(const StageParams& P, const int e0, un
     double nb[4], zn[2][2];
     if (active) {
         if (P.snel[0] > 0) {
-            const int nx = P.snel[0], ny = P.snel[1];
-            const int r = e / nx, ex = e - r * nx, ez = r / ny, ey = r - ez * ny;
+            int ex, ey, ez;
+            struct_coords(P, e, ex, ey, ez);
             auto node = [&](int f) {
                 const int eB = struct_neighbour(P, ex, ey, ez, e, f);
                 return eB < 0 ? kConnPEC : eB * N3 + face_local<N>(opposite_face(f), i, j);
