@@ -150,12 +150,12 @@ void host_block_free(void* p) {
     }
 }
 
-bool snap_axis_normals(std::vector<ElemGeo>& geo) {
+bool snap_axis_normals(std::vector<ElemGeo>& geo, double tol) {
     constexpr int axis[6] = {1, 0, 1, 0, 2, 2};
     for (const ElemGeo& G : geo)
         for (int f = 0; f < 6; ++f)
             for (int c = 0; c < 3; ++c)
-                if (c != axis[f] && !(std::abs(G.nrm[f][c]) <= 1e-12)) return false;
+                if (c != axis[f] && !(std::abs(G.nrm[f][c]) <= tol)) return false;
     for (ElemGeo& G : geo)
         for (int f = 0; f < 6; ++f)
             for (int c = 0; c < 3; ++c)
@@ -244,7 +244,8 @@ nwb_status analyse_mesh(const nwb_mesh_desc* m, Analysis* A, bool true_pmc) {
             A->conn[6 * static_cast<size_t>(e) + f] = (eB << 6) | found;
         }
     }
-    if (affine && box) box = snap_axis_normals(A->egeo);
+    A->box_metrics = affine && box;
+    if (A->box_metrics) box = snap_axis_normals(A->egeo);
     A->geo = !affine ? nwb::GEO_NODAL : (box ? nwb::GEO_BOX : nwb::GEO_AFFINE);
     if (!affine) {
         A->egeo.clear();

@@ -1,5 +1,5 @@
 // nwb_internal.h -- types shared by the host side (nwb_api.cpp) and the CUDA
-// kernels (stage_kernels.cu, diag_kernels.cu).
+// kernels (stage_kernel.cuh and its siblings, diag_kernels.cu).
 #pragma once
 
 #include <atomic>
@@ -183,13 +183,14 @@ struct Analysis {
     std::vector<ElemGeo> egeo;
     std::vector<int> conn;
     std::vector<double> jac_e;
+    bool box_metrics = false;  // metrics constant per element and diagonal, whatever the normals
 };
+// Do the face normals of every element lie along the axes of an axis-aligned element
+// (faces 1, 3: x; 0, 2: y; 4, 5: z) to tol?  If so their other components are
+// set to exactly zero, which the axis-aligned class's kernels take for granted.
+bool snap_axis_normals(std::vector<ElemGeo>& geo, double tol = 1e-12);
 // true_pmc: bc_type 2 faces become kConnPMC (per-node class: neighbour -2) instead
 // of the reference's PEC mirror.
-// Do the face normals of every element lie along the axes of an axis-aligned element
-// (faces 1, 3: x; 0, 2: y; 4, 5: z) to 1e-12?  If so their other components are
-// set to exactly zero, which the axis-aligned class's kernels take for granted.
-bool snap_axis_normals(std::vector<ElemGeo>& geo);
 nwb_status analyse_mesh(const nwb_mesh_desc* m, Analysis* A, bool true_pmc = false);
 
 // Box meshes without per-node arrays (box_mesh.cpp).

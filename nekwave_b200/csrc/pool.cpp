@@ -689,7 +689,11 @@ nwb_status nwb_pool_add(nwb_pool* p, const nwb_mesh_desc* m, double c0, double d
     } catch (const std::bad_alloc&) {
         return set_error(NWB_ENOMEM, "nwb_pool_add: out of host memory");
     }
-    if (A.geo != nwb::GEO_BOX)
+    // Elements a ten-thousandth as thick as wide can have normals further off the axes than
+    // 1e-12 from the rounding of their corners alone; the pool has no affine class to sort
+    // them into and takes them as axis-aligned.
+    const bool box = A.geo == nwb::GEO_BOX || (A.box_metrics && nwb::snap_axis_normals(A.egeo, 1e-9));
+    if (!box)
         return set_error(NWB_EINVAL, "nwb_pool_add: the pool takes axis-aligned affine (box) meshes");
     for (int i = 0; i < nprobes; ++i)
         if (probe_elem[i] < 0 || probe_elem[i] >= m->nelt)

@@ -62,6 +62,21 @@ def test_normals_off_the_axes_leave_the_axis_aligned_class(gpu, N):
     s.finalize()
 
 
+def test_pool_takes_normals_off_the_axes_by_rounding(gpu):
+    """1e-11 moves one right-hand side by about as much relative to its largest entry."""
+    m = O.box_mesh(4, (2, 2, 2), (0, 0, 0), (1, 1, 1))
+    t = 1e-11
+    m.nx, m.ny = m.nx - t * m.ny, t * m.nx + m.ny
+    dt = 0.1 * O.dxmin(m)
+    u = random_state(m, 4)
+    pool = CavityPool(64 << 20, max_slots=2)
+    s = pool.add(solver_for(m, 1.0)._keep_mesh, 1.0, dt, 3)
+    pool.upload(s, u)
+    pool.step(3)
+    assert rel_l2(pool.results(s, energy=False, probes=False)["state"], O.step(m, 1.0, dt, 3, u)[0]) < 1e-9
+    pool.close()
+
+
 @pytest.mark.parametrize("N", range(2, 11))
 @pytest.mark.parametrize("kind", ["affine", "nodal"])
 def test_general_shapes_with_ragged_tiles(gpu, N, kind):
