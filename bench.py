@@ -38,7 +38,9 @@ sys.path.insert(0, ROOT)
 METRIC = "GDOF-stage/s"
 WORKLOAD = dict(workload="periodic_box_32x32x32_N8_central", nel=(32, 32, 32), N=8,
                 periodic=True, c0=0.0, cfl=0.5, sigma=0.1)
-BYTES_PER_DOF_STAGE = 32  # FP64 u and k, each read and written once
+# FP64, mean of the five stages of a step: u read and written in each, k written in the first
+# four and read in the last four (144 B per DOF and step)
+BYTES_PER_DOF_STAGE = 144 / 5
 
 
 def workload_spec(name, nel_override, seed):
@@ -385,7 +387,7 @@ def run_batch(args, rank, world):
                          "frac": achieved / peak, "traffic": pool_traffic(seed=args.seed + rank),
                          "peak_source": peak_kind,
                          "kernel": "one stage: the per-N stage kernels of every N present",
-                         "per_unit": "32 B per DOF-stage x 6 x nodes (all cavities) per stage"},
+                         "per_unit": "28.8 B per DOF-stage (144 B per step) x 6 x nodes (all cavities)"},
             "serial_fp64_single_mesh": {"value": serial, "unit": METRIC,
                                         "sample": "first 48 instances solved one at a time with "
                                                   "the single-mesh FP64 solver (CUDA graph per step)",

@@ -1,10 +1,12 @@
-// batch.cu -- kernels of the multi-cavity pool: one persistent launch per LSRK
-// stage advances every resident cavity, whatever its N and element count.
+// batch.cu -- kernels of the multi-cavity pool.
 //
-// Blocks of kBatchThreads threads take tiles (EPB consecutive elements of one
-// cavity) from a work list through a per-stage atomic counter, largest tiles
-// first, and run the same fused stage tile as the single-mesh kernel
-// (stage_tile in stage_kernel.cuh) with the N-specialised shape of that tile.
+// One launch per order and LSRK stage advances that order's resident cavities:
+// a block takes the tile (EPB consecutive elements of one cavity) that the work
+// list has at its index and runs the single-mesh default's tile of that order
+// (stage_bulk.cuh, stage_quad.cuh, stage_dmma.cuh) on the slot's arrays.  The other
+// mode is one persistent launch per stage whatever the orders: blocks of
+// kBatchThreads threads take tiles through a per-stage atomic counter, largest
+// first, and run the tile of its order that fits such a block.
 // A cavity's arithmetic does not depend on which other cavities share the
 // launch, so each result is bit-identical alone and in any mix.
 #include "batch.cuh"
@@ -23,7 +25,7 @@ using stage::stage_tile;
 
 // Shape per N for the batch kernel's blocks (kBatchThreads = 128): KS threads
 // per column, EPB elements, ALG the kernel family -- the single-mesh default's
-// family and arithmetic for each N (stage_variants.h entry 0), in a shape that
+// arithmetic for each N, in a shape that
 // fits, so a cavity in the pool evolves bit for bit as it does alone.  N = 8 in
 // FP64 runs the field-split tensor-core tile (stage_dmma.cuh, 128 threads) as the
 // single-mesh default does; ALG below is its FP32-bulk shape.

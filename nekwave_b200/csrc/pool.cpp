@@ -2,7 +2,7 @@
 //
 // The reference solves one mesh per process (Case::simulate, src/case.cpp:529-660).
 // A pool keeps many cavities ("slots") resident in HBM at once and advances all
-// active ones with one persistent launch per LSRK stage (batch.cu):
+// active ones with one launch per LSRK stage and order (batch.cu):
 //   * admission by a fixed HBM budget: the pool owns one arena allocated at
 //     creation and sub-allocates every slot's buffers from it, so admitting a
 //     cavity never calls cudaMalloc and fails with NWB_EBUSY when it does not fit
@@ -12,8 +12,9 @@
 //     staging and every copy is queued in stream order behind the steps in
 //     flight; status and results can be read back the same way
 //     (nwb_pool_query_begin/end, nwb_pool_results_async);
-//   * a step of all slots is one CUDA graph (5 stage launches, diagnostics,
-//     step epilogue) replayed as often as needed; slots that have taken their
+//   * a step of all slots, or a few steps, is one CUDA graph (per order a chain of
+//     stage launches; energy tiles where a step records energy; step epilogue)
+//     replayed as often as needed; slots that have taken their
 //     steps fall idle on the device, and slots can be added or removed between
 //     replays (the graph reads the slot table and the work list from device
 //     memory, so it stays valid);
@@ -412,9 +413,6 @@ struct nwb_pool {
         return false;
     }
 
-    // Queues nsteps steps, kManySteps at a time while that many are left: an order's chain
-    // then runs on through them, and no launch is spent on energy tiles in steps that record
-    // none.  B200, 16 small cavities, per step: 79 -> 74 us.
     // A pool whose cavities change often keeps to single steps: the longer graph is captured
     // for a call of at least four of it.
     bool use_many(int nsteps) const {
@@ -427,6 +425,9 @@ struct nwb_pool {
         return g ? NWB_OK : capture(0, &g, many ? kManySteps : 1, diag != 0);
     }
 
+    // Queues nsteps steps, kManySteps at a time while that many are left: an order's chain
+    // then runs on through them, and no launch is spent on energy tiles in steps that record
+    // none.  B200, 16 small cavities, per step: 79 -> 74 us.
     nwb_status run(int nsteps) {
         nwb_status r = ensure_graph();
         if (r != NWB_OK) return r;

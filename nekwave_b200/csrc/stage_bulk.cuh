@@ -8,8 +8,10 @@
 // face and column phases as in the other one-tile forms, with k read from
 // shared memory.  Against the per-thread cp.async loads of those forms this
 // takes a few hundred load instructions per block off the issue slots, and the
-// column phase no longer waits on L2 for each plane's k: on B200 the stage runs
-// 4-10% faster at 5, 6, 7 and 9 points (the defaults there).
+// column phase no longer waits on L2 for each plane's k.  It is the FP64 default of
+// the axis-aligned class but at 4 points (four threads per column) and 8 (tensor-core
+// tile), and carries the general classes and FP32-bulk from 4 points up
+// (stage_variants.h, GeneralShape and F32Shape have the figures).
 //
 // Bulk copies start and end on 16-byte boundaries.  A tile whose first node or
 // length is odd (odd N) is copied from the boundary at or below its first value
