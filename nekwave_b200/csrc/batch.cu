@@ -195,8 +195,12 @@ __device__ __forceinline__ StageParams slot_params(const SlotDev& S, const Batch
     P.fplus = nullptr;
     P.nfp = 0;
     P.err = nullptr;
-    P.snel[0] = P.snel[1] = P.snel[2] = 0;  // connections from the slot's table
-    P.spmask = 0;
+    for (int x = 0; x < 3; ++x) P.snel[x] = S.snel[x];
+    for (int x = 0; x < 2; ++x) {
+        P.sdiv[x] = S.sdiv[x];
+        P.sshift[x] = S.sshift[x];
+    }
+    P.spmask = S.spmask;
     for (int x = 0; x < 10; ++x) P.zl[x] = S.zl[x];
     P.c0 = S.c0;
     P.a = bs.a;

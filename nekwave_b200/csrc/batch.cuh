@@ -31,8 +31,9 @@ struct SlotDev {
     int done;               // steps taken
     int par;                // ping-pong parity at the start of the next step
     int active;             // 1 while done < nsteps
-    int energy_now;         // set by the diagnostics when this step records energy
-    int _pad;
+    int snel[3], spmask;    // structured box: elements per axis and periodic axes, or 0
+    unsigned sdiv[2];       // StageParams::sdiv, sshift
+    int sshift[2];
 };
 
 // One tile of work: EPB consecutive elements of one slot.

@@ -597,10 +597,9 @@ int box_conn(int ex, int ey, int ez, int f, const int nel[3], int pm) {
     return nb < 0 ? nwb::kConnPEC : ((nb << 6) | (opp[f] << 3));
 }
 
-// Recognises the connection table of a structured box mesh (elements x-fastest,
-// identity face orientations): the stage kernels can then find neighbours from
-// the element index.  Returns false and leaves nel at 0 for any other table.
-bool detect_structure(const std::vector<int>& conn, int nelt, int nel[3], int* pm) {
+}  // namespace
+
+bool nwb::detect_structure(const int* conn, int nelt, int nel[3], int* pm) {
     nel[0] = nel[1] = nel[2] = 0;
     *pm = 0;
     auto step = [&](int e, int f) { const int cd = conn[6 * static_cast<size_t>(e) + f];
@@ -636,6 +635,8 @@ bool detect_structure(const std::vector<int>& conn, int nelt, int nel[3], int* p
     *pm = mask;
     return true;
 }
+
+namespace {
 
 // Allocates and uploads a solver from analysed geometry.  m supplies the
 // per-node arrays of the general class and may be null for the affine classes.
@@ -711,7 +712,7 @@ nwb_status create_solver(const nwb_mesh_desc* m, int N, int nelt, const double* 
         ce = cudaMemset(s->dconn + 6 * static_cast<size_t>(nelt), 0, 4 * sizeof(int));
         if (ce != cudaSuccess) return bail(fail(NWB_ECUDA, "memset: %s", cudaGetErrorString(ce)));
         NWB_H2D(s->djac_e, A.jac_e.data(), sizeof(double) * nelt);
-        detect_structure(A.conn, nelt, s->snel, &s->spmask);
+        nwb::detect_structure(A.conn.data(), nelt, s->snel, &s->spmask);
     } else {
         const size_t nfp = static_cast<size_t>(s->nfp);
         try {

@@ -185,6 +185,10 @@ struct Analysis {
     std::vector<double> jac_e;
     bool box_metrics = false;  // metrics constant per element and diagonal, whatever the normals
 };
+// Recognises the connection table of a structured box mesh (elements x-fastest, identity face
+// orientations): the stage kernels can then find neighbours from the element index.  Returns
+// false and leaves nel at 0 for any other table.
+bool detect_structure(const int* conn, int nelt, int nel[3], int* pm);
 // Do the face normals of every element lie along the axes of an axis-aligned element
 // (faces 1, 3: x; 0, 2: y; 4, 5: z) to tol?  If so their other components are
 // set to exactly zero, which the axis-aligned class's kernels take for granted.

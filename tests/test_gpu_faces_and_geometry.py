@@ -150,3 +150,36 @@ def test_few_and_many_elements_give_a_cavity_the_same_bits(gpu, N):
             np.testing.assert_array_equal(pool.results(slots[nels.index(LARGE[N])])["state"], s.downloadState())
             s.finalize()
         pool.close()
+
+
+@pytest.mark.parametrize("periodic", [(True, True, True), (True, False, True), (False, False, False)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_pool_and_solver_find_the_same_neighbours(gpu, periodic, precision):
+    """Boxes one element wide, periodic and closed, structured in solver and pool: the same bits."""
+    pulses = [(1.0 - 0.2 * c, 0.4, 0.6, 0.5, 0.2 + 0.05 * c) for c in range(6)]
+    boxes = [(N, nel) for N in (3, 4, 6, 8, 9) for nel in ((1, 1, 1), (1, 3, 2), (2, 1, 5), (3, 2, 1))]
+    pool = CavityPool(256 << 20, max_slots=len(boxes), precision=precision)
+    slots = [pool.add_box(N, nel, (0, 0, 0), (1, 1, 1), 1.0, 1e-3, 3, periodic=periodic) for N, nel in boxes]
+    for q in slots:
+        pool.init_pulse(q, pulses)
+    pool.step(3)
+    for q, (N, nel) in zip(slots, boxes):
+        s = DgSolver(precision)
+        s.initializeBox(N, nel, (0, 0, 0), (1, 1, 1), 1.0, periodic=periodic)
+        s.initPulse(pulses)
+        s.steps(1e-3, 3)
+        np.testing.assert_array_equal(pool.results(q, energy=False, probes=False)["state"], s.downloadState())
+        s.finalize()
+    pool.close()
+
+
+def test_pool_takes_a_table_that_is_no_structured_box(gpu):
+    m = half_turned_box(5, (3, 2, 2))
+    dt = 0.1 * O.dxmin(m)
+    u = random_state(m, 5)
+    pool = CavityPool(64 << 20, max_slots=2)
+    s = pool.add(solver_for(m, 1.0)._keep_mesh, 1.0, dt, 3)
+    pool.upload(s, u)
+    pool.step(3)
+    assert rel_l2(pool.results(s, energy=False, probes=False)["state"], O.step(m, 1.0, dt, 3, u)[0]) < 1e-12
+    pool.close()
