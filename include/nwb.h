@@ -279,13 +279,13 @@ nwb_status nwb_time_stage_kernel(nwb_solver* s, double dt, int nstages, float* m
  * sub-allocated from it, so nwb_pool_add never calls cudaMalloc and returns
  * NWB_EBUSY when the cavity does not fit (admission by HBM budget).  Outside the
  * arena the pool holds its slot table and two work lists (sized at creation for
- * any admissible set of cavities: 16 bytes each per 18 KB of budget at most) and
- * a pinned host staging area (2 x 48 MB).  nwb_pool_add, _add_box, _init_pulse,
+ * any admissible set of cavities: 16 bytes each per 18 KB of budget at most, and
+ * 0.9 MB) and a pinned host staging area (2 x 48 MB).  nwb_pool_add, _add_box, _init_pulse,
  * _upload (states up to 48 MB), _remove and _step queue their device work in
  * stream order and return without waiting for the steps already in flight.
  * nwb_pool_step advances every uploaded, unfinished slot by up to nsteps steps
  * with one launch per LSRK stage and N present (or one persistent launch for
- * every N, nwb_pool_set_mode), replayed from one CUDA graph per step; a slot stops
+ * every N, nwb_pool_set_mode), replayed from CUDA graphs of one or four steps; a slot stops
  * by itself after its own nsteps.  Slots take axis-aligned box meshes (nwb_mesh_desc as above),
  * their own c0 and dt, up to 8 probes given as (element, tensor Lagrange
  * weights [3][N]) as ProbeManager builds them (src/probe.cpp:33-189), and record

@@ -704,7 +704,7 @@ nwb_status create_solver(const nwb_mesh_desc* m, int N, int nelt, const double* 
     if (s->geo != nwb::GEO_NODAL) {
         NWB_TRY(dalloc(&s->dgeo, static_cast<size_t>(nelt), &tot));
         // padded to a multiple of four entries: bulk copies of a tile's connections
-        // are 16-byte aligned at both ends (stage_ws.cuh)
+        // are 16-byte aligned at both ends (stage_bulk.cuh)
         NWB_TRY(dalloc(&s->dconn, 6 * static_cast<size_t>(nelt) + 4, &tot));
         NWB_TRY(dalloc(&s->djac_e, static_cast<size_t>(nelt), &tot));
         NWB_H2D(s->dgeo, A.egeo.data(), sizeof(nwb::ElemGeo) * nelt);
