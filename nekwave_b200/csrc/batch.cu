@@ -581,7 +581,7 @@ batch_epilogue_kernel(SlotDev* __restrict__ slots, const int* __restrict__ slot_
                 const int i = m % N, j = (m / N) % N, k = m / N2;
                 w[q] = wr[i] * ws[j] * wt[k];
 #pragma unroll
-                for (int c = 0; c < 6; ++c) v[q][c] = __ldcg(up + c * st + m);
+                for (int c = 0; c < 6; ++c) v[q][c] = stage::ld_state(up + c * st + m);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q)

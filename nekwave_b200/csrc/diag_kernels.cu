@@ -162,10 +162,11 @@ maxnorm_final_kernel(const double* __restrict__ partial, int n, double* __restri
 // them in node order, with separate multiply and add roundings as on the host, so the
 // values equal the reference's bit for bit on the same state and weights.  (One thread
 // per component loading as it adds waited for L2 at every fourth node.)  The weights are
-// loaded before grid_wait(): the launch may overlap the stage before it.
+// loaded before the wait: the launch may overlap the stage before it.  So the state is
+// not (launch_overlapped): coherent loads behind the wait.
 constexpr int kProbeThreads = 192;
 __global__ void __launch_bounds__(kProbeThreads)
-probe_kernel(const double* __restrict__ u, long long stride, int N3,
+probe_kernel(const double* u, long long stride, int N3,
              const long long* __restrict__ offset, const double* __restrict__ w, int nprobes,
              double* __restrict__ out) {
     __shared__ double prod[6][1000];
@@ -176,7 +177,7 @@ probe_kernel(const double* __restrict__ u, long long stride, int N3,
     for (int p = lane; p < N3; p += 32) prod[c][p] = wp[p];
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
 #pragma unroll 4
-    for (int p = lane; p < N3; p += 32) prod[c][p] = __dmul_rn(prod[c][p], up[p]);
+    for (int p = lane; p < N3; p += 32) prod[c][p] = __dmul_rn(prod[c][p], __ldcg(up + p));
     __syncwarp();
     if (lane != 0) return;
     double acc = 0.0;

@@ -42,6 +42,13 @@ cudaError_t set_smem_once(K kern, int smem, std::atomic<int>* flags) {
 // elements of 5 points 20.5 -> 16.4 us, 792 of 7 points 67.8 -> 66.0, 512 of 8 points 52.6 ->
 // 49.7; large meshes the same (32^3 elements of 8 points 2910 -> 2820 us with the copies
 // now issued before a block's other work).
+//
+// What a kernel so launched may read how: tables that no kernel writes (D, geometry,
+// connections, metrics, weights) at any time and by any path.  The states, the LSRK register
+// and whatever else a launch before it writes, only behind grid_wait() and by coherent loads
+// (stage::ld_state, cp.async, bulk copies): never by __ldg or through a const __restrict__
+// pointer, whose path asks that nothing writes the data while the kernel lives -- and up to
+// three launches live at once, the buffer one stage reads being the one the next writes.
 template <typename... P, typename... A>
 cudaError_t launch_overlapped(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, bool overlap,
                               const A&... args) {

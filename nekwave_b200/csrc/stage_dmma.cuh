@@ -75,7 +75,8 @@ __device__ __forceinline__ void dmma8_z_gather(const StageParams& P, int e, int 
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const double* u = P.u_in + (c == 0 ? ca : cb) * S;
-        z[c] = pair ? __ldg(reinterpret_cast<const double2*>(u + v0)) : make_double2(__ldg(u + v0), __ldg(u + v1));
+        z[c] = pair ? ld_state(reinterpret_cast<const double2*>(u + v0))
+                    : make_double2(ld_state(u + v0), ld_state(u + v1));
     }
 }
 

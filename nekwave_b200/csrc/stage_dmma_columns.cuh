@@ -32,7 +32,7 @@ __device__ __forceinline__ void dmma8_columns(const StageParams& P, const double
     double* const o1 = P.u_out + (dst + ROLE) * S + ebase + m0;
     double* const o2 = P.u_out + (dst + 2) * S + ebase + m0;
     auto load_k = [&](const double* p) {
-        return kread ? __ldcg(reinterpret_cast<const double2*>(p)) : make_double2(0.0, 0.0);
+        return kread ? ld_state(reinterpret_cast<const double2*>(p)) : make_double2(0.0, 0.0);
     };
     auto update = [&](double* kp, double* op, const double* up, double2 kold, double r0, double r1) {
         const double kn0 = A * kold.x + DT * r0, kn1 = A * kold.y + DT * r1;

@@ -42,6 +42,14 @@ __device__ __forceinline__ void grid_launch_dependents() {
 }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
+// Loads of what the launch before may still have been writing when this one started (the
+// states and the LSRK register), behind grid_wait(): coherent at L2, where that
+// launch's stores are.  Not __ldg: its path is for data that nobody writes while the kernel
+// lives (launch_overlapped), which the tables are and these are not.  L1 gains nothing here:
+// a trace's 32-byte sectors are used by one warp once.
+__device__ __forceinline__ double ld_state(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ double2 ld_state(const double2* p) { return __ldcg(p); }
+
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc) {
     unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
@@ -267,7 +275,7 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const int e0,
                     for (int c = 0; c < 6; ++c) vals[c] = s_u[c * CS + sidx];
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) vals[c] = __ldg(P.u_in + c * S + vB);
+                    for (int c = 0; c < 6; ++c) vals[c] = ld_state(P.u_in + c * S + vB);
                 }
                 jmp[0] = vals[0] - Exm; jmp[1] = vals[1] - Eym; jmp[2] = vals[2] - Ezm;
                 jmp[3] = vals[3] - Hxm; jmp[4] = vals[4] - Hym; jmp[5] = vals[5] - Hzm;
@@ -421,7 +429,7 @@ __device__ __forceinline__ void stage_tile(const StageParams& P, const int e0,
         double kold[6];
 #pragma unroll
         for (int c = 0; c < 6; ++c)
-            kold[c] = !kread ? 0.0 : (KSMEM ? s_k[c * CS + sl] : __ldcg(P.k + c * S + g));
+            kold[c] = !kread ? 0.0 : (KSMEM ? s_k[c * CS + sl] : ld_state(P.k + c * S + g));
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
             const double kn = A * kold[c] + DT * rhs[c];

@@ -120,7 +120,7 @@ __device__ __forceinline__ void stage_tile_mma8(const StageParams& P, const int 
             if (o & 2) b = N - 1 - b;
             const long long vB = static_cast<long long>(eB) * N3 + face_local<N>(fB, a, b);
 #pragma unroll
-            for (int c = 0; c < 6; ++c) nb[d][c] = __ldg(P.u_in + c * S + vB);
+            for (int c = 0; c < 6; ++c) nb[d][c] = ld_state(P.u_in + c * S + vB);
         } else {
 #pragma unroll
             for (int c = 0; c < 6; ++c) nb[d][c] = 0.0;
@@ -133,7 +133,7 @@ __device__ __forceinline__ void stage_tile_mma8(const StageParams& P, const int 
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) kold[n][c] = kread ? __ldcg(P.k + c * S + gbase + tid + 128 * n) : 0.0;
+        for (int c = 0; c < 6; ++c) kold[n][c] = kread ? ld_state(P.k + c * S + gbase + tid + 128 * n) : 0.0;
     cp_async_wait<0>();
     __syncthreads();
 

@@ -400,7 +400,7 @@ __device__ __forceinline__ void gather2(const StageParams& P, const int e0, cons
             }
         }
 #pragma unroll
-        for (int c = 0; c < 6; ++c) G.nb[q][c] = __ldg(P.u_in + c * S + vB);
+        for (int c = 0; c < 6; ++c) G.nb[q][c] = ld_state(P.u_in + c * S + vB);
     }
 }
 
@@ -502,7 +502,7 @@ __device__ __forceinline__ void face_phase_global(const StageParams& P, const in
             const int pq = fp - f * N2;
             const long long g = static_cast<long long>(e) * N3 + face_local<N>(f, pq % N, pq / N);
 #pragma unroll
-            for (int c = 0; c < 6; ++c) own[q][c] = __ldg(P.u_in + c * S + g);
+            for (int c = 0; c < 6; ++c) own[q][c] = ld_state(P.u_in + c * S + g);
         }
     }
 #pragma unroll
@@ -662,10 +662,10 @@ __device__ __forceinline__ void gather_box_values(const StageParams& P, const in
             }
         }
         const double* u = P.u_in + vB;
-        v[0] = __ldg(u + ca * S);
-        v[1] = __ldg(u + cb * S);
-        v[2] = __ldg(u + (3 + ca) * S);
-        v[3] = __ldg(u + (3 + cb) * S);
+        v[0] = ld_state(u + ca * S);
+        v[1] = ld_state(u + cb * S);
+        v[2] = ld_state(u + (3 + ca) * S);
+        v[3] = ld_state(u + (3 + cb) * S);
     };
 #pragma unroll
     for (int x = 0; x < FPT; ++x) {
@@ -770,8 +770,8 @@ __device__ __forceinline__ void face_phase_box_global(const StageParams& P, cons
         const int ca = (f & 1) ? 1 : 2, cb = (f & 1) ? 2 : 0;
         const double* own = P.u_in + static_cast<long long>(e0 + team) * N3 + face_local<N>(f, p, q);
         double j[4], F[4];
-        box_jumps(G.vB[x], G.nb[x], __ldg(own + ca * S), __ldg(own + cb * S), __ldg(own + (3 + ca) * S),
-                  __ldg(own + (3 + cb) * S), j);
+        box_jumps(G.vB[x], G.nb[x], ld_state(own + ca * S), ld_state(own + cb * S), ld_state(own + (3 + ca) * S),
+                  ld_state(own + (3 + cb) * S), j);
         box_flux<TC>(__ldg(&Gp->nrm[f][(f & 1) ? 0 : 1]), P.c0, __ldg(&Gp->lift[f]), j, F);
         double* out = sflux + (team * 4 + f) * 4 * N2 + pq;
 #pragma unroll
@@ -1139,7 +1139,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
             for (int c = 0; c < 3; ++c)
                 knext[c] = !kread ? 0.0
                          : (KSM ? Kf[(dst + c) * CS + i + RP * j]
-                                : __ldcg(P.k + (dst + c) * S + ebase + i + N * j));
+                                : ld_state(P.k + (dst + c) * S + ebase + i + N * j));
         }
 #pragma unroll (CD ? N : 1)
         for (int k = 0; k < N; ++k) {
@@ -1154,12 +1154,12 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
 #pragma unroll
                     for (int c = 0; c < 3; ++c)
                         knext[c] = !kread ? 0.0
-                                 : (KSM ? Kf[(dst + c) * CS + ms + PP] : __ldcg(P.k + (dst + c) * S + g + N2));
+                                 : (KSM ? Kf[(dst + c) * CS + ms + PP] : ld_state(P.k + (dst + c) * S + g + N2));
                 }
             } else {
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    kold[c] = !kread ? 0.0 : (KSM ? Kf[(dst + c) * CS + ms] : __ldcg(P.k + (dst + c) * S + g));
+                    kold[c] = !kread ? 0.0 : (KSM ? Kf[(dst + c) * CS + ms] : ld_state(P.k + (dst + c) * S + g));
             }
             double mnow[GEO == GEO_NODAL ? 9 : 1];
             if constexpr (GEO == GEO_NODAL) {
@@ -1322,7 +1322,7 @@ __device__ __forceinline__ void compute2(const StageParams& P, const int e0, con
             double kold[6];
 #pragma unroll
             for (int c = 0; c < 6; ++c)
-                kold[c] = !kread ? 0.0 : (KSM ? sk[c * CS + team * EN3 + ms] : __ldcg(P.k + c * S + g));
+                kold[c] = !kread ? 0.0 : (KSM ? sk[c * CS + team * EN3 + ms] : ld_state(P.k + c * S + g));
             double rhs[6];
             if constexpr (GEO == GEO_BOX) {
                 TC Hz_r = 0, Hy_r = 0, Ez_r = 0, Ey_r = 0;

@@ -68,8 +68,8 @@ __device__ __forceinline__ void quad_columns(const StageParams& P, const double*
     double* const k2 = P.k + (dst + 2) * S + ebase + m0;
     double* const o1 = P.u_out + (dst + ROLE) * S + ebase + m0;
     double* const o2 = P.u_out + (dst + 2) * S + ebase + m0;
-    auto load_k1 = [&](int k) { return !kread ? 0.0 : (KSM ? k1s[N2 * k] : __ldcg(k1 + N2 * k)); };
-    auto load_k2 = [&](int k) { return !kread ? 0.0 : (KSM ? k2s[N2 * k] : __ldcg(k2 + N2 * k)); };
+    auto load_k1 = [&](int k) { return !kread ? 0.0 : (KSM ? k1s[N2 * k] : ld_state(k1 + N2 * k)); };
+    auto load_k2 = [&](int k) { return !kread ? 0.0 : (KSM ? k2s[N2 * k] : ld_state(k2 + N2 * k)); };
     auto update = [&](double* kp, double* op, double u, double kold, double r) {
         const double kn = A * kold + DT * r;
         if (kwrite) __stcs(kp, kn);
@@ -173,16 +173,16 @@ __device__ __forceinline__ void quad_tile(const StageParams& P, const int e0, un
     grid_wait();
     if (vB >= 0) {
         const double* u = P.u_in + vB;
-        nb[0] = __ldg(u + ca * S);
-        nb[1] = __ldg(u + cb * S);
-        nb[2] = __ldg(u + (3 + ca) * S);
-        nb[3] = __ldg(u + (3 + cb) * S);
+        nb[0] = ld_state(u + ca * S);
+        nb[1] = ld_state(u + cb * S);
+        nb[2] = ld_state(u + (3 + ca) * S);
+        nb[3] = ld_state(u + (3 + cb) * S);
     }
 #pragma unroll
     for (int s = 0; s < 2; ++s)
         if (zv[s] >= 0) {
-            zn[s][0] = __ldg(P.u_in + zd * S + zv[s]);
-            zn[s][1] = __ldg(P.u_in + zs * S + zv[s]);
+            zn[s][0] = ld_state(P.u_in + zd * S + zv[s]);
+            zn[s][1] = ld_state(P.u_in + zs * S + zv[s]);
         }
     if (!bulk_wait_tile<N, EPB, KSM, GEO_BOX, false>(P, smem, tid)) return;
     const int off = static_cast<int>((static_cast<long long>(e0) * N3) & 1) + team * N3;
