@@ -339,7 +339,7 @@ struct nwb_solver {
     size_t flush_bytes = 0;
     nwb::StageConfig cfg{};
     int variant = 0;
-    int dflt = 0;  // what variant 0 stands for on this mesh (nwb::stage_default_variant)
+    int dflt = 0;  // the shape that is variant 0 on this mesh (nwb::stage_default_variant)
     long long launches = 0;
     size_t device_bytes = 0;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
@@ -348,7 +348,9 @@ struct nwb_solver {
     bool is_box = false;
     nwb::BoxPulse box{};
 
-    int shape(int v) const { return v == 0 ? dflt : v; }
+    // Number of variant v in the list of shapes: on a mesh of few elements the shape for them
+    // and the large default swap their numbers, so that every shape has one.
+    int shape(int v) const { return v == 0 ? dflt : v == dflt ? 0 : v; }
 
     nwb::StageParams params(int stage, double dt) const {
         nwb::StageParams P{};

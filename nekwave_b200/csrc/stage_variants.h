@@ -27,7 +27,7 @@
 // while the tile's copies fly (at 4 points four threads per column); k in shared memory but
 // at 10 points, where it is read from L2 (the blocks that then fit pay more); the L2 pull
 // only at 6 points.  A mesh of few elements takes another shape as its variant 0
-// (NWB_SMALL).  Per step, former default -> now: 90^3 of 2 points 2080 -> 1574 us, 62^3 of 3
+// (NWB_SMALL), and there the number of that shape stands for the large default.  Per step, former default -> now: 90^3 of 2 points 2080 -> 1574 us, 62^3 of 3
 // points 2218 -> 1545 us, 50^3 of 4 points 1569 -> 1405 us, 22^3 of 9 points 1500 -> 1337 us
 // (there the pull and the z-column order had paid while the faces kept the L1 pipe busy),
 // 20^3 of 10 points 1995 -> 1703 us.
