@@ -313,6 +313,9 @@ nwb_status nwb_pool_init_pulse(nwb_pool* p, int slot, const double* pulse /* [30
 /* Initial state [6*npts]; the slot starts stepping with the next nwb_pool_step. */
 nwb_status nwb_pool_upload(nwb_pool* p, int slot, const double* host_state, size_t n);
 nwb_status nwb_pool_step(nwb_pool* p, int nsteps);      /* asynchronous */
+/* nwb_pool_sync, _query, _query_end and _results answer NWB_ETIMEOUT, the first of them that
+ * is called, when a stage kernel's bounded wait expired before the point that they wait for: the
+ * states stepped since the last such call are then not valid (as nwb_sync of a solver). */
 nwb_status nwb_pool_sync(nwb_pool* p);
 /* status[s]: -1 free, 0 added (no state yet), 1 running, 2 finished; done[s]:
  * steps taken.  Synchronises the pool's stream. */

@@ -143,7 +143,7 @@ batch_stage_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
         P.flift = nullptr;
         P.fplus = nullptr;
         P.nfp = 0;
-        P.err = nullptr;
+        P.err = nullptr;  // no bounded waits in this launch's tiles
         P.snel[0] = P.snel[1] = P.snel[2] = 0;  // connections from the slot's table
         P.spmask = 0;
         for (int x = 0; x < 10; ++x) P.zl[x] = S.zl[x];
@@ -173,6 +173,7 @@ batch_stage_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
 struct BatchStage {
     double a, b;
     int stage, dry;
+    int* err;  // the pool's status word: a bulk tile whose bounded wait expires records it there
     bool overlap() const { return stage > 0; }
 };
 
@@ -194,7 +195,7 @@ __device__ __forceinline__ StageParams slot_params(const SlotDev& S, const Batch
     P.flift = nullptr;
     P.fplus = nullptr;
     P.nfp = 0;
-    P.err = nullptr;
+    P.err = bs.err;
     for (int x = 0; x < 3; ++x) P.snel[x] = S.snel[x];
     for (int x = 0; x < 2; ++x) {
         P.sdiv[x] = S.sdiv[x];
@@ -648,9 +649,9 @@ int max_batch_smem() {
 }  // namespace
 
 cudaError_t launch_batch_stage_n(int N, int f32, int form, int stage, const SlotDev* slots,
-                                 const WorkItem* work, int ntiles, int dry, const double* Dh,
+                                 const WorkItem* work, int ntiles, int dry, const double* Dh, int* err,
                                  cudaStream_t st) {
-    const BatchStage bs{dry ? 0.0 : kRk4a[stage], dry ? 0.0 : kRk4b[stage], stage, dry};
+    const BatchStage bs{dry ? 0.0 : kRk4a[stage], dry ? 0.0 : kRk4b[stage], stage, dry, err};
     switch (N) {
 #define NWB_CASE(n) \
         case n: return f32 ? launch_n<n, true>(form, bs, slots, work, ntiles, Dh, st) \

@@ -59,8 +59,9 @@ cudaError_t launch_batch_stage(int f32, int stage, const SlotDev* slots, const W
 // the host when every resident cavity of that N shares it (lets the kernel take D
 // from its parameters), else null.
 // form: batch_form_n of that N's resident elements, also when the tiles were cut.
+// err: device pointer of the word in which an expired bounded wait is recorded.
 cudaError_t launch_batch_stage_n(int N, int f32, int form, int stage, const SlotDev* slots,
-                                 const WorkItem* work, int ntiles, int dry, const double* Dh,
+                                 const WorkItem* work, int ntiles, int dry, const double* Dh, int* err,
                                  cudaStream_t st);
 // Kernel form of a per-N launch over nelt elements in all (0: the large one), as the
 // single solver's default follows its mesh's size; elements per block of a form.

@@ -220,6 +220,18 @@ struct nwb_pool {
     bool snap_pending = false;
     std::vector<unsigned> snap_gen;
     unsigned next_gen = 1;
+    // status word of the stage kernels, in mapped host memory (host_block_alloc)
+    int* h_err = nullptr;
+    int* d_err = nullptr;
+
+    // After a wait for the device: has a stage kernel recorded an expired bounded wait?
+    nwb_status check_waits(const char* who) {
+        const int err = *const_cast<volatile int*>(h_err);
+        if (err == 0) return NWB_OK;
+        *const_cast<volatile int*>(h_err) = 0;
+        return set_error(NWB_ETIMEOUT, "%s: a stage kernel's bounded wait expired (code %d); the cavities stepped "
+                                       "since the last check are not valid", who, err);
+    }
 
     template <class T>
     T* ptr(const Range& r) const {
@@ -349,7 +361,7 @@ struct nwb_pool {
             for (int n = 0; n < nsteps && e == cudaSuccess; ++n) {
                 for (int s = 0; s < 5 && e == cudaSuccess; ++s)
                     e = nwb::launch_batch_stage_n(N, f32, n_form[N], s, d_slots, d_work_n + n_off[N], n_cnt[N], dry,
-                                                  all_canon ? canonD[N] : nullptr, c);
+                                                  all_canon ? canonD[N] : nullptr, d_err, c);
                 if (dry) continue;
                 if (e == cudaSuccess && diag)
                     e = nwb::launch_batch_diag(d_slots, d_work + w_off[N], w_cnt[N], nullptr, 1,
@@ -396,7 +408,7 @@ struct nwb_pool {
         grid = sms * std::min(3, by_smem);  // the kernel is built for 3 resident blocks
         diag_grid = sms * 4;
         for (int N = 2; N <= 10; ++N) {  // one-time kernel attribute set-up, outside capture
-            cudaError_t e = nwb::launch_batch_stage_n(N, f32, 0, 0, nullptr, nullptr, 0, 0, nullptr, st);
+            cudaError_t e = nwb::launch_batch_stage_n(N, f32, 0, 0, nullptr, nullptr, 0, 0, nullptr, nullptr, st);
             if (e != cudaSuccess) return set_error(NWB_ECUDA, "per-N set-up: %s", cudaGetErrorString(e));
         }
         return NWB_OK;
@@ -538,6 +550,12 @@ nwb_status nwb_pool_create(size_t hbm_budget_bytes, int max_slots, nwb_precision
     if (e == cudaSuccess) e = cudaMalloc(&p->d_work_n, sizeof(nwb::WorkItem) * p->work_n_cap);
     if (e == cudaSuccess) e = cudaMalloc(&p->d_slot_list, sizeof(int) * max_slots);
     if (e == cudaSuccess) e = p->stage.init();
+    if (e == cudaSuccess) {
+        p->h_err = static_cast<int*>(nwb::host_block_alloc());
+        e = p->h_err ? cudaHostGetDevicePointer(reinterpret_cast<void**>(&p->d_err), p->h_err, 0)
+                     : cudaErrorMemoryAllocation;
+        if (p->h_err) *p->h_err = 0;
+    }
     if (e == cudaSuccess)
         e = cudaHostAlloc(reinterpret_cast<void**>(&p->h_snap), sizeof(nwb::SlotDev) * max_slots + kResultBlock,
                           cudaHostAllocDefault);
@@ -799,7 +817,7 @@ nwb_status nwb_pool_step(nwb_pool* p, int nsteps) {
 nwb_status nwb_pool_sync(nwb_pool* p) {
     if (!p) return set_error(NWB_EINVAL, "nwb_pool_sync: null pool");
     NWB_PCU(cudaStreamSynchronize(p->st));
-    return NWB_OK;
+    return p->check_waits("nwb_pool_sync");
 }
 
 nwb_status nwb_pool_query(nwb_pool* p, int* status, int* done, int cap) {
@@ -820,7 +838,7 @@ nwb_status nwb_pool_query(nwb_pool* p, int* status, int* done, int cap) {
         if (status) status[s] = st;
         if (done) done[s] = h.used ? tmp[s].done : 0;
     }
-    return NWB_OK;
+    return p->check_waits("nwb_pool_query");
 }
 
 nwb_status nwb_pool_query_begin(nwb_pool* p) {
@@ -854,7 +872,7 @@ nwb_status nwb_pool_query_end(nwb_pool* p, int* status, int* done, int cap) {
         if (status) status[s] = st;
         if (done) done[s] = current ? d.done : 0;
     }
-    return NWB_OK;
+    return p->check_waits("nwb_pool_query_end");
 }
 
 nwb_status nwb_pool_results_async(nwb_pool* p, int s, double* state, double* energy, double* probes) {
@@ -900,8 +918,11 @@ nwb_status nwb_pool_results(nwb_pool* p, int s, double* state, double* energy, d
     if (eb && pinned) std::memcpy(energy, block, eb);
     if (pb && pinned) std::memcpy(probes, block + eb, pb);
     if (pinned_state) std::memcpy(state, block + eb + pb, sb);
-    return NWB_OK;
+    return p->check_waits("nwb_pool_results");
 }
+
+// The host's view of the pool's status word, for the test of its reports (not in nwb.h).
+int* nwb_pool_status_word_(nwb_pool* p) { return p ? p->h_err : nullptr; }
 
 nwb_status nwb_pool_remove(nwb_pool* p, int s) {
     if (!p || s < 0 || s >= p->max_slots) return set_error(NWB_EINVAL, "nwb_pool_remove: bad argument");
@@ -1013,6 +1034,7 @@ nwb_status nwb_pool_destroy(nwb_pool* p) {
     if (p->fork_ev) cudaEventDestroy(p->fork_ev);
     if (p->snap_ev) cudaEventDestroy(p->snap_ev);
     if (p->h_snap) cudaFreeHost(p->h_snap);
+    nwb::host_block_free(p->h_err);
     p->stage.destroy();
     if (p->st) cudaStreamDestroy(p->st);
     delete p;
