@@ -286,8 +286,9 @@ nwb_status nwb_time_stage_kernel(nwb_solver* s, double dt, int nstages, float* m
  * nwb_pool_step advances every uploaded, unfinished slot by up to nsteps steps
  * with one launch per LSRK stage and N present (or one persistent launch for
  * every N, nwb_pool_set_mode), replayed from CUDA graphs of one or four steps; a slot stops
- * by itself after its own nsteps.  Slots take axis-aligned box meshes (nwb_mesh_desc as above),
- * their own c0 and dt, up to 8 probes given as (element, tensor Lagrange
+ * by itself after its own nsteps.  Slots take axis-aligned box meshes (nwb_mesh_desc as above;
+ * where the metrics are diagonal and the normals are not along the axes, the general flux
+ * applies, in FP64, with the results but not the bits of nwb_solver), their own c0 and dt, up to 8 probes given as (element, tensor Lagrange
  * weights [3][N]) as ProbeManager builds them (src/probe.cpp:33-189), and record
  * the energy every energy_every steps (index 0 = initial state, NaN where not
  * recorded) and all six probe components every step.  Each slot's arithmetic is

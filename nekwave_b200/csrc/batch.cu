@@ -126,7 +126,7 @@ batch_stage_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict
         if (t >= ntiles) break;
         const WorkItem w = work[t];
         const SlotDev& S = slots[w.slot];
-        if (!S.active) continue;
+        if (!S.active || S.oblique) continue;
         const int par = S.par ^ (stage & 1);
         StageParams P;
         P.u_in = S.u[par];
@@ -497,6 +497,34 @@ cudaError_t launch_n(int form, const BatchStage& bs, const SlotDev* slots, const
     }
 }
 
+// The stage of the slots whose metrics are diagonal and whose normals are not along the axes
+// (arrays of a user's own: no mesher makes them).  The axis-aligned class's tiles take the
+// normals for granted, so these slots have the first family's general tile, in FP64 in both
+// precisions.  Launched only where an order has such a slot.
+template <int N>
+__global__ void __launch_bounds__(kBatchThreads)
+batch_oblique_kernel(const SlotDev* __restrict__ slots, const WorkItem* __restrict__ work,
+                     const __grid_constant__ BatchStage bs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    using B = BShape<N>;
+    const WorkItem w = work[blockIdx.x];
+    const SlotDev& S = slots[w.slot];
+    if (!S.active || !S.oblique) return;
+    const StageParams P = slot_params(S, bs);
+    stage_tile<N, GEO_AFFINE, false, B::KS, B::EPB, false, false>(P, w.e0, smem, threadIdx.x);
+}
+
+template <int N>
+cudaError_t launch_oblique_n(const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
+                             cudaStream_t st) {
+    constexpr int smem = SmemLayout<N, false, BShape<N>::EPB, false>::total;
+    auto kern = batch_oblique_kernel<N>;
+    static std::atomic<int> attr_set[kMaxDeviceSlots];  // per kernel and device
+    if (cudaError_t e = set_smem_once(kern, smem, attr_set); e != cudaSuccess) return e;
+    if (ntiles <= 0) return cudaSuccess;
+    return launch_overlapped(kern, ntiles, kBatchThreads, smem, st, false, slots, work, bs);
+}
+
 // Does this slot record energy after the step it is taking now (post = 1), or
 // is this the initial-state record (post = 0)?
 __device__ __forceinline__ bool wants_energy(const SlotDev& S, int post) {
@@ -656,6 +684,18 @@ cudaError_t launch_batch_stage_n(int N, int f32, int form, int stage, const Slot
 #define NWB_CASE(n) \
         case n: return f32 ? launch_n<n, true>(form, bs, slots, work, ntiles, Dh, st) \
                            : launch_n<n, false>(form, bs, slots, work, ntiles, Dh, st);
+        NWB_CASE(2) NWB_CASE(3) NWB_CASE(4) NWB_CASE(5) NWB_CASE(6) NWB_CASE(7) NWB_CASE(8)
+        NWB_CASE(9) NWB_CASE(10)
+#undef NWB_CASE
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_batch_oblique(int N, int stage, const SlotDev* slots, const WorkItem* work, int ntiles, int dry,
+                                 cudaStream_t st) {
+    const BatchStage bs{dry ? 0.0 : kRk4a[stage], dry ? 0.0 : kRk4b[stage], stage, dry, nullptr};
+    switch (N) {
+#define NWB_CASE(n) case n: return launch_oblique_n<n>(bs, slots, work, ntiles, st);
         NWB_CASE(2) NWB_CASE(3) NWB_CASE(4) NWB_CASE(5) NWB_CASE(6) NWB_CASE(7) NWB_CASE(8)
         NWB_CASE(9) NWB_CASE(10)
 #undef NWB_CASE

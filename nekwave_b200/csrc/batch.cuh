@@ -34,6 +34,7 @@ struct SlotDev {
     int snel[3], spmask;    // structured box: elements per axis and periodic axes, or 0
     unsigned sdiv[2];       // StageParams::sdiv, sshift
     int sshift[2];
+    int oblique;            // diagonal metrics with normals off the axes: launch_batch_oblique's
 };
 
 // One tile of work: EPB consecutive elements of one slot.
@@ -62,6 +63,11 @@ cudaError_t launch_batch_stage(int f32, int stage, const SlotDev* slots, const W
 // err: device pointer of the word in which an expired bounded wait is recorded.
 cudaError_t launch_batch_stage_n(int N, int f32, int form, int stage, const SlotDev* slots,
                                  const WorkItem* work, int ntiles, int dry, const double* Dh, int* err,
+                                 cudaStream_t st);
+// The same stage of the oblique slots among the work items [work, work + ntiles) of one N,
+// cut with batch_shape(N) elements (those of the other launches leave them out).  A plain
+// launch, not an overlapped one: the next stage of that N may overlap it.
+cudaError_t launch_batch_oblique(int N, int stage, const SlotDev* slots, const WorkItem* work, int ntiles, int dry,
                                  cudaStream_t st);
 // Kernel form of a per-N launch over nelt elements in all (0: the large one), as the
 // single solver's default follows its mesh's size; elements per block of a form.

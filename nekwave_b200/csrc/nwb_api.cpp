@@ -150,17 +150,29 @@ void host_block_free(void* p) {
     }
 }
 
-bool snap_axis_normals(std::vector<ElemGeo>& geo, double tol) {
-    constexpr int axis[6] = {1, 0, 1, 0, 2, 2};
-    for (const ElemGeo& G : geo)
+namespace {
+constexpr int kFaceAxis[6] = {1, 0, 1, 0, 2, 2};
+}
+
+bool snap_axis_normals(std::vector<ElemGeo>& geo) {
+    for (const ElemGeo& G : geo) {
+        double scale = 0.0;
+        for (int c = 0; c < 9; ++c) scale = std::max(scale, std::abs(G.met[c]));
         for (int f = 0; f < 6; ++f)
             for (int c = 0; c < 3; ++c)
-                if (c != axis[f] && !(std::abs(G.nrm[f][c]) <= tol)) return false;
+                if (c != kFaceAxis[f] &&
+                    !(std::abs(G.nrm[f][c] * G.met[4 * kFaceAxis[f]]) <= 1e-12 * scale))
+                    return false;
+    }
+    axis_normals(geo);
+    return true;
+}
+
+void axis_normals(std::vector<ElemGeo>& geo) {
     for (ElemGeo& G : geo)
         for (int f = 0; f < 6; ++f)
             for (int c = 0; c < 3; ++c)
-                if (c != axis[f]) G.nrm[f][c] = 0.0;
-    return true;
+                if (c != kFaceAxis[f]) G.nrm[f][c] = 0.0;
 }
 
 nwb_status analyse_mesh(const nwb_mesh_desc* m, Analysis* A, bool true_pmc) {

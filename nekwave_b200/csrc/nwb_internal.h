@@ -196,10 +196,16 @@ struct Analysis {
 // orientations): the stage kernels can then find neighbours from the element index.  Returns
 // false and leaves nel at 0 for any other table.
 bool detect_structure(const int* conn, int nelt, int nel[3], int* pm);
-// Do the face normals of every element lie along the axes of an axis-aligned element
-// (faces 1, 3: x; 0, 2: y; 4, 5: z) to tol?  If so their other components are
-// set to exactly zero, which the axis-aligned class's kernels take for granted.
-bool snap_axis_normals(std::vector<ElemGeo>& geo, double tol = 1e-12);
+// Do the face normals of every element with diagonal metrics lie along the axes (faces 1,
+// 3: x; 0, 2: y; 4, 5: z)?  If so their other components are set to exactly zero, which the
+// axis-aligned class's kernels take for granted (axis_normals does it in any case).  What a
+// component off the axis adds to a right-hand side is as large as an off-diagonal metric of
+// itself times the face's metric, so it is measured as those are: against the element's
+// largest metric (to 1e-12).  A bound on the component alone would take elements a
+// hundred-thousandth as thick as wide, whose corners' rounding turns the normals of their
+// narrow faces by 1e-11, for oblique ones.
+bool snap_axis_normals(std::vector<ElemGeo>& geo);
+void axis_normals(std::vector<ElemGeo>& geo);
 // true_pmc: bc_type 2 faces become kConnPMC (per-node class: neighbour -2) instead
 // of the reference's PEC mirror.
 nwb_status analyse_mesh(const nwb_mesh_desc* m, Analysis* A, bool true_pmc = false);

@@ -194,6 +194,7 @@ struct nwb_pool {
     nwb::WorkItem* d_work_n = nullptr;
     int work_n_cap = 0;
     int n_off[11] = {}, n_cnt[11] = {};
+    int n_oblique[11] = {};  // that N's oblique slots (SlotDev::oblique), not in its tiles
     int n_form[11] = {};  // kernel form of that N's launches (nwb::batch_form_n)
     // that N's range of the work list (energy tiles) and its slots (d_slot_list)
     int w_off[11] = {}, w_cnt[11] = {}, s_off[11] = {}, s_cnt[11] = {};
@@ -299,16 +300,23 @@ struct nwb_pool {
             s_cnt[N] = static_cast<int>(list.size()) - s_off[N];
         }
         std::vector<nwb::WorkItem> wn;
+        int had_oblique = 0, has_oblique = 0;
         for (int N = 2; N <= 10; ++N) {
             n_off[N] = static_cast<int>(wn.size());
             long long total = 0;
-            for (const SlotHost& h : slots)
-                if (h.used && h.N == N) total += h.nelt;
+            had_oblique += n_oblique[N];
+            n_oblique[N] = 0;
+            for (const SlotHost& h : slots) {
+                if (!h.used || h.N != N) continue;
+                if (h.dev.oblique) ++n_oblique[N];
+                else total += h.nelt;
+            }
+            has_oblique += n_oblique[N];
             n_form[N] = nwb::batch_form_n(N, f32, total);
             const int epb = nwb::batch_epb_n(N, f32, n_form[N]);
             for (int s = 0; s < max_slots; ++s) {
                 const SlotHost& h = slots[s];
-                if (!h.used || h.N != N) continue;
+                if (!h.used || h.N != N || h.dev.oblique) continue;
                 for (int e0 = 0; e0 < h.nelt; e0 += epb) wn.push_back(nwb::WorkItem{s, e0, N, 0});
             }
             n_cnt[N] = static_cast<int>(wn.size()) - n_off[N];
@@ -322,9 +330,15 @@ struct nwb_pool {
         if (r == NWB_OK) r = h2d(d_ntiles, &ntiles, sizeof(int));
         if (r == NWB_OK) r = h2d(d_slot_list, list.data(), sizeof(int) * list.size());
         if (r != NWB_OK) return r;
-        if (mode == 1) drop_graph();  // per-N grids follow the tile counts
+        // per-N grids follow the tile counts
+        if (mode == 1 || had_oblique || has_oblique) drop_graph();
         work_dirty = false;
         return NWB_OK;
+    }
+
+    cudaError_t launch_oblique(int N, int stage, int dry, cudaStream_t c) {
+        if (!n_oblique[N]) return cudaSuccess;
+        return nwb::launch_batch_oblique(N, stage, d_slots, d_work + w_off[N], w_cnt[N], dry, c);
     }
 
     // One step (dry = 1: its five stages with a = b = dt = 0, for timing).  Mode 1: the
@@ -340,6 +354,7 @@ struct nwb_pool {
             for (int s = 0; s < 5; ++s) {
                 cudaError_t e = nwb::launch_batch_stage(f32, s, d_slots, d_work, d_ntiles, d_counters, grid,
                                                         graph_smem, dry, st);
+                for (int N = 2; N <= 10 && e == cudaSuccess; ++N) e = launch_oblique(N, s, dry, st);
                 if (e != cudaSuccess) return set_error(NWB_ECUDA, "batch stage: %s", cudaGetErrorString(e));
             }
             if (dry) return NWB_OK;
@@ -351,7 +366,7 @@ struct nwb_pool {
         }
         NWB_PCU(cudaEventRecord(fork_ev, st));
         for (int N = 10; N >= 2; --N) {
-            if (!n_cnt[N]) continue;
+            if (!s_cnt[N]) continue;
             cudaStream_t c = side[N];
             NWB_PCU(cudaStreamWaitEvent(c, fork_ev, 0));
             bool all_canon = true;
@@ -359,9 +374,11 @@ struct nwb_pool {
                 if (slots[q].used && slots[q].N == N && !slots[q].dcanon) all_canon = false;
             cudaError_t e = cudaSuccess;
             for (int n = 0; n < nsteps && e == cudaSuccess; ++n) {
-                for (int s = 0; s < 5 && e == cudaSuccess; ++s)
+                for (int s = 0; s < 5 && e == cudaSuccess; ++s) {
                     e = nwb::launch_batch_stage_n(N, f32, n_form[N], s, d_slots, d_work_n + n_off[N], n_cnt[N], dry,
                                                   all_canon ? canonD[N] : nullptr, d_err, c);
+                    if (e == cudaSuccess) e = launch_oblique(N, s, dry, c);
+                }
                 if (dry) continue;
                 if (e == cudaSuccess && diag)
                     e = nwb::launch_batch_diag(d_slots, d_work + w_off[N], w_cnt[N], nullptr, 1,
@@ -409,6 +426,7 @@ struct nwb_pool {
         diag_grid = sms * 4;
         for (int N = 2; N <= 10; ++N) {  // one-time kernel attribute set-up, outside capture
             cudaError_t e = nwb::launch_batch_stage_n(N, f32, 0, 0, nullptr, nullptr, 0, 0, nullptr, nullptr, st);
+            if (e == cudaSuccess && n_oblique[N]) e = nwb::launch_batch_oblique(N, 0, nullptr, nullptr, 0, 0, st);
             if (e != cudaSuccess) return set_error(NWB_ECUDA, "per-N set-up: %s", cudaGetErrorString(e));
         }
         return NWB_OK;
@@ -576,7 +594,7 @@ namespace {
 nwb_status admit(nwb_pool* p, int N, int nelt, const double* D, const double* w3,
                  const nwb::ElemGeo* egeo, const int* conn, double c0, double dt, int nsteps,
                  int nprobes, const int* probe_elem, const double* probe_w, int energy_every,
-                 int* slot_out, SlotHost** host_out) {
+                 bool oblique, int* slot_out, SlotHost** host_out) {
     int s = -1;
     for (int i = 0; i < p->max_slots; ++i)
         if (!p->slots[i].used) {
@@ -646,6 +664,7 @@ nwb_status admit(nwb_pool* p, int N, int nelt, const double* D, const double* w3
     // 3.742 -> 3.729 ms
     if (nwb::detect_structure(conn, nelt, d.snel, &d.spmask))
         for (int x = 0; x < 2; ++x) nwb::set_divider(d.snel[x], &d.sdiv[x], &d.sshift[x]);
+    d.oblique = oblique ? 1 : 0;
     d.stride = h.stride;
     d.c0 = c0;
     d.dt = dt;
@@ -713,17 +732,15 @@ nwb_status nwb_pool_add(nwb_pool* p, const nwb_mesh_desc* m, double c0, double d
     } catch (const std::bad_alloc&) {
         return set_error(NWB_ENOMEM, "nwb_pool_add: out of host memory");
     }
-    // Elements a ten-thousandth as thick as wide can have normals further off the axes than
-    // 1e-12 from the rounding of their corners alone; the pool has no affine class to sort
-    // them into and takes them as axis-aligned.
-    const bool box = A.geo == nwb::GEO_BOX || (A.box_metrics && nwb::snap_axis_normals(A.egeo, 1e-9));
-    if (!box)
+    // diagonal metrics with normals off the axes: a launch of their own (the solver sorts such
+    // a mesh into the affine class)
+    if (!A.box_metrics)
         return set_error(NWB_EINVAL, "nwb_pool_add: the pool takes axis-aligned affine (box) meshes");
     for (int i = 0; i < nprobes; ++i)
         if (probe_elem[i] < 0 || probe_elem[i] >= m->nelt)
             return set_error(NWB_EINVAL, "nwb_pool_add: probe element out of range");
     return admit(p, m->N, m->nelt, m->D, m->w3, A.egeo.data(), A.conn.data(), c0, dt, nsteps, nprobes,
-                 probe_elem, probe_w, energy_every, slot_out, nullptr);
+                 probe_elem, probe_w, energy_every, A.geo != nwb::GEO_BOX, slot_out, nullptr);
 }
 
 nwb_status nwb_pool_add_box(nwb_pool* p, int N, int nelx, int nely, int nelz, double xmin,
@@ -745,7 +762,7 @@ nwb_status nwb_pool_add_box(nwb_pool* p, int N, int nelx, int nely, int nelz, do
     try {
         nwb::gll(N, z, w, D);
         nwb::box_geometry(N, nelx, nely, nelz, lo, hi, periodic_mask, z, w, geo, conn);
-        nwb::snap_axis_normals(geo);
+        nwb::axis_normals(geo);
         nwb::box_probes(N, nelx, nely, nelz, lo, hi, z, nprobes, probe_xyz, pe, pw);
     } catch (const std::bad_alloc&) {
         return set_error(NWB_ENOMEM, "nwb_pool_add_box: out of host memory");
@@ -756,7 +773,7 @@ nwb_status nwb_pool_add_box(nwb_pool* p, int N, int nelx, int nely, int nelz, do
             for (int i = 0; i < N; ++i) w3[i + N * (j + N * k)] = w[i] * w[j] * w[k];
     SlotHost* h = nullptr;
     nwb_status r = admit(p, N, static_cast<int>(nelt), D.data(), w3.data(), geo.data(), conn.data(), c0,
-                         dt, nsteps, nprobes, pe.data(), pw.data(), energy_every, slot_out, &h);
+                         dt, nsteps, nprobes, pe.data(), pw.data(), energy_every, false, slot_out, &h);
     if (r != NWB_OK) return r;
     h->is_box = true;
     nwb::BoxPulse& b = h->box;
