@@ -195,6 +195,7 @@ struct nwb_pool {
     int work_n_cap = 0;
     int n_off[11] = {}, n_cnt[11] = {};
     int n_oblique[11] = {};  // that N's oblique slots (SlotDev::oblique), not in its tiles
+    bool n_canon[11] = {};   // do that N's slots all use the pool's D for it?
     int n_form[11] = {};  // kernel form of that N's launches (nwb::batch_form_n)
     // that N's range of the work list (energy tiles) and its slots (d_slot_list)
     int w_off[11] = {}, w_cnt[11] = {}, s_off[11] = {}, s_cnt[11] = {};
@@ -267,58 +268,59 @@ struct nwb_pool {
     // The device copy of slot s's record, queued in stream order (no host wait).
     nwb_status write_slot(int s) { return h2d(d_slots + s, &slots[s].dev, sizeof(nwb::SlotDev)); }
 
-    // Work list: every tile of every used slot, largest tiles first, so the
-    // dynamic tile counter hands out the long tiles early.
+    // The work list: every tile of every used slot, in order of nodes per tile, so that the
+    // dynamic tile counter hands out the long tiles early.  Every tile of an order but a
+    // slot's last has the same nodes, so this goes order by order: each order's tiles are one
+    // range, and in it each slot's.  d_work_n holds the same elements cut for the per-N
+    // launches, d_slot_list the slots, both order by order.
     nwb_status rebuild_work() {
         if (!work_dirty) return NWB_OK;
-        std::vector<nwb::WorkItem> w;
+        std::vector<int> of[11], orders, list;  // the used slots of each order: one pass over the table
+        for (int s = 0; s < max_slots; ++s)
+            if (slots[s].used) of[slots[s].N].push_back(s);
         smem_needed = 0;
-        for (int s = 0; s < max_slots; ++s) {
-            const SlotHost& h = slots[s];
-            if (!h.used) continue;
-            smem_needed = std::max(smem_needed, nwb::batch_smem(h.N, f32));
-            for (int t = 0; t < h.ntiles; ++t) w.push_back(nwb::WorkItem{s, t * h.epb, h.N, t});
-        }
-        std::stable_sort(w.begin(), w.end(), [&](const nwb::WorkItem& a, const nwb::WorkItem& b) {
-            const long long ca = static_cast<long long>(slots[a.slot].epb) * a.N * a.N * a.N;
-            const long long cb = static_cast<long long>(slots[b.slot].epb) * b.N * b.N * b.N;
-            return ca > cb;
-        });
-        ntiles = static_cast<int>(w.size());
-        // the list is sorted by nodes per tile, which differ between the orders, and stable:
-        // each order's tiles are one range, and in it each slot's
-        for (int N = 2; N <= 10; ++N) w_off[N] = w_cnt[N] = 0;
-        for (int t = 0; t < ntiles; ++t) {
-            if (w[t].tile == 0) slots[w[t].slot].work_off = t;
-            if (w_cnt[w[t].N]++ == 0) w_off[w[t].N] = t;
-        }
-        std::vector<int> list;
         for (int N = 2; N <= 10; ++N) {
+            if (!of[N].empty()) {
+                orders.push_back(N);
+                smem_needed = std::max(smem_needed, nwb::batch_smem(N, f32));
+            }
             s_off[N] = static_cast<int>(list.size());
-            for (int s = 0; s < max_slots; ++s)
-                if (slots[s].used && slots[s].N == N) list.push_back(s);
-            s_cnt[N] = static_cast<int>(list.size()) - s_off[N];
+            s_cnt[N] = static_cast<int>(of[N].size());
+            list.insert(list.end(), of[N].begin(), of[N].end());
         }
-        std::vector<nwb::WorkItem> wn;
+        std::stable_sort(orders.begin(), orders.end(), [&](int a, int b) {
+            return nwb::batch_shape(a, f32).epb * a * a * a > nwb::batch_shape(b, f32).epb * b * b * b;
+        });
+        std::vector<nwb::WorkItem> w, wn;
+        for (int N = 2; N <= 10; ++N) w_off[N] = w_cnt[N] = 0;
+        for (int N : orders) {
+            w_off[N] = static_cast<int>(w.size());
+            for (int s : of[N]) {
+                SlotHost& h = slots[s];
+                h.work_off = static_cast<int>(w.size());
+                for (int t = 0; t < h.ntiles; ++t) w.push_back(nwb::WorkItem{s, t * h.epb, N, t});
+            }
+            w_cnt[N] = static_cast<int>(w.size()) - w_off[N];
+        }
+        ntiles = static_cast<int>(w.size());
         int had_oblique = 0, has_oblique = 0;
         for (int N = 2; N <= 10; ++N) {
             n_off[N] = static_cast<int>(wn.size());
             long long total = 0;
             had_oblique += n_oblique[N];
             n_oblique[N] = 0;
-            for (const SlotHost& h : slots) {
-                if (!h.used || h.N != N) continue;
-                if (h.dev.oblique) ++n_oblique[N];
-                else total += h.nelt;
+            n_canon[N] = true;
+            for (int s : of[N]) {
+                if (slots[s].dev.oblique) ++n_oblique[N];
+                else total += slots[s].nelt;
+                n_canon[N] = n_canon[N] && slots[s].dcanon;
             }
             has_oblique += n_oblique[N];
             n_form[N] = nwb::batch_form_n(N, f32, total);
             const int epb = nwb::batch_epb_n(N, f32, n_form[N]);
-            for (int s = 0; s < max_slots; ++s) {
-                const SlotHost& h = slots[s];
-                if (!h.used || h.N != N || h.dev.oblique) continue;
-                for (int e0 = 0; e0 < h.nelt; e0 += epb) wn.push_back(nwb::WorkItem{s, e0, N, 0});
-            }
+            for (int s : of[N])
+                for (int e0 = 0; e0 < slots[s].nelt && !slots[s].dev.oblique; e0 += epb)
+                    wn.push_back(nwb::WorkItem{s, e0, N, 0});
             n_cnt[N] = static_cast<int>(wn.size()) - n_off[N];
         }
         // both lists were sized at creation for every admissible cavity set
@@ -369,14 +371,11 @@ struct nwb_pool {
             if (!s_cnt[N]) continue;
             cudaStream_t c = side[N];
             NWB_PCU(cudaStreamWaitEvent(c, fork_ev, 0));
-            bool all_canon = true;
-            for (int q = 0; q < max_slots; ++q)
-                if (slots[q].used && slots[q].N == N && !slots[q].dcanon) all_canon = false;
             cudaError_t e = cudaSuccess;
             for (int n = 0; n < nsteps && e == cudaSuccess; ++n) {
                 for (int s = 0; s < 5 && e == cudaSuccess; ++s) {
                     e = nwb::launch_batch_stage_n(N, f32, n_form[N], s, d_slots, d_work_n + n_off[N], n_cnt[N], dry,
-                                                  all_canon ? canonD[N] : nullptr, d_err, c);
+                                                  n_canon[N] ? canonD[N] : nullptr, d_err, c);
                     if (e == cudaSuccess) e = launch_oblique(N, s, dry, c);
                 }
                 if (dry) continue;
