@@ -21,6 +21,7 @@
 //   * per-slot energy history and probe traces are recorded on the device.
 #include "batch.cuh"
 #include "nwb.h"
+#include "pool_schedule.h"
 
 #include <algorithm>
 #include <cmath>
@@ -161,8 +162,6 @@ struct SlotHost {
     unsigned gen = 0;     // admission generation: status snapshots of an older one are ignored
     bool dcanon = false;  // its D equals the pool's D for its N (the GLL operator)
     bool uploaded = false;
-    long long queued = 0;   // pool steps queued since the initial state: every one takes an
-                            // unfinished slot one step on, so steps done = min(queued, nsteps)
     int work_off = 0;       // first of its ntiles entries in the work list
     bool is_box = false;
     nwb::BoxPulse box{};
@@ -182,6 +181,7 @@ struct nwb_pool {
     Arena arena;
     int max_slots = 0;
     std::vector<SlotHost> slots;
+    nwb::StepSchedule schedule;
     nwb::SlotDev* d_slots = nullptr;
     nwb::WorkItem* d_work = nullptr;
     int work_cap = 0;
@@ -431,17 +431,6 @@ struct nwb_pool {
         return NWB_OK;
     }
 
-    // Does a slot record its energy in one of the next nsteps steps (at every energy_every-th
-    // step and at its last)?
-    bool wants_energy(int nsteps) const {
-        for (const SlotHost& h : slots) {
-            if (!h.used || !h.uploaded || h.queued >= h.nsteps) continue;
-            const long long q = h.queued, last = std::min<long long>(q + nsteps, h.nsteps);
-            if (last / h.energy_every > q / h.energy_every || last == h.nsteps) return true;
-        }
-        return false;
-    }
-
     // A pool whose cavities change often keeps to single steps: the longer graph is captured
     // for a call of at least four of it.
     bool use_many(int nsteps) const {
@@ -463,13 +452,12 @@ struct nwb_pool {
         while (nsteps > 0) {
             const int many = use_many(nsteps);
             const int n = many ? kManySteps : 1;
-            const int diag = mode == 0 || wants_energy(n);
+            const int diag = mode == 0 || schedule.records(n);
             r = need_graph(many, diag);
             if (r != NWB_OK) return r;
             NWB_PCU(cudaGraphLaunch(graph[many][diag], st));
             launches += 7 * n;
-            for (SlotHost& h : slots)
-                if (h.uploaded) h.queued += n;
+            schedule.advance(n);
             nsteps -= n;
         }
         return NWB_OK;
@@ -495,13 +483,14 @@ struct nwb_pool {
         }
         launches += 2;
         h.uploaded = true;
-        h.queued = 0;
+        schedule.start(s, h.nsteps, h.energy_every);
         return NWB_OK;
     }
 
     void release_slot(int s) {
         for (const Range& r : slots[s].ranges) arena.release(r);
         slots[s] = SlotHost{};
+        schedule.remove(s);
     }
 };
 
@@ -520,6 +509,7 @@ nwb_status nwb_pool_create(size_t hbm_budget_bytes, int max_slots, nwb_precision
     p->f32 = prec == NWB_FP32_BULK;
     p->max_slots = max_slots;
     p->slots.resize(max_slots);
+    p->schedule = nwb::StepSchedule(max_slots);
     auto bail = [&](nwb_status r) {
         nwb_pool_destroy(p);
         return r;
@@ -914,9 +904,9 @@ nwb_status nwb_pool_results(nwb_pool* p, int s, double* state, double* energy, d
     if (!p || s < 0 || s >= p->max_slots) return set_error(NWB_EINVAL, "nwb_pool_results: bad argument");
     SlotHost& h = p->slots[s];
     if (!h.used) return set_error(NWB_ENOTFOUND, "nwb_pool_results: slot %d is free", s);
-    // the parity follows from the steps queued (SlotHost::queued): no copy of the record
-    // ahead of the state's.  Results come through a pinned block, with one wait for all.
-    const int par = static_cast<int>(std::min<long long>(h.queued, h.nsteps) & 1);
+    // the parity follows from the steps queued: no copy of the record ahead of the state's.
+    // Results come through a pinned block, with one wait for all.
+    const int par = p->schedule.taken(s) & 1;
     const size_t eb = energy ? sizeof(double) * (h.nsteps + 1) : 0;
     const size_t pb = probes && h.nprobes ? sizeof(double) * 6 * h.nprobes * (h.nsteps + 1) : 0;
     const size_t sb = state ? sizeof(double) * 6 * static_cast<size_t>(h.npts) : 0;
