@@ -27,6 +27,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -218,6 +219,7 @@ struct nwb_pool {
     // table copied into pinned memory, and each slot's generation when it was taken
     nwb::SlotDev* h_snap = nullptr;
     char* h_result = nullptr;  // kResultBlock bytes of pinned memory behind it (nwb_pool_results)
+    std::mutex result_mu;      // held while a call uses it
     cudaEvent_t snap_ev = nullptr;
     bool snap_pending = false;
     std::vector<unsigned> snap_gen;
@@ -912,6 +914,7 @@ nwb_status nwb_pool_results(nwb_pool* p, int s, double* state, double* energy, d
     const size_t sb = state ? sizeof(double) * 6 * static_cast<size_t>(h.npts) : 0;
     const bool pinned = eb + pb <= kResultBlock, pinned_state = sb && pinned && eb + pb + sb <= kResultBlock;
     char* const block = p->h_result;
+    std::lock_guard<std::mutex> lock(p->result_mu);
     if (eb) NWB_PCU(cudaMemcpyAsync(pinned ? block : static_cast<void*>(energy), h.dev.energy, eb,
                                     cudaMemcpyDeviceToHost, p->st));
     if (pb) NWB_PCU(cudaMemcpyAsync(pinned ? block + eb : static_cast<void*>(probes), h.dev.probes, pb,

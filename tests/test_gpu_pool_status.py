@@ -3,6 +3,7 @@ the next call that waits for the device reports it.  The word is set from the ho
 wait of a kernel is made to run out."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
 from nekwave_b200 import _lib
@@ -35,4 +36,23 @@ def test_an_expired_wait_is_reported_once(gpu, call):
         wait()
     assert e.value.status == _lib.NWB_ETIMEOUT and "bounded wait" in str(e.value)
     wait()
+    pool.close()
+
+
+def test_results_of_several_slots_at_once(gpu):
+    """Threads that each read another slot's results share the pool's pinned block, one at a
+    time; ctypes calls run side by side."""
+    from concurrent.futures import ThreadPoolExecutor
+    n = 6
+    pool = CavityPool(256 << 20, max_slots=n)
+    slots = [pool.add_box(4 + i % 3, (4, 3, 2), (0, 0, 0), (1, 1, 1), 1.0, 1e-3, 4) for i in range(n)]
+    for i, s in enumerate(slots):
+        pool.init_pulse(s, [(1.0 + i, 0.4, 0.5, 0.6, 0.2)] * 6)
+    pool.step(4)
+    want = [pool.results(s) for s in slots]
+    with ThreadPoolExecutor(n) as ex:
+        for _ in range(50):
+            for w, r in zip(want, ex.map(pool.results, slots)):
+                np.testing.assert_array_equal(r["state"], w["state"])
+                np.testing.assert_array_equal(r["energy"], w["energy"])
     pool.close()
