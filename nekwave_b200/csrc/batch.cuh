@@ -84,17 +84,6 @@ cudaError_t launch_batch_diag(SlotDev* slots, const WorkItem* work, int ntiles, 
 // counters (when given).
 cudaError_t launch_batch_epilogue(SlotDev* slots, const int* slot_list, int first_slot, int nslots, int post,
                                   int* counters, bool overlap, cudaStream_t st);
-// Gaussian pulses on the nodes of an axis-aligned box cavity: component c gets
-// pulse[c*5+0] * exp(-|x - (pulse[c*5+1..3])|^2 / pulse[c*5+4]^2) (zero where
-// pulse[c*5+4] <= 0), node positions from the box's uniform element grid.
-struct BoxPulse {
-    double lo[3], h[3];
-    int nel[3];
-    int N;
-    double pulse[30];
-    double z[10];  // GLL nodes
-};
-cudaError_t launch_box_pulse(const BoxPulse& b, double* u, long long stride, cudaStream_t st);
 
 // Shape per N used by the batch kernel and its dynamic shared memory need.
 BatchShape batch_shape(int N, int f32);

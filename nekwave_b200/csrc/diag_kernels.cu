@@ -192,6 +192,35 @@ __global__ void l2_flush_kernel(int4* __restrict__ buf, size_t n16) {
         buf[x] = make_int4(static_cast<int>(x), 0, 0, 0);
 }
 
+// Gaussian pulses on the nodes of a box (launch_box_pulse).  Here, in a small module, and not
+// beside the pool's kernels: the first launch from a module loads the whole of it.
+__global__ void box_pulse_kernel(const BoxPulse b, double* __restrict__ u, long long stride) {
+    const int N = b.N, N3 = N * N * N;
+    const long long npts = static_cast<long long>(b.nel[0]) * b.nel[1] * b.nel[2] * N3;
+    for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < npts;
+         p += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long e = p / N3;
+        const int m = static_cast<int>(p - e * N3);
+        const int i = m % N, j = (m / N) % N, k = m / (N * N);
+        const int ex = static_cast<int>(e % b.nel[0]);
+        const int ey = static_cast<int>((e / b.nel[0]) % b.nel[1]);
+        const int ez = static_cast<int>(e / (static_cast<long long>(b.nel[0]) * b.nel[1]));
+        const double x = b.lo[0] + (ex + 0.5 * (b.z[i] + 1.0)) * b.h[0];
+        const double y = b.lo[1] + (ey + 0.5 * (b.z[j] + 1.0)) * b.h[1];
+        const double z = b.lo[2] + (ez + 0.5 * (b.z[k] + 1.0)) * b.h[2];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            const double* q = b.pulse + 5 * c;
+            double v = 0.0;
+            if (q[4] > 0.0) {
+                const double dx = x - q[1], dy = y - q[2], dz = z - q[3];
+                v = q[0] * exp(-(dx * dx + dy * dy + dz * dz) / (q[4] * q[4]));
+            }
+            u[c * stride + p] = v;
+        }
+    }
+}
+
 }  // namespace
 
 int energy_blocks(int nelt) {
@@ -226,6 +255,11 @@ cudaError_t launch_probes(const double* u, long long stride, int N3, const long 
     if (nprobes <= 0) return cudaSuccess;
     return launch_overlapped(probe_kernel, nprobes, kProbeThreads, 0, st, true, u, stride, N3, offset, w, nprobes,
                              out);
+}
+
+cudaError_t launch_box_pulse(const BoxPulse& b, double* u, long long stride, cudaStream_t st) {
+    box_pulse_kernel<<<148 * 8, 256, 0, st>>>(b, u, stride);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_l2_flush(void* buf, size_t bytes, cudaStream_t st) {

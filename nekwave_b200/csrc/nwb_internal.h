@@ -245,6 +245,18 @@ cudaError_t launch_stage_n(int geo, int f32, int variant, const StageParams* p, 
 template <int N>
 int stage_variant_count_n(int geo, int f32);
 
+// Gaussian pulses on the nodes of an axis-aligned box cavity (diag_kernels.cu): component c gets
+// pulse[c*5+0] * exp(-|x - (pulse[c*5+1..3])|^2 / pulse[c*5+4]^2) (zero where
+// pulse[c*5+4] <= 0), node positions from the box's uniform element grid.
+struct BoxPulse {
+    double lo[3], h[3];
+    int nel[3];
+    int N;
+    double pulse[30];
+    double z[10];  // GLL nodes
+};
+cudaError_t launch_box_pulse(const BoxPulse& b, double* u, long long stride, cudaStream_t st);
+
 // FP64 energy of the state u (diag_kernels.cu): nblocks partial sums, then one
 // fixed-order final sum into *out (device).  J comes from jac_e (per element,
 // affine meshes) or jac_n (per node).
