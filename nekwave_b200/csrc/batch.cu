@@ -291,7 +291,8 @@ template <> struct NBulk<7> { static constexpr int EPB = 1, MINB = 4, KSM = 1, A
 template <> struct NBulk<9> { static constexpr int EPB = 1, MINB = 2, KSM = 1, AHEAD = 0; };
 template <> struct NBulk<10> { static constexpr int EPB = 1, MINB = 2, KSM = 0, AHEAD = 0; };
 
-// The four-threads-per-column form, for launches over few elements (NWB_SMALL): form 1.
+// The four-threads-per-column form, for launches over few elements (NWB_SMALL): form 1.  Not at
+// 8 points.
 template <int N> struct NQuad { static constexpr int EPB = 1, MINB = 2, KSM = 1; };
 template <> struct NQuad<2> { static constexpr int EPB = 8, MINB = 4, KSM = 1; };
 template <> struct NQuad<3> { static constexpr int EPB = 2, MINB = 8, KSM = 1; };
@@ -406,20 +407,18 @@ cudaError_t launch_quad_n(const BatchStage& bs, const SlotDev* slots, const Work
 }
 
 // The form of a per-N launch (batch_form_n): 0 large, 1 four threads per column, 2 (6 points)
-// one element per block.
+// one element per block.  4 and 8 points have one form.
 template <int N, bool CD>
 cudaError_t launch_form_n(int form, const BatchStage& bs, const SlotDev* slots, const WorkItem* work, int ntiles,
                           const DParam& dp, cudaStream_t st) {
     if constexpr (N == 4) return launch_quad_n<N, CD>(bs, slots, work, ntiles, dp, st);
+    else if constexpr (N == 8) return launch_dmma8_n<CD>(bs, slots, work, ntiles, dp, st);
     else {
         if (form == 1) return launch_quad_n<N, CD>(bs, slots, work, ntiles, dp, st);
         if constexpr (N == 6)
             if (form == 2) return launch_bulk_n<N, 1, 5, true, false, CD>(bs, slots, work, ntiles, dp, st);
-        if constexpr (N == 8) return launch_dmma8_n<CD>(bs, slots, work, ntiles, dp, st);
-        else {
-            using B = NBulk<N>;
-            return launch_bulk_n<N, B::EPB, B::MINB, B::KSM != 0, (B::AHEAD > 0), CD>(bs, slots, work, ntiles, dp, st);
-        }
+        using B = NBulk<N>;
+        return launch_bulk_n<N, B::EPB, B::MINB, B::KSM != 0, (B::AHEAD > 0), CD>(bs, slots, work, ntiles, dp, st);
     }
 }
 
@@ -684,12 +683,8 @@ int epb_n(int f32, int form) {
         else return NShape<N>::EPB;
     }
     if constexpr (N == 4) return NQuad<N>::EPB;
-    else {
-        if (form == 1) return NQuad<N>::EPB;
-        if (form == 2 || N == 8) return 1;
-        if constexpr (N != 8) return NBulk<N>::EPB;
-        else return 1;
-    }
+    else if constexpr (N == 8) return 1;
+    else return form == 1 ? NQuad<N>::EPB : form == 2 ? 1 : NBulk<N>::EPB;
 }
 }  // namespace
 

@@ -24,10 +24,9 @@
 //          D(k,l) are compile-time indices into a kernel-parameter copy of D (Dc,
 //          StageParams::Dc or the pool's per-N parameter) and enter the FMAs as
 //          constant-bank operands instead of shared loads.
-//   FACEFIRST (without PIPE) the whole face phase runs from global memory (own and
-//          neighbour traces, connections, normals and lifts through the read-only
-//          path) while the tile's copies are in flight; the column phase follows
-//          the wait.  The face phase's latency then overlaps the tile's.
+//   FACEFIRST (without PIPE; axis-aligned, SPLIT) the whole face phase runs from global
+//          memory (own and neighbour traces, connections, normals and lifts) while the
+//          tile's copies are in flight; the column phase follows the wait.  The face phase's latency then overlaps the tile's.
 //   DSMEM  (with SPLIT) the D rows a thread contracts with are read from shared
 //          memory at each use instead of being held in 2N registers, which buys
 //          resident blocks for the latency-bound orders at the price of more
@@ -472,70 +471,6 @@ __device__ __forceinline__ void face_phase2(const StageParams& P, const int e0, 
 #pragma unroll
             for (int c = 0; c < 6; ++c) F[c * N2] = lift * static_cast<double>(fl[c]);
         }
-    }
-}
-
-// Face phase from global memory only: own and neighbour traces, connections (or
-// the box structure), normals and lifts, so that it runs while the tile's copies
-// are in flight.  Writes the lifted fluxes into sflux like face_phase2; the caller
-// synchronises after waiting for the tile.
-template <int N, int GEO, bool F32, int KS, int EPB>
-__device__ __forceinline__ void face_phase_global(const StageParams& P, const int e0, double* sflux,
-                                                  const int tid) {
-    using TC = typename std::conditional<F32, float, double>::type;
-    constexpr int N2 = N * N, N3 = N2 * N;
-    constexpr int TPE = KS * N2;
-    constexpr int FPT = face_points_per_thread<N, KS>();
-    const int team = tid / TPE;
-    const int lt = tid - team * TPE;
-    const int e = e0 + team;
-    if (team >= min(EPB, P.nelt - e0)) return;
-    const long long S = P.stride;
-    FaceGather<FPT, GEO == GEO_NODAL> G;
-    gather2<N, GEO, KS, EPB, false, false>(P, e0, nullptr, nullptr, tid, G);
-    double own[FPT][6];
-#pragma unroll
-    for (int q = 0; q < FPT; ++q) {
-        const int fp = lt + q * TPE;
-        if (fp < 6 * N2) {
-            const int f = fp / N2;
-            const int pq = fp - f * N2;
-            const long long g = static_cast<long long>(e) * N3 + face_local<N>(f, pq % N, pq / N);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) own[q][c] = ld_state(P.u_in + c * S + g);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < FPT; ++q) {
-        const int fp = lt + q * TPE;
-        if (fp >= 6 * N2) break;
-        const int f = fp / N2;
-        const int pq = fp - f * N2;
-        double nxd, nyd, nzd, lift;
-        if constexpr (GEO == GEO_NODAL) {
-            nxd = G.nl[q][0];
-            nyd = G.nl[q][1];
-            nzd = G.nl[q][2];
-            lift = G.nl[q][3];
-        } else {
-            const ElemGeo* Gp = P.geo + e;
-            nxd = __ldg(&Gp->nrm[f][0]);
-            nyd = __ldg(&Gp->nrm[f][1]);
-            nzd = __ldg(&Gp->nrm[f][2]);
-            lift = __ldg(&Gp->lift[f]);
-        }
-        double jmp[6];
-        if (G.vB[q] < 0) {
-            wall_jumps(G.vB[q], own[q][0], own[q][1], own[q][2], own[q][3], own[q][4], own[q][5], jmp);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) jmp[c] = G.nb[q][c] - own[q][c];
-        }
-        TC fl[6];
-        face_flux<TC, GEO, N>(f, nxd, nyd, nzd, P.c0, jmp, fl);
-        double* F = sflux + (team * 6 + f) * 6 * N2 + pq;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) F[c * N2] = lift * static_cast<double>(fl[c]);
     }
 }
 
@@ -1428,13 +1363,12 @@ __global__ void __launch_bounds__(EPB * KS * N * N, MINB)
     auto sg = [&](int b) { return reinterpret_cast<ElemGeo*>(smem + L::geo0 + b * L::geo_b); };
     auto sc = [&](int b) { return reinterpret_cast<int*>(smem + L::conn0 + b * L::conn_b); };
     static_assert(!((EARLY || FACEFIRST) && PIPE), "early forms belong to the one-tile form");
+    static_assert(!FACEFIRST || box_faces<GEO, SPLIT>(), "face phase first: axis-aligned field split");
     FaceRegs<N, GEO, KS, SPLIT> G;
     issue2<N, GEO, EPB, NT, PAD>(P, t * EPB, su(0), sg(0), sc(0), tid);
     cp_async_commit();
     if constexpr (!PIPE) {
-        if constexpr (FACEFIRST && box_faces<GEO, SPLIT>())
-            face_phase_box_global<N, F32, KS, EPB>(P, t * EPB, sflux, tid, G);
-        else if constexpr (FACEFIRST) face_phase_global<N, GEO, F32, KS, EPB>(P, t * EPB, sflux, tid);
+        if constexpr (FACEFIRST) face_phase_box_global<N, F32, KS, EPB>(P, t * EPB, sflux, tid, G);
         else if constexpr (EARLY && box_faces<GEO, SPLIT>())
             gather_box<N, KS, EPB, PAD, false>(P, t * EPB, nullptr, nullptr, tid, G);
         else if constexpr (EARLY) gather2<N, GEO, KS, EPB, PAD, false>(P, t * EPB, nullptr, nullptr, tid, G);
