@@ -105,8 +105,10 @@ struct HostSlab {
     std::vector<int> free;  // block numbers
 };
 constexpr int kSlabBlocks = 256;
-std::mutex g_slab_mu;
-std::vector<HostSlab> g_slabs;
+// Not destroyed at exit: a program's own static objects may give their solvers back after this
+// library's would have gone.
+std::mutex& g_slab_mu = *new std::mutex;
+std::vector<HostSlab>& g_slabs = *new std::vector<HostSlab>;
 }  // namespace
 
 void* host_block_alloc() {
