@@ -51,7 +51,7 @@ struct BatchShape {
 
 // Batch launchers (batch.cu).
 // stage: 0..4.  counters[stage] is the dynamic tile counter of that stage.
-// dry = 1 runs the stage with a = b = dt = 0 (timing only: u_out = u_in, k = 0).
+// dry = 1 runs the stage with a = b = dt = 0 (timing only: u_out = u_in).
 cudaError_t launch_batch_stage(int f32, int stage, const SlotDev* slots, const WorkItem* work,
                                const int* ntiles, int* counters, int grid, int smem, int dry,
                                cudaStream_t st);

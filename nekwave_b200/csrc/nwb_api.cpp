@@ -1112,8 +1112,7 @@ nwb_status nwb_solver_set_variant(nwb_solver* s, int variant) {
 
 // Times every launch shape of the stage kernel on this solver's mesh and keeps
 // the fastest.  The timed launches use a = b = dt = 0, so they leave the state
-// bit for bit as it was and reset the LSRK register to zero (which the first
-// stage of every step multiplies by a = 0 anyway).
+// bit for bit as it was; what they leave in the LSRK register no step reads.
 nwb_status nwb_solver_autotune(nwb_solver* s, int reps, int* best, float* ms_out, int ms_cap) {
     if (!s || reps < 1) return fail(NWB_EINVAL, "nwb_solver_autotune: bad argument");
     const int nv = nwb::stage_variant_count(s->N, s->geo, s->f32);

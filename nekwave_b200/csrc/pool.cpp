@@ -990,9 +990,8 @@ nwb_status nwb_pool_set_mode(nwb_pool* p, int mode) {
 }
 
 // Times the five stage launches of both modes on the resident cavities (dry
-// stages: a = b = dt = 0, which leaves every state as it is and zeroes the LSRK
-// registers, which the first stage of the next step multiplies by a = 0) and
-// keeps the faster mode.
+// stages: a = b = dt = 0, which leaves every state as it is; what they leave in the LSRK
+// registers the next step does not read) and keeps the faster mode.
 nwb_status nwb_pool_autotune(nwb_pool* p, int reps, int* best_mode, float* ms_out /* [2] */) {
     if (!p || reps < 1) return set_error(NWB_EINVAL, "nwb_pool_autotune: bad argument");
     float t[2] = {0.f, 0.f};

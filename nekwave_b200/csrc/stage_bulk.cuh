@@ -259,8 +259,9 @@ struct MeshPull {
 
 // AHEAD (0, 1, 2): block b also pulls into L2 the tile of the block that starts
 // about AHEAD/2 waves of resident blocks later, so that block's bulk copies read L2
-// instead of DRAM; 0: no pull.  On B200 this pays where few blocks are resident
-// (6 and 9 points: 3 and 2 per SM), whose tile waits the other blocks hide least.
+// instead of DRAM; 0: no pull.  On B200 this pays at 6 points (3 resident blocks
+// per SM, whose tile waits the other blocks hide least); at 9 points, with 2, it paid only
+// while the faces kept the L1 pipe busy.
 template <int N, int GEO, int KS, int EPB, int MINB, bool CONSTD, bool DSMEM, bool KSM, bool EARLY,
           bool ZCOL, bool VROW, bool ILP2, int AHEAD, bool F32, int KIO>
 __global__ void __launch_bounds__(EPB * KS * N * N, MINB)

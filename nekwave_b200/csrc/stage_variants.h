@@ -35,7 +35,7 @@
 // geometry classes, whose default is the first entry that is not FP64-only and
 // which have that one variant.  The autotuner (nwb_solver_autotune) times every
 // variant of the axis-aligned class on the caller's own mesh.  The pool's per-N
-// kernels (batch.cu NShape/BShape) use the same arithmetic as the default.
+// kernels (batch.cu) use the same arithmetic as the default.
 #pragma once
 
 // The default of meshes with few elements: X(n, i), in order -- up to n elements variant 0
